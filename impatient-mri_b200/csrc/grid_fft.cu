@@ -9,6 +9,7 @@
 // other with a single barrier in between.
 #include "common.cuh"
 #include "grid_fft.cuh"
+#include "grid_fft2.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -199,34 +200,6 @@ __device__ __forceinline__ void stage_generic(const float2 *__restrict__ A, floa
     }
 }
 
-struct AxisArgs {
-    long long S;       // element stride of the axis (product of the faster lengths)
-    int n, ln;         // axis length and its log2 (when a power of two)
-    int cw, lcw, rs;   // lines per block (power of two), log2(cw), tile row stride
-    int nst;           // stages
-    unsigned char rad[24];
-    // Pruning.  Outputs kept along this axis: j < klo or j >= n - khi (klo = n:
-    // all).  Lines: only those whose coordinates along the faster axes are kept
-    // there, enumerated compactly: nf faster axes (outer first) with kept
-    // ranges [0, flo) and [fg - fhi, fg); Sc = product of their kept counts.
-    int klo, khi;
-    int nf;
-    int flo[2], fhi[2], fg[2];
-    long long Sc;
-};
-
-// Offset (within S) of compact line index ic over the kept faster coordinates.
-__device__ __forceinline__ long long line_offset(const AxisArgs &p, long long ic) {
-    auto ex = [](long long c, int lo, int hi, int g) -> long long {
-        return c < lo ? c : c + (g - lo - hi);
-    };
-    if (p.nf == 0) return ic;
-    if (p.nf == 1) return ex(ic, p.flo[0], p.fhi[0], p.fg[0]);
-    const long long inner = p.flo[1] + p.fhi[1];
-    const long long y = ic / inner, z = ic - y * inner;
-    return ex(y, p.flo[0], p.fhi[0], p.fg[0]) * p.fg[1] + ex(z, p.flo[1], p.fhi[1], p.fg[1]);
-}
-
 constexpr int kLoadUnroll = 4;  // global loads a thread issues before its shared stores
 
 // One axis pass.  Block b takes lines l0 = b cw .. l0 + cw - 1 (line l = o S + i
@@ -383,6 +356,7 @@ cudaError_t grid_fft_create(GridFft *f, int n0, int n1, int n2, int batch) {
                               (const void *)k_fft_axis<true, true>})
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        if (e == cudaSuccess) e = fft2_setup();
         if (e != cudaSuccess) return e;
     }
     for (int a = 0; a < 3; ++a) {
@@ -427,11 +401,12 @@ void grid_fft_destroy(GridFft *f) {
 }
 
 cudaError_t grid_fft_exec(const GridFft &f, float2 *data, bool inverse, cudaStream_t st) {
-    return grid_fft_exec_cropped(f, data, inverse, nullptr, st);
+    return grid_fft_exec_cropped(f, data, inverse, nullptr, st, f.batch);
 }
 
 cudaError_t grid_fft_exec_cropped(const GridFft &f, float2 *data, bool inverse,
-                                  const int keep_half[3], cudaStream_t st) {
+                                  const int keep_half[3], cudaStream_t st, int batch) {
+    if (batch < 1 || batch % f.batch) return cudaErrorInvalidValue;
     // kept output range per axis: [0, lo) and [n - hi, n)
     int klo[3], khi[3];
     for (int a = 0; a < 3; ++a) {
@@ -451,7 +426,7 @@ cudaError_t grid_fft_exec_cropped(const GridFft &f, float2 *data, bool inverse,
         if (len == 1) continue;
         AxisArgs p;
         p.S = 1;
-        long long O = f.batch;
+        long long O = batch;
         for (int b = a + 1; b < 3; ++b) p.S *= f.n[b];
         for (int b = 0; b < a; ++b) O *= f.n[b];
         p.n = len;
@@ -475,14 +450,21 @@ cudaError_t grid_fft_exec_cropped(const GridFft &f, float2 *data, bool inverse,
             gap = gap || khi[b] > 0;
             ++p.nf;
         }
-        p.cw = f.cw[a];
+        const int two = fft2_lines(len);  // 0: a length of the Stockham kernel only
+        p.cw = two ? (p.S > 1 ? pow2_divisor_le(p.S, two) : two) : f.cw[a];
         if (p.S > 1 && gap) {  // a block's columns must be consecutive in memory
             while (p.cw > 1 && (p.Sc % p.cw || inner_lo % p.cw || inner_hi % p.cw)) p.cw >>= 1;
         }
         p.lcw = ilog2i(p.cw);
+        p.lines = p.S > 1 ? O * p.Sc : O;
+        if (two) {
+            const cudaError_t e = fft2_launch(data, p, f.tw[a], inverse, st);
+            if (e != cudaSuccess) return e;
+            continue;
+        }
         p.rs = row_stride(len, p.cw);
         const size_t smem = sizeof(float2) * 2 * (size_t)p.cw * p.rs;
-        const long long blocks = (p.S > 1 ? O * p.Sc : O) / p.cw;
+        const long long blocks = p.lines / p.cw;
         if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
         const bool p2 = (len & (len - 1)) == 0;
         const unsigned nb = (unsigned)blocks;

@@ -48,8 +48,8 @@ cudaError_t grid_fft_exec(const GridFft &f, float2 *data, bool inverse, cudaStre
 // axis a, outputs j < keep_half[a] and j >= n[a] - keep_half[a] (0: all).  Each
 // axis pass (fastest first) transforms only the lines whose faster coordinates
 // are kept and stores only its kept outputs; everything else of `data` is left
-// undefined.
+// undefined.  `batch` (a multiple of f.batch) is the number of grids in `data`.
 cudaError_t grid_fft_exec_cropped(const GridFft &f, float2 *data, bool inverse,
-                                  const int keep_half[3], cudaStream_t st);
+                                  const int keep_half[3], cudaStream_t st, int batch);
 
 }  // namespace imp

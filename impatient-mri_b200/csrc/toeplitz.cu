@@ -744,7 +744,7 @@ cudaError_t ToepSolver::compute_q(const float *kx, const float *ky, const float 
         k_grid_w<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(grid_, kx, ky, kz, t_, nullptr,
                                                              nullptr, cfg_.M, g, tau_, t0_, l);
         T_TRY(cudaGetLastError());
-        T_TRY(grid_fft_exec_cropped(gfq_, grid_, true, crop_of(g).v, st_));
+        T_TRY(grid_fft_exec_cropped(gfq_, grid_, true, crop_of(g).v, st_, 1));
         float2 *qf_l = fast_ ? qf_ : qf_ + (size_t)l * G2_;
         k_q_post<<<gridn(G2_), kVB, 0, st_>>>(grid_, g, n2d, qf_l,
                                              q_out_r ? q_out_r + (size_t)l * G2_ : nullptr,
@@ -794,7 +794,7 @@ cudaError_t ToepSolver::compute_fhd(const float *kx, const float *ky, const floa
                 grid_, kx, ky, kz, t_, kd_r + (size_t)c * cfg_.M, kd_i + (size_t)c * cfg_.M,
                 cfg_.M, g, tau_, t0_, l);
             T_TRY(cudaGetLastError());
-            T_TRY(grid_fft_exec_cropped(gff_, grid_, true, crop_of(g).v, st_));
+            T_TRY(grid_fft_exec_cropped(gff_, grid_, true, crop_of(g).v, st_, 1));
             k_fh_post<<<gridn(N_), kVB, 0, st_>>>(grid_, g, nvd, N_, sens_ + (size_t)c * N_,
                                                  eph_ + (size_t)l * N_, fhd_);
             T_TRY(cudaGetLastError());

@@ -86,3 +86,21 @@ def test_grid_fft_rejects_unsupported(pkg, ctx):
     y = np.zeros(8192, np.float32)
     with pytest.raises(pkg.ImpError, match="UNSUPPORTED"):
         pkg.grid_fft(ctx, y, y.copy(), 1, 1, 8192)
+
+
+# lengths n = R1 R2 of the two-pass register kernel (grid_fft2.cu): smallest, odd
+# radices, both ends of the shared-memory tile, and their neighbours that the
+# Stockham kernel takes (22 = 2 x 11, 34 = 2 x 17)
+@pytest.mark.parametrize("n", [8, 12, 22, 24, 34, 36, 40, 56, 72, 120, 168, 240, 360, 392, 448,
+                               504, 512, 560, 640, 672, 784, 896, 1024])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_two_pass_lengths(pkg, ctx, n, inverse):
+    """Each length as the contiguous axis (a line count that leaves the last block partial),
+    as a strided axis of even and of odd width, and batched."""
+    rng = np.random.default_rng(n)
+    for shape, batch in (((1, 5, n), 3), ((3, n, 6), 1), ((n, 5, 3), 1), ((n, 2, 32), 2)):
+        x = rng.standard_normal((batch, *shape)) + 1j * rng.standard_normal((batch, *shape))
+        x = x.astype(np.complex64)
+        got = run(pkg, ctx, x, shape, batch, inverse, device=True)
+        ref = want(x.astype(np.complex128), inverse)
+        assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < TOL
