@@ -338,11 +338,13 @@ int pow2_divisor_le(long long v, int cap) {
 
 }  // namespace
 
+bool grid_fft_length_ok(int n) { return n >= 1 && n <= kGridFftMaxN && radices_fit(n); }
+
 cudaError_t grid_fft_create(GridFft *f, int n0, int n1, int n2, int batch) {
     grid_fft_destroy(f);
     const int n[3] = {n0, n1, n2};
     for (int a = 0; a < 3; ++a) {
-        if (n[a] < 1 || n[a] > kGridFftMaxN || !radices_fit(n[a])) return cudaErrorInvalidValue;
+        if (!grid_fft_length_ok(n[a])) return cudaErrorInvalidValue;
         f->n[a] = n[a];
     }
     if (batch < 1) return cudaErrorInvalidValue;
@@ -379,7 +381,8 @@ cudaError_t grid_fft_create(GridFft *f, int n0, int n1, int n2, int batch) {
         f->smem[a] = sizeof(float2) * 2 * (size_t)cw * f->rs[a];
         std::vector<float2> h(len);
         for (int j = 0; j < len; ++j) {
-            const double ang = -2.0 * kPiD * (double)j / (double)len;
+            const int e = fft2_lines(len) ? fft2_twiddle_exp(len, j) : j;
+            const double ang = -2.0 * kPiD * (double)e / (double)len;
             h[j] = make_float2((float)std::cos(ang), (float)std::sin(ang));
         }
         cudaError_t e = cudaMalloc(&f->tw[a], sizeof(float2) * len);

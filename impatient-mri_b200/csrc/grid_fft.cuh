@@ -22,7 +22,7 @@ namespace imp {
 struct GridFft {
     int n[3] = {1, 1, 1};  // axis lengths, n[2] fastest (2-D: n[0] = 1)
     int batch = 1;
-    float2 *tw[3] = {nullptr, nullptr, nullptr};  // exp(-2 pi i j / n[a]), j < n[a]
+    float2 *tw[3] = {nullptr, nullptr, nullptr};  // exp(-2 pi i e / n[a]), n[a] entries
     int nfac[3] = {0, 0, 0};
     unsigned char fac[3][24] = {};                // radix sequence per axis
     int cw[3] = {1, 1, 1};                        // lines per block
@@ -33,6 +33,8 @@ struct GridFft {
 };
 
 constexpr int kGridFftMaxN = 4096;
+// Axis lengths that a plan takes: up to kGridFftMaxN, prime factors up to 255.
+bool grid_fft_length_ok(int n);
 
 // Plans a transform of `batch` grids of n0 x n1 x n2 (n2 fastest; pass n0 = 1
 // for 2-D, n0 = n1 = 1 for 1-D).  Allocates the twiddle tables (device

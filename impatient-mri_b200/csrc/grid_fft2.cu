@@ -54,6 +54,7 @@ constexpr size_t smem2(int cw) {
 template <int R1, int R2>
 __global__ void __launch_bounds__(kT2) k_fft2(float2 *__restrict__ data, const AxisArgs p,
                                               const float2 *__restrict__ tw, const bool inv) {
+    // tw[k2 R1 + j1] = w_n^{j1 k2}: the threads of a warp read neighbouring entries
     extern __shared__ float2 sm[];
     constexpr int n = R1 * R2;
     const bool contig = p.S == 1;
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(kT2) k_fft2(float2 *__restrict__ data, const A
         float2 *dst = sm + j1 * s1 + c * sc;
         dst[0] = v[0];
 #pragma unroll
-        for (int q = 1; q < R2; ++q) dst[q * s2] = cmul(v[q], __ldg(&tw[j1 * q]));
+        for (int q = 1; q < R2; ++q) dst[q * s2] = cmul(v[q], __ldg(&tw[q * R1 + j1]));
     }
     __syncthreads();
     for (int it = threadIdx.x; it < R2 * cw; it += blockDim.x) {
@@ -130,6 +131,11 @@ const Entry *entry_of(int n) {
 }  // namespace
 
 int fft2_lines(int n) { return entry_of(n) ? lines_of(n) : 0; }
+
+int fft2_twiddle_exp(int n, int i) {
+    const int r1 = n / entry_of(n)->r2;
+    return (i % r1) * (i / r1);
+}
 
 cudaError_t fft2_setup() {
     for (const Entry &e : kEntries) {

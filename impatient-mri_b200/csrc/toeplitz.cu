@@ -111,89 +111,120 @@ __device__ __forceinline__ float kb_transform(float u, float beta) {
     return 1.f;
 }
 
-// Scatter gridding of one time segment, one warp per sample: each sample's
-// separable KB footprint is added into the ifftshifted position (X + gs/2) mod
-// gs of every cell X it covers (ready for the inverse FFT).  The lanes take the
-// cells of the footprint's two fastest-varying axes (z and y in 3-D, y and x in 2-D; up to
-// 9 x 9 at OS 2), so one atomic instruction of the warp updates a few
-// contiguous runs of the grid instead of 32 scattered cells, and the outer
-// axis is looped.  The per-axis KB weights are computed once per sample into
-// shared memory.
+// Scatter gridding, one warp per sample: each sample's separable KB footprint
+// is added into the ifftshifted position (X + gs/2) mod gs of every cell X it
+// covers (ready for the inverse FFT), for a batch of grids at once: segments
+// [l0, l0 + nl) x coils [0, nc) of dr / di, grid (l - l0) nc + c at
+// `cells` elements each.  A sample's footprint, indices and KB weights are
+// formed once for the (at most two) segments whose Hanning window covers it
+// and for all coils, whose values the lanes load in parallel; one launch per
+// (segment, coil) had recomputed them each time and was too short to fill the
+// GPU (256x256, 16 coils, 13 segments: 208 launches of 14 us).  The lanes take
+// the cells of the footprint's two fastest-varying axes (z and y in 3-D, y and
+// x in 2-D; up to 9 x 9 at OS 2), so one atomic instruction of the warp updates
+// a few contiguous runs of a grid instead of 32 scattered cells, and the outer
+// axis is looped.  Bound by the L2's atomic rate (about 3e12 cells per second).
 constexpr int kGridWarps = 8;
+constexpr int kGridCoils = 32;  // coils per launch at most
 
 __global__ void __launch_bounds__(kGridWarps * 32)
-    k_grid_w(float2 *grid, const float *kx, const float *ky, const float *kz, const float *t,
-             const float *dr, const float *di, int M, GridSpec g, float tau, float t0, int l) {
+    k_grid_w(float2 *grid, size_t cells, const float *kx, const float *ky, const float *kz,
+             const float *t, const float *dr, const float *di, int M, GridSpec g, float tau,
+             float t0, int l0, int nl, int nc) {
     __shared__ float wsh[kGridWarps][3][kMaxTaps];
+    __shared__ float2 vsh[kGridWarps][kGridCoils];
+    if (!(tau > 0.f)) return;  // every window is empty
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float(&ws)[3][kMaxTaps] = wsh[wid];
+    float2(&vs)[kGridCoils] = vsh[wid];
     const float inv_os = 1.0f / g.os;
     // loop axis A, lane axes B (slower) and Cc (faster)
     const int A = g.is3d ? 0 : 2, B = g.is3d ? 1 : 0, Cc = g.is3d ? 2 : 1;
     for (int s = blockIdx.x * kGridWarps + wid; s < M; s += gridDim.x * kGridWarps) {
-        const float h = hanning(__ldg(&t[s]), tau, l, t0);
-        if (h == 0.f) continue;  // warp-uniform: every lane reads the same sample
-        float vr = h, vi = 0.f;
-        if (dr) {
-            vr = h * __ldg(&dr[s]);
-            vi = h * (di ? __ldg(&di[s]) : 0.f);
-            if (vr == 0.f && vi == 0.f) continue;
-        }
-        const float k3[3] = {__ldg(&kx[s]), __ldg(&ky[s]), g.is3d ? __ldg(&kz[s]) : 0.f};
+        // segments around t: every lane reads the same sample, so all of this is warp-uniform
+        const float ts = __ldg(&t[s]);
+        const float xs = (ts - t0) / tau;
+        if (!(xs > (float)l0 - 2.f && xs < (float)(l0 + nl) + 1.f)) continue;
+        const int lf = (int)floorf(xs);
+        const int la = max(l0, lf - 1), lb = min(l0 + nl, lf + 3);
+        bool ready = false;
         int lo[3], cnt[3];
-        float cc[3];
+        for (int l = la; l < lb; ++l) {
+            const float h = hanning(ts, tau, l, t0);
+            if (h == 0.f) continue;
+            __syncwarp();  // the previous segment's values have been read
+            if (dr)
+                for (int c = lane; c < nc; c += 32) {
+                    const size_t i = (size_t)c * M + s;
+                    vs[c] = make_float2(h * __ldg(&dr[i]), h * (di ? __ldg(&di[i]) : 0.f));
+                }
+            else if (lane == 0)
+                vs[0] = make_float2(h, 0.f);
+            if (!ready) {
+                ready = true;
+                const float k3[3] = {__ldg(&kx[s]), __ldg(&ky[s]), g.is3d ? __ldg(&kz[s]) : 0.f};
+                float cc[3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (a == 2 && !g.is3d) {
-                lo[2] = 0;
-                cnt[2] = 1;
-                cc[2] = 0.f;
-                continue;
+                for (int a = 0; a < 3; ++a) {
+                    if (a == 2 && !g.is3d) {
+                        lo[2] = 0;
+                        cnt[2] = 1;
+                        cc[2] = 0.f;
+                        continue;
+                    }
+                    const float c = g.os * (g.kscale * k3[a] + 0.5f * (float)g.img[a]);
+                    const float r = 0.5f * kKW * g.os;
+                    int a0 = (int)ceilf(c - r), a1 = (int)floorf(c + r);
+                    a0 = max(a0, 0);
+                    a1 = min(a1, g.gs[a] - 1);
+                    a1 = min(a1, a0 + kMaxTaps - 1);
+                    lo[a] = a0;
+                    cnt[a] = max(a1 - a0 + 1, 0);
+                    cc[a] = c;
+                }
+                for (int q = lane; q < 3 * kMaxTaps; q += 32) {
+                    const int a = q / kMaxTaps, j = q - a * kMaxTaps;
+                    if (j < cnt[a])
+                        ws[a][j] = (a == 2 && !g.is3d)
+                                       ? 1.f
+                                       : kb_weight(fabsf(cc[a] - (float)(lo[a] + j)) * inv_os,
+                                                   g.beta);
+                }
             }
-            const float c = g.os * (g.kscale * k3[a] + 0.5f * (float)g.img[a]);
-            const float r = 0.5f * kKW * g.os;
-            int a0 = (int)ceilf(c - r), a1 = (int)floorf(c + r);
-            a0 = max(a0, 0);
-            a1 = min(a1, g.gs[a] - 1);
-            a1 = min(a1, a0 + kMaxTaps - 1);
-            lo[a] = a0;
-            cnt[a] = max(a1 - a0 + 1, 0);
-            cc[a] = c;
-        }
-        for (int q = lane; q < 3 * kMaxTaps; q += 32) {
-            const int a = q / kMaxTaps, j = q - a * kMaxTaps;
-            if (j < cnt[a])
-                ws[a][j] = (a == 2 && !g.is3d)
-                               ? 1.f
-                               : kb_weight(fabsf(cc[a] - (float)(lo[a] + j)) * inv_os, g.beta);
-        }
-        __syncwarp();
-        // Shifted index lo + j + gs / 2 of a covered cell is below 2 gs: it wraps
-        // at most once (one conditional subtraction, no division per cell).  The
-        // loop axis steps by a fixed stride and wraps once.
-        const int nbc = cnt[B] * cnt[Cc];
-        int a0 = g.is3d ? lo[A] + g.gs[A] / 2 : 0;
-        if (a0 >= g.gs[A]) a0 -= g.gs[A];
-        const size_t astride = g.is3d ? (size_t)g.gs[1] * g.gs[2] : 0;
-        const size_t awrap = astride * g.gs[A];
-        const int rowlen = g.is3d ? g.gs[2] : g.gs[1];  // stride of axis B
-        for (int p = lane; p < nbc; p += 32) {
-            const int jb = p / cnt[Cc], jc = p - jb * cnt[Cc];
-            const float wbc = ws[B][jb] * ws[Cc][jc];
-            if (wbc == 0.f) continue;
-            int ib = lo[B] + jb + g.gs[B] / 2;
-            if (ib >= g.gs[B]) ib -= g.gs[B];
-            int ic = lo[Cc] + jc + g.gs[Cc] / 2;
-            if (ic >= g.gs[Cc]) ic -= g.gs[Cc];
-            size_t cell = (size_t)a0 * astride + (size_t)ib * rowlen + ic;
-            int ia = a0;
-            for (int ja = 0; ja < cnt[A]; ++ja) {
-                const float ww = wbc * ws[A][ja];
-                if (ww != 0.f) atomicAdd(&grid[cell], make_float2(ww * vr, ww * vi));
-                cell += astride;
-                if (++ia == g.gs[A]) {
-                    ia = 0;
-                    cell -= awrap;
+            __syncwarp();
+            // Shifted index lo + j + gs / 2 of a covered cell is below 2 gs: it wraps
+            // at most once (one conditional subtraction, no division per cell).  The
+            // loop axis steps by a fixed stride and wraps once.
+            float2 *gl = grid + (size_t)(l - l0) * nc * cells;
+            const int nbc = cnt[B] * cnt[Cc];
+            int a0 = g.is3d ? lo[A] + g.gs[A] / 2 : 0;
+            if (a0 >= g.gs[A]) a0 -= g.gs[A];
+            const size_t astride = g.is3d ? (size_t)g.gs[1] * g.gs[2] : 0;
+            const size_t awrap = astride * g.gs[A];
+            const int rowlen = g.is3d ? g.gs[2] : g.gs[1];  // stride of axis B
+            for (int p = lane; p < nbc; p += 32) {
+                const int jb = p / cnt[Cc], jc = p - jb * cnt[Cc];
+                const float wbc = ws[B][jb] * ws[Cc][jc];
+                if (wbc == 0.f) continue;
+                int ib = lo[B] + jb + g.gs[B] / 2;
+                if (ib >= g.gs[B]) ib -= g.gs[B];
+                int ic = lo[Cc] + jc + g.gs[Cc] / 2;
+                if (ic >= g.gs[Cc]) ic -= g.gs[Cc];
+                size_t cell = (size_t)a0 * astride + (size_t)ib * rowlen + ic;
+                int ia = a0;
+                for (int ja = 0; ja < cnt[A]; ++ja) {
+                    const float ww = wbc * ws[A][ja];
+                    if (ww != 0.f)
+                        for (int c = 0; c < nc; ++c) {
+                            const float2 v = vs[c];
+                            atomicAdd(&gl[(size_t)c * cells + cell],
+                                      make_float2(ww * v.x, ww * v.y));
+                        }
+                    cell += astride;
+                    if (++ia == g.gs[A]) {
+                        ia = 0;
+                        cell -= awrap;
+                    }
                 }
             }
         }
@@ -219,49 +250,44 @@ __device__ __forceinline__ void vox_xyz(size_t q, const int nv[3], bool is3d, in
     }
 }
 
-// Value of image voxel (x, y, z) of a gridding problem after the inverse FFT:
-// fftshift, crop of the centre and deapodisation.
-__device__ __forceinline__ float2 grid_image_value(const float2 *A, const GridSpec &g, int x,
-                                                   int y, int z) {
+// Where image voxel (x, y, z) of a gridding problem sits after the inverse FFT
+// (fftshift and crop of the centre), and its deapodisation factor.
+struct GridAt {
+    size_t idx;
+    float s;
+};
+__device__ __forceinline__ GridAt grid_at(const GridSpec &g, int x, int y, int z) {
     const int c[3] = {x, y, z};
-    size_t idx = 0;
+    GridAt r{0, 1.f};
     float kern = 1.f;
     for (int a = 0; a < 3; ++a) {
         const int off = g.gs[a] / 2 - g.img[a] / 2;
         const int j = (c[a] + off + g.gs[a] / 2) % g.gs[a];
-        idx = idx * g.gs[a] + j;
+        r.idx = r.idx * g.gs[a] + j;
         if (a < 2 || g.is3d)
             kern *= kb_transform(((float)c[a] - 0.5f * (float)g.img[a]) / (float)g.img[a], g.beta);
     }
     const float osd = g.is3d ? g.os * g.os * g.os : g.os * g.os;
-    const float s = 1.0f / (kern * osd);
-    const float2 v = A[idx];
-    return make_float2(v.x * s, v.y * s);
+    r.s = 1.0f / (kern * osd);
+    return r;
 }
 
-// Q_l from the inverse-FFT'd grid: optional export in the reference layout and
-// the ifftshifted copy that feeds Qf_l = FFT(ifftshift(Q_l)).
-__global__ void k_q_post(const float2 *A, GridSpec g, NV n2, float2 *fftbuf, float *qr,
-                         float *qi, size_t G2) {
+// Q_l of nl segments from the inverse-FFT'd grids, in the reference layout; a
+// voxel's index and deapodisation (sinh per axis) serve all of them.
+__global__ void k_q_post(const float2 *A, size_t cells, GridSpec g, NV n2, float *qr, float *qi,
+                         size_t G2, int nl) {
     // n2: the 2N grid in voxel axis order
     const int nv[3] = {n2.v[0], n2.v[1], n2.v[2]};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < G2;
          q += (size_t)gridDim.x * blockDim.x) {
         int x, y, z;
         vox_xyz(q, nv, g.is3d, x, y, z);
-        const float2 v = grid_image_value(A, g, x, y, z);
-        if (qr) {
-            qr[q] = v.x;
-            qi[q] = v.y;
+        const GridAt at = grid_at(g, x, y, z);
+        for (int l = 0; l < nl; ++l) {
+            const float2 v = A[(size_t)l * cells + at.idx];
+            qr[(size_t)l * G2 + q] = v.x * at.s;
+            qi[(size_t)l * G2 + q] = v.y * at.s;
         }
-        // ifftshift in voxel axis order
-        size_t o;
-        if (!g.is3d)
-            o = (size_t)((x + nv[0] / 2) % nv[0]) * nv[1] + (y + nv[1] / 2) % nv[1];
-        else
-            o = ((size_t)((y + nv[0] / 2) % nv[0]) * nv[1] + (x + nv[1] / 2) % nv[1]) * nv[2] +
-                (z + nv[2] / 2) % nv[2];
-        fftbuf[o] = v;
     }
 }
 
@@ -283,22 +309,30 @@ __global__ void k_q_shift(const float *qr, const float *qi, NV n2, bool is3d, fl
     }
 }
 
-// F^H d accumulation of one (coil, segment): acc += conj(S_c) e^{+i w tau_l} image.
-__global__ void k_fh_post(const float2 *A, GridSpec g, NV nv3, size_t N,
-                          const float2 *sens_c, const float2 *eph_l, float2 *acc) {
+// F^H d accumulation of a batch of grids, segments [l0, l0 + nl) x nc coils:
+// acc += sum_l e^{+i w tau_l} sum_c conj(S_c) image_{l,c}.
+__global__ void k_fh_post(const float2 *A, size_t cells, GridSpec g, NV nv3, size_t N,
+                          const float2 *sens, const float2 *eph, float2 *acc, int nl, int nc) {
     const int nv[3] = {nv3.v[0], nv3.v[1], nv3.v[2]};
     for (size_t r = blockIdx.x * (size_t)blockDim.x + threadIdx.x; r < N;
          r += (size_t)gridDim.x * blockDim.x) {
         int x, y, z;
         vox_xyz(r, nv, g.is3d, x, y, z);
-        const float2 v = grid_image_value(A, g, x, y, z);
-        const float2 e = eph_l[r];  // exp(-i w tau_l)
-        const float2 ve = cmulc(e, v);
-        const float2 s = sens_c ? sens_c[r] : make_float2(1.f, 0.f);
-        const float2 u = cmulc(s, ve);
+        const GridAt at = grid_at(g, x, y, z);
         float2 a = acc[r];
-        a.x += u.x;
-        a.y += u.y;
+        for (int l = 0; l < nl; ++l) {
+            const float2 *Al = A + (size_t)l * nc * cells + at.idx;
+            float2 u = make_float2(0.f, 0.f);
+#pragma unroll 4
+            for (int c = 0; c < nc; ++c) {
+                const float2 w = cmulc(sens[(size_t)c * N + r], Al[(size_t)c * cells]);
+                u.x += w.x;
+                u.y += w.y;
+            }
+            const float2 ve = cmulc(eph[(size_t)l * N + r], make_float2(u.x * at.s, u.y * at.s));
+            a.x += ve.x;  // eph = exp(-i w tau_l)
+            a.y += ve.y;
+        }
         acc[r] = a;
     }
 }
@@ -609,12 +643,12 @@ void ToepSolver::release() {
     }
     reg_.release();
     void *bufs[] = {sens_, eph_, fm_, qf_, big_, x_, r_, p_, q_, best_, fhd_, w_, dots_,
-                    t_, grid_, qf2_, b1_, tw_};
+                    t_, grid_, qf2_, b1_, tw_, tw_f_};
     for (void *b : bufs)
         if (b) cudaFree(b);
     sens_ = eph_ = qf_ = big_ = x_ = r_ = p_ = q_ = best_ = fhd_ = grid_ = nullptr;
-    qf2_ = b1_ = tw_ = nullptr;
-    fast_ = false;
+    qf2_ = b1_ = tw_ = tw_f_ = nullptr;
+    fast_ = rows_ = false;
     fm_ = w_ = t_ = nullptr;
     dots_ = nullptr;
     grid_cells_ = 0;
@@ -625,7 +659,8 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
                               cudaStream_t st) {
     // Same sizes and stream: keep buffers, FFT plans and (same CG terms) the
     // captured iteration graph; only the per-call inputs are refreshed.
-    const bool same_shape = dots_ && st == st_ && cfg.nx == cfg_.nx && cfg.ny == cfg_.ny &&
+    const bool same_shape = (cfg.q_only ? t_ != nullptr : dots_ != nullptr) && st == st_ &&
+                            cfg.q_only == cfg_.q_only && cfg.nx == cfg_.nx && cfg.ny == cfg_.ny &&
                             cfg.nz == cfg_.nz && cfg.C == cfg_.C && cfg.M == cfg_.M &&
                             (int)cfg.ntime_segs == L_;
     if (same_shape) {
@@ -644,6 +679,8 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
         t0_ = tb[0];
         const int L1 = L_ + 1, C = cfg.C;
         T_TRY(cudaMemcpyAsync(t_, t, sizeof(float) * cfg.M, cudaMemcpyDeviceToDevice, st));
+        launches_ = 0;
+        if (cfg.q_only) return cudaSuccess;
         k_pack_sens_c<<<gridn((size_t)C * N_), kVB, 0, st>>>(sens_, sensi_r, sensi_i,
                                                             (size_t)C * N_);
         k_eph<<<gridn((size_t)L1 * N_), kVB, 0, st>>>(eph_, fm, N_, L1, tau_, t0_);
@@ -684,14 +721,25 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     const int L1 = L_ + 1, C = cfg.C;
     T_TRY(cudaMalloc(&t_, sizeof(float) * cfg.M));
     T_TRY(cudaMemcpyAsync(t_, t, sizeof(float) * cfg.M, cudaMemcpyDeviceToDevice, st));
+    launches_ = 0;
+    if (cfg.q_only) return cudaSuccess;
     T_TRY(cudaMalloc(&sens_, sizeof(float2) * C * N_));
     T_TRY(cudaMalloc(&eph_, sizeof(float2) * L1 * N_));
-    // The pruned FFT engine needs power-of-two image sizes; other sizes (and
-    // IMP_TOEP_PADDED=1) use the zero-padded chain on the grid transform.
+    // 2-D images run on the mixed-radix row engine (sides up to its longest
+    // length), 3-D images of power-of-two sides on the plane engine; other sizes
+    // (and IMP_TOEP_PADDED=1) use the zero-padded chain on the grid transform.
     const char *force_padded = std::getenv("IMP_TOEP_PADDED");
-    fast_ = !(force_padded && force_padded[0] == '1') &&
-            toep_fft_plan(nv[0], is3d ? nv[1] : 1, is3d ? nv[2] : nv[1], C, &fp_);
-    if (fast_) {
+    const bool pruned = !(force_padded && force_padded[0] == '1');
+    rows_ = pruned && !is3d && toep_rows_plan(nv[0], nv[1], C, L1, &rp_);
+    fast_ = pruned && is3d && toep_fft_plan(nv[0], nv[1], nv[2], C, &fp_);
+    if (rows_) {
+        qf_segs_ = (int)std::min<size_t>(
+            L1, std::max<size_t>(1, ((size_t)128 << 20) / (sizeof(float2) * rp_.q_elems())));
+        T_TRY(cudaMalloc(&qf_, sizeof(float2) * rp_.q_elems() * qf_segs_));
+        T_TRY(cudaMalloc(&qf2_, sizeof(float2) * rp_.q_elems() * L1));
+        T_TRY(cudaMalloc(&b1_, sizeof(float2) * rp_.b1_elems()));
+        T_TRY(toep_rows_twiddles(rp_, &tw_, &tw_f_));
+    } else if (fast_) {
         T_TRY(cudaMalloc(&qf_, sizeof(float2) * G2_));  // one segment, before permutation
         T_TRY(cudaMalloc(&qf2_, sizeof(float2) * L1 * G2_));
         T_TRY(cudaMalloc(&b1_, sizeof(float2) * fp_.b1_elems()));
@@ -709,27 +757,40 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     T_TRY(cudaGetLastError());
     // the 2N grid: batched over the coils for the zero-padded chain, single
     // for Qf_l (2-D grids are [n2[0]][n2[1]], 3-D [n2[0]][n2[1]][n2[2]])
-    const int d0 = is3d ? n2[0] : 1, d1 = is3d ? n2[1] : n2[0], d2 = is3d ? n2[2] : n2[1];
-    if (!fast_) T_TRY(grid_fft_create(&gf2_, d0, d1, d2, C));
+    int d0 = is3d ? n2[0] : 1, d1 = is3d ? n2[1] : n2[0], d2 = is3d ? n2[2] : n2[1];
+    if (rows_) {  // the engine's lengths; a doubled side that no grid takes stays refused
+        if (!grid_fft_length_ok(d1) || !grid_fft_length_ok(d2)) return cudaErrorInvalidValue;
+        d1 = 2 * rp_.es;
+        d2 = 2 * rp_.ef;
+    }
+    if (!fast_ && !rows_) T_TRY(grid_fft_create(&gf2_, d0, d1, d2, C));
     T_TRY(grid_fft_create(&gf1_, d0, d1, d2, 1));
     launches_ = 2;
     return set_reg();
 }
 
-cudaError_t ToepSolver::ensure_grid_plan(const GridSpec &g, GridFft *plan) {
+// Plan of one grid and room for `batch` of them.
+cudaError_t ToepSolver::ensure_grid_plan(const GridSpec &g, GridFft *plan, int batch) {
     const int d0 = g.is3d ? g.gs[0] : 1, d1 = g.is3d ? g.gs[1] : g.gs[0];
     const int d2 = g.is3d ? g.gs[2] : g.gs[1];
-    if (plan->tw[0] || plan->tw[1] || plan->tw[2]) {
-        if (plan->n[0] == d0 && plan->n[1] == d1 && plan->n[2] == d2) return cudaSuccess;
-    }
-    T_TRY(grid_fft_create(plan, d0, d1, d2, 1));
-    if (g.cells() > grid_cells_) {
+    const bool planned = plan->tw[0] || plan->tw[1] || plan->tw[2];
+    if (!planned || plan->n[0] != d0 || plan->n[1] != d1 || plan->n[2] != d2)
+        T_TRY(grid_fft_create(plan, d0, d1, d2, 1));
+    const size_t need = g.cells() * batch;
+    if (need > grid_cells_) {
         if (grid_) cudaFree(grid_);
         grid_ = nullptr;
-        T_TRY(cudaMalloc(&grid_, sizeof(float2) * g.cells()));
-        grid_cells_ = g.cells();
+        grid_cells_ = 0;
+        T_TRY(cudaMalloc(&grid_, sizeof(float2) * need));
+        grid_cells_ = need;
     }
     return cudaSuccess;
+}
+
+// Gridding grids per batch: as many as half of the L2 holds (the scatter's
+// atomics, the transform and the crop then stay in L2), at least one.
+static size_t grid_batch(const GridSpec &g) {
+    return std::max<size_t>(1, ((size_t)64 << 20) / (sizeof(float2) * g.cells()));
 }
 
 cudaError_t ToepSolver::compute_q(const float *kx, const float *ky, const float *kz,
@@ -737,30 +798,37 @@ cudaError_t ToepSolver::compute_q(const float *kx, const float *ky, const float 
     const bool is3d = cfg_.nz > 1;
     const int img[3] = {2 * cfg_.nx, 2 * cfg_.ny, is3d ? 2 * cfg_.nz : 1};
     const GridSpec g = grid_spec(img, cfg_.os_q, true, 2.0f);
-    T_TRY(ensure_grid_plan(g, &gfq_));
+    const int nb = (int)std::min<size_t>(grid_batch(g), L_ + 1);
+    T_TRY(ensure_grid_plan(g, &gfq_, nb));
     const NV n2d{{n2[0], n2[1], n2[2]}};
-    for (int l = 0; l <= L_; ++l) {
-        T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells(), st_));
-        k_grid_w<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(grid_, kx, ky, kz, t_, nullptr,
-                                                             nullptr, cfg_.M, g, tau_, t0_, l);
+    for (int l = 0; l <= L_; l += nb) {
+        const int nl = std::min(nb, L_ + 1 - l);
+        T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells() * nl, st_));
+        k_grid_w<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(grid_, g.cells(), kx, ky, kz, t_,
+                                                             nullptr, nullptr, cfg_.M, g, tau_,
+                                                             t0_, l, nl, 1);
         T_TRY(cudaGetLastError());
-        T_TRY(grid_fft_exec_cropped(gfq_, grid_, true, crop_of(g).v, st_, 1));
-        float2 *qf_l = fast_ ? qf_ : qf_ + (size_t)l * G2_;
-        k_q_post<<<gridn(G2_), kVB, 0, st_>>>(grid_, g, n2d, qf_l,
-                                             q_out_r ? q_out_r + (size_t)l * G2_ : nullptr,
-                                             q_out_i ? q_out_i + (size_t)l * G2_ : nullptr, G2_);
+        T_TRY(grid_fft_exec_cropped(gfq_, grid_, true, crop_of(g).v, st_, nl));
+        k_q_post<<<gridn(G2_), kVB, 0, st_>>>(grid_, g.cells(), g, n2d, q_out_r + (size_t)l * G2_,
+                                             q_out_i + (size_t)l * G2_, G2_, nl);
         T_TRY(cudaGetLastError());
-        T_TRY(grid_fft_exec(gf1_, qf_l, false, st_));
-        launches_ += 2 + gfq_.passes() + gf1_.passes();
-        if (fast_) {
-            T_TRY(toep_fft_qf(fp_, qf2_ + (size_t)l * G2_, qf_l, 1.0f / (float)G2_, st_));
-            ++launches_;
-        }
+        launches_ += 2 + gfq_.passes();
     }
     return cudaStreamSynchronize(st_);
 }
 
 cudaError_t ToepSolver::load_q(const float *q_r, const float *q_i) {
+    if (rows_) {
+        for (int l = 0; l <= L_; l += qf_segs_) {
+            const int nl = std::min(qf_segs_, L_ + 1 - l);
+            T_TRY(toep_rows_embed(rp_, qf_, q_r + (size_t)l * G2_, q_i + (size_t)l * G2_, nl, st_));
+            T_TRY(grid_fft_exec_cropped(gf1_, qf_, false, nullptr, st_, nl));
+            T_TRY(toep_rows_qf(rp_, qf2_ + (size_t)l * rp_.q_elems(), qf_,
+                               1.0f / (float)rp_.q_elems(), nl, st_));
+            launches_ += 2 + gf1_.passes();
+        }
+        return cudaStreamSynchronize(st_);
+    }
     const NV n2d{{n2[0], n2[1], n2[2]}};
     for (int l = 0; l <= L_; ++l) {
         float2 *qf_l = fast_ ? qf_ : qf_ + (size_t)l * G2_;
@@ -780,23 +848,27 @@ cudaError_t ToepSolver::load_q(const float *q_r, const float *q_i) {
 cudaError_t ToepSolver::compute_fhd(const float *kx, const float *ky, const float *kz,
                                     const float *kd_r, const float *kd_i, float *fhd_r,
                                     float *fhd_i) {
-    const bool is3d = cfg_.nz > 1;
     const int img[3] = {cfg_.nx, cfg_.ny, cfg_.nz};
     const GridSpec g = grid_spec(img, cfg_.os_fh, false, 1.0f);
-    T_TRY(ensure_grid_plan(g, &gff_));
+    // batches of coils x segments: the coils of a launch share each sample's weights
+    const size_t room = grid_batch(g);
+    const int nc_b = (int)std::min<size_t>(room, std::min(cfg_.C, kGridCoils));
+    const int nl_b = (int)std::min<size_t>(std::max<size_t>(room / nc_b, 1), L_ + 1);
+    T_TRY(ensure_grid_plan(g, &gff_, nc_b * nl_b));
     const NV nvd{{nv[0], nv[1], nv[2]}};
-    (void)is3d;
     T_TRY(cudaMemsetAsync(fhd_, 0, sizeof(float2) * N_, st_));
-    for (int c = 0; c < cfg_.C; ++c)
-        for (int l = 0; l <= L_; ++l) {
-            T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells(), st_));
+    for (int c = 0; c < cfg_.C; c += nc_b)
+        for (int l = 0; l <= L_; l += nl_b) {
+            const int nc = std::min(nc_b, cfg_.C - c), nl = std::min(nl_b, L_ + 1 - l);
+            T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells() * nc * nl, st_));
             k_grid_w<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(
-                grid_, kx, ky, kz, t_, kd_r + (size_t)c * cfg_.M, kd_i + (size_t)c * cfg_.M,
-                cfg_.M, g, tau_, t0_, l);
+                grid_, g.cells(), kx, ky, kz, t_, kd_r + (size_t)c * cfg_.M,
+                kd_i + (size_t)c * cfg_.M, cfg_.M, g, tau_, t0_, l, nl, nc);
             T_TRY(cudaGetLastError());
-            T_TRY(grid_fft_exec_cropped(gff_, grid_, true, crop_of(g).v, st_, 1));
-            k_fh_post<<<gridn(N_), kVB, 0, st_>>>(grid_, g, nvd, N_, sens_ + (size_t)c * N_,
-                                                 eph_ + (size_t)l * N_, fhd_);
+            T_TRY(grid_fft_exec_cropped(gff_, grid_, true, crop_of(g).v, st_, nc * nl));
+            k_fh_post<<<gridn(N_), kVB, 0, st_>>>(grid_, g.cells(), g, nvd, N_,
+                                                 sens_ + (size_t)c * N_, eph_ + (size_t)l * N_,
+                                                 fhd_, nl, nc);
             T_TRY(cudaGetLastError());
             launches_ += 2 + gff_.passes();
         }
@@ -815,6 +887,8 @@ cudaError_t ToepSolver::apply_aha(const float2 *p, float2 *q) {
     const int C = cfg_.C;
     const float scale = 1.0f / (float)G2_;
     const double *dots = dots_;
+    if (rows_)
+        return toep_rows_apply(rp_, q, p, sens_, eph_, b1_, qf2_, done_flag(), tw_, tw_f_, st_);
     if (fast_) {
         const int *done = reinterpret_cast<const int *>(
             reinterpret_cast<const char *>(dots_ + T_SCAL * kTBlocks) + offsetof(TScal, done));
@@ -917,7 +991,7 @@ cudaError_t ToepSolver::solve(const float *fhd_r, const float *fhd_i, float *x_r
     k_t_setup<<<1, 1, 0, st_>>>(dots_, 1.0e-16);  // recon.cu:2112
     T_TRY(cudaGetLastError());
     launches_ += 5;
-    const int iter_launches = 3 * (L_ + 1) + 3 + (reg_.on() ? 1 : 0);  // one CG iteration
+    const int iter_launches = aha_launches() + 3 + (reg_.on() ? 1 : 0);  // one CG iteration
     if (cfg_.use_graphs && !g_iter_) T_TRY(capture_graph(st_, &g_iter_, &ToepSolver::cg_iteration, this));
     for (int tv_i = 0; tv_i < std::max(cfg_.tv ? cfg_.tv_num : 1, 1); ++tv_i) {
         if (tv_i != 0) {
@@ -933,7 +1007,7 @@ cudaError_t ToepSolver::solve(const float *fhd_r, const float *fhd_i, float *x_r
         k_t_init<<<kTBlocks, kVB, 0, st_>>>(r_, p_, fhd_, q_, N, dots_);
         k_t_init_finish<<<1, kVB, 0, st_>>>(dots_);
         T_TRY(cudaGetLastError());
-        launches_ += 3 * (L_ + 1) + 3;
+        launches_ += aha_launches() + 3;
         for (int it = 0; it < cfg_.cg_num; ++it) {
             if (g_iter_)
                 T_TRY(cudaGraphLaunch(g_iter_, st_));
@@ -974,8 +1048,8 @@ cudaError_t ToepSolver::solve_from(const float *fhd_r, const float *fhd_i, float
     k_t_init<<<kTBlocks, kVB, 0, st_>>>(r_, p_, fhd_, q_, N, dots_);
     k_t_init_finish<<<1, kVB, 0, st_>>>(dots_);
     T_TRY(cudaGetLastError());
-    launches_ += 3 * (L_ + 1) + 3;
-    const int iter_launches = 3 * (L_ + 1) + 3 + (reg_.on() ? 1 : 0);
+    launches_ += aha_launches() + 3;
+    const int iter_launches = aha_launches() + 3 + (reg_.on() ? 1 : 0);
     const TScal *S = reinterpret_cast<const TScal *>(dots_ + T_SCAL * kTBlocks);
     int it = 0;
     while (it < max_iter) {
@@ -1123,8 +1197,9 @@ imp_status imp_toeplitz_q(imp_context *ctx, const imp_toeplitz_options *opt, flo
         (s = imp::to_device_staged(ctx, t, num_k, &dt, nullptr)))
         return s;
     imp::ToepSolver &ts = solver_q_of(ctx);
-    IMP_CUDA(ts.setup(toep_cfg_nopen(opt, nx, ny, nz, 1, num_k), dt, nullptr, nullptr, nullptr,
-                      ctx->dev_err, ctx->stream),
+    imp::ToepConfig qcfg = toep_cfg_nopen(opt, nx, ny, nz, 1, num_k);
+    qcfg.q_only = true;
+    IMP_CUDA(ts.setup(qcfg, dt, nullptr, nullptr, nullptr, ctx->dev_err, ctx->stream),
              "toeplitz setup");
     const size_t nq = (size_t)ts.segments() * ts.q_elems();
     float *dqr, *dqi;

@@ -9,6 +9,7 @@
 #include "grid_fft.cuh"
 #include "sparse_reg.cuh"
 #include "toep_fft.cuh"
+#include "toep_rows.cuh"
 
 namespace imp {
 
@@ -42,6 +43,7 @@ struct ToepConfig {
     float tv_eps = 1e-6f;
     bool use_graphs = true;
     const imp_sparse *reg = nullptr;  // -reg roughness matrix (host COO), null = off
+    bool q_only = false;  // compute_q only: no coils, phases, engine or CG buffers
 };
 
 class ToepSolver {
@@ -56,8 +58,8 @@ public:
     cudaError_t setup(const ToepConfig &cfg, const float *t, const float *fm,
                       const float *sensi_r, const float *sensi_i, unsigned *dev_err,
                       cudaStream_t st);
-    // Q_l by gridding (kx, ky, kz device [M]); q_out (optional, device) gets
-    // Q in the reference layout [(L+1)][2N grid] as split re/im.
+    // Q_l by gridding (kx, ky, kz device [M]) into q_out (device), in the
+    // reference layout [(L+1)][2N grid] as split re/im.
     cudaError_t compute_q(const float *kx, const float *ky, const float *kz, float *q_out_r,
                           float *q_out_i);
     // Q_l given (reference layout, split re/im, device).
@@ -87,7 +89,7 @@ private:
     const int *done_flag() const;
     cudaError_t set_reg();
     cudaError_t cg_iteration();
-    cudaError_t ensure_grid_plan(const GridSpec &g, GridFft *plan);
+    cudaError_t ensure_grid_plan(const GridSpec &g, GridFft *plan, int batch);
 
     ToepConfig cfg_;
     SparseReg reg_;            // -reg: C and C^T on the device
@@ -121,7 +123,13 @@ private:
     ToepFftPlan fp_;
     float2 *qf2_ = nullptr;    // [(L+1)][G2] Qf_l in parity-major order, scaled 1/G2
     float2 *b1_ = nullptr;     // [C][half spectrum] engine scratch
-    float2 *tw_ = nullptr;     // twiddle table
+    float2 *tw_ = nullptr;     // twiddle table (rows_: of the slow axis)
+    // 2-D: mixed-radix row engine
+    bool rows_ = false;
+    ToepRowsPlan rp_;
+    int qf_segs_ = 1;          // segments of qf_ scratch
+    float2 *tw_f_ = nullptr;   // twiddle table of the fast axis
+    int aha_launches() const { return rows_ ? rp_.launches() : 3 * (L_ + 1); }
 };
 
 }  // namespace imp

@@ -429,3 +429,34 @@ def test_cli_toeplitz_gridding(pkg, tmp_path):
     print(r.stdout[-2000:], r.stderr[-2000:], file=sys.stderr)
     assert r.returncode == 0
     assert rel(read_pairs(tmp_path / "out.file", c["ix"].size), c["out"]) < TOL_IMG
+
+
+# ------------------------------------------------------------- gridding batches
+
+
+@pytest.mark.parametrize("dims,C,L,M", [((16, 12, 1), 34, 3, 300), ((512, 512, 1), 3, 5, 400),
+                                        ((16, 16, 8), 5, 9, 200)])
+def test_fhd_batches_match_oracle(pkg, ctx, dims, C, L, M):
+    """F^H d whose (segment, coil) grids take several batches: more coils than one launch
+    takes, and grids (1024 x 1024 at oversampling 2) of which a batch holds fewer than the
+    segments x coils."""
+    rng = np.random.default_rng(C + L)
+    nx, ny, nz = dims
+    N = nx * ny * nz
+    c = dict(dims=dims, L=L, cg=1, fdp=1e-2, tv_num=0, os_q=2.0, os_fh=2.0,
+             t=np.sort(rng.uniform(0.0, 0.01, M)).astype(np.float32),
+             kx=rng.uniform(-nx / 2, nx / 2 - 1, M).astype(np.float32),
+             ky=rng.uniform(-ny / 2, ny / 2 - 1, M).astype(np.float32),
+             kz=(rng.uniform(-nz / 2, nz / 2 - 1, M) if nz > 1 else np.zeros(M)).astype(np.float32),
+             fm=rng.uniform(-300.0, 300.0, N).astype(np.float32),
+             sens=(rng.standard_normal((C, N)) + 1j * rng.standard_normal((C, N))).astype(
+                 np.complex64))
+    kd = (rng.standard_normal((C, M)) + 1j * rng.standard_normal((C, M))).astype(np.complex64)
+    c["kdata"] = kd
+    got = gpu_fhd(pkg, ctx, opts_of(pkg, c), c)
+    want = T.compute_fhd(c["kx"], c["ky"], c["kz"], c["t"], dims, L, c["os_fh"], kd, c["sens"],
+                         c["fm"])
+    # FP32 grid coordinates: half an ulp of c < gs moves a sample by up to gs 2^-25 cells,
+    # a phase of pi / os per cell at the image's edge
+    tol = max(TOL_OP, np.pi * max(nx, ny) * 2.0 ** -25)
+    assert rel(got, np.asarray(want).reshape(-1)) < tol
