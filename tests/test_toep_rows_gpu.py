@@ -1,0 +1,65 @@
+"""The 2-D mixed-radix F^H F engine (toep_rows.cu): one A^H A (+ lambda D^H D) application
+against the FP64 oracle over the lengths of its table, the sides between them (which run on the
+next length), uneven coil counts and several segments; refused sizes stay refused."""
+import numpy as np
+import pytest
+
+from test_toeplitz_gpu import TOL_OP, gpu_apply, grid_elems, opts_of, oracle_apply, rel
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(pkg):
+    c = pkg.Context(0)
+    yield c
+    c.close()
+
+
+def make(dims, C, L, seed):
+    rng = np.random.default_rng(seed)
+    nx, ny, nz = dims
+    N, M, G = nx * ny * nz, 64, grid_elems(dims)
+    c = dict(dims=dims, L=L, cg=1, fdp=1e-2, tv_num=0, os_q=2.0, os_fh=1.5,
+             t=np.sort(rng.uniform(0.0, 0.01, M)).astype(np.float32), kx=np.zeros(M, np.float32),
+             fm=rng.uniform(-300.0, 300.0, N).astype(np.float32),
+             sens=(rng.standard_normal((C, N)) + 1j * rng.standard_normal((C, N))).astype(
+                 np.complex64))
+    if C == 1:
+        c["sens"] = np.ones((1, N), np.complex64)
+    cplx = lambda *s: (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+    return c, cplx(L + 1, G), cplx(N)
+
+
+# (x, y): x is the strided (column) axis, y the contiguous (row) axis
+SIZES = [(2, 2), (16, 16), (14, 18), (32, 48), (46, 34), (64, 80), (82, 96), (112, 98), (128, 144),
+         (146, 160), (192, 162), (194, 200), (240, 202), (242, 256), (288, 258), (290, 320),
+         (336, 322), (338, 384), (400, 386), (402, 448), (480, 450), (482, 512), (576, 10),
+         (10, 576), (578, 12), (12, 578), (642, 8), (8, 642), (770, 6), (6, 770), (900, 4), (4, 900),
+         (1024, 2), (2, 1024)]
+
+
+@pytest.mark.parametrize("nx,ny", SIZES)
+def test_lengths_match_oracle(pkg, ctx, nx, ny):
+    c, Q, p = make((nx, ny, 1), 2, 1, nx * 7 + ny)
+    got = gpu_apply(pkg, ctx, opts_of(pkg, c), c, Q, p)
+    assert rel(got, oracle_apply(c, Q, p, c["fdp"])) < TOL_OP
+
+
+@pytest.mark.parametrize("C,L", [(1, 0), (1, 12), (7, 1), (11, 0), (13, 2)])
+def test_coils_and_segments_match_oracle(pkg, ctx, C, L):
+    """Clusters of one rank, of a prime count, and ranks with unequal numbers of transforms."""
+    c, Q, p = make((36, 50, 1), C, L, 100 * C + L)
+    got = gpu_apply(pkg, ctx, opts_of(pkg, c), c, Q, p)
+    assert rel(got, oracle_apply(c, Q, p, c["fdp"])) < TOL_OP
+
+
+def test_sizes_past_the_table(pkg, ctx):
+    """A side longer than the table runs the zero-padded chain; a doubled side with a prime
+    factor above 255 is refused as before."""
+    c, Q, p = make((1040, 4, 1), 2, 0, 5)
+    got = gpu_apply(pkg, ctx, opts_of(pkg, c), c, Q, p)
+    assert rel(got, oracle_apply(c, Q, p, c["fdp"])) < TOL_OP
+    c, Q, p = make((2 * 257, 4, 1), 1, 0, 6)
+    with pytest.raises(pkg.ImpError):
+        gpu_apply(pkg, ctx, opts_of(pkg, c), c, Q, p)
