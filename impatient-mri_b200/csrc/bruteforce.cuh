@@ -114,6 +114,7 @@ private:
     cudaError_t tune_shapes(bool adj);
 
     BfConfig cfg_;
+    unsigned char *img_ = nullptr;  // B operand image of the FP16 tensor-core kernel
     NuPlan plan_;          // C, CG, G, Npad, use_z and the shared sensitivities
     NuLaunch fwd_, adj_;   // one launch shape for all slices
     int S_ = 0, kb_ = 1;   // slices; vector-kernel blocks per slice

@@ -330,6 +330,9 @@ void BfBatch::release() {
     dots_ = nullptr;
     plan_.kgeo = plan_.vgeo = nullptr;  // views of the buffers above
     plan_.sens = nullptr;
+    if (img_) cudaFree(img_);
+    img_ = plan_.img = nullptr;
+    plan_.img_bytes = 0;
     S_ = 0;
 }
 
@@ -380,6 +383,18 @@ cudaError_t BfBatch::setup(const BfConfig &cfg, int S, const int *k_off, const f
     plan_.kgeo = kgeo_;
     plan_.vgeo = vgeo_;
     plan_.sens = sens_;
+    // B operand image of the FP16 tensor-core kernel (without the memory: the TF32 one)
+    if (nu_tc_enabled() && (CG > 8 || nu_tc_forced())) {
+        const size_t need = nu_image_bytes(
+            CG, (size_t)G * std::max<size_t>((size_t)mpad_total_, (size_t)S * Npad));
+        if (cudaMalloc(&img_, need) == cudaSuccess) {
+            plan_.img = img_;
+            plan_.img_bytes = need;
+        } else {
+            cudaGetLastError();
+            img_ = nullptr;
+        }
+    }
     // one launch shape for every slice: the heuristic, replaced by the batch's
     // tuned shape (tune_shapes) when tuning is on
     fwd_ = nu_default_launch(plan_, false);
@@ -496,9 +511,9 @@ cudaError_t BfBatch::tune_shapes(bool adj) {
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     const int max_ours = adj ? Npad : max_mpad_;
     auto run = [&](const NuLaunch &c) {
-        return adj ? nu_partials_batch(plan_, c, true, S_, max_ours, tab_adj_, vgeo_, kgeo_, in,
+        return adj ? nu_partials_batch(plan_, c, true, S_, max_ours, in_elems / CG, tab_adj_, vgeo_, kgeo_, in,
                                        part, err_, st_)
-                   : nu_partials_batch(plan_, c, false, S_, max_ours, tab_fwd_, kgeo_, vgeo_, in,
+                   : nu_partials_batch(plan_, c, false, S_, max_ours, in_elems / CG, tab_fwd_, kgeo_, vgeo_, in,
                                        part, err_, st_);
     };
     float best = 1e30f;
@@ -537,7 +552,7 @@ cudaError_t BfBatch::run_init() {
     const BbSlice *tv = static_cast<const BbSlice *>(tab_vec_);
     k_bb_pack_image<<<dim3(kb_, S_), kVB, 0, st_>>>(xs_, x_, sens_, Npad, CG, G);
     BB_TRY(cudaGetLastError());
-    BB_TRY(nu_partials_batch(plan_, fwd_, false, S_, max_mpad_, tab_fwd_, kgeo_, vgeo_, xs_, pf_,
+    BB_TRY(nu_partials_batch(plan_, fwd_, false, S_, max_mpad_, (size_t)S_ * G * Npad, tab_fwd_, kgeo_, vgeo_, xs_, pf_,
                              err_, st_));
     k_bb_init<<<dim3(kb_, S_), kVB, 0, st_>>>(af_, rpk_, y_, pf_, fwd_.split, tv, plan_.C, CG, G);
     BB_TRY(cudaGetLastError());
@@ -552,14 +567,14 @@ cudaError_t BfBatch::run_iteration() {
     const Grid3 gd{cfg_.n0, cfg_.n1, cfg_.n2};
     const BbSlice *tv = static_cast<const BbSlice *>(tab_vec_);
     const dim3 grid(kb_, S_);
-    BB_TRY(nu_partials_batch(plan_, adj_, true, S_, Npad, tab_adj_, vgeo_, kgeo_, rpk_, pa_, err_,
+    BB_TRY(nu_partials_batch(plan_, adj_, true, S_, Npad, (size_t)mpad_total_ * G, tab_adj_, vgeo_, kgeo_, rpk_, pa_, err_,
                              st_));
     k_bb_grad<<<grid, kVB, 0, st_>>>(g_, pa_, adj_.split * G, plan_.N, Npad, x_, w_, gd,
                                      cfg_.fd ? 1 : 0, cfg_.lambda, dots_, kb_);
     BB_TRY(cudaGetLastError());
     k_bb_dir<<<grid, kVB, 0, st_>>>(d_, xs_, g_, sens_, Npad, CG, G, dots_, kb_);
     BB_TRY(cudaGetLastError());
-    BB_TRY(nu_partials_batch(plan_, fwd_, false, S_, max_mpad_, tab_fwd_, kgeo_, vgeo_, xs_, pf_,
+    BB_TRY(nu_partials_batch(plan_, fwd_, false, S_, max_mpad_, (size_t)S_ * G * Npad, tab_fwd_, kgeo_, vgeo_, xs_, pf_,
                              err_, st_));
     k_bb_q<<<grid, kVB, 0, st_>>>(q_, pf_, fwd_.split, tv, plan_.C, CG, G, dots_, kb_);
     BB_TRY(cudaGetLastError());

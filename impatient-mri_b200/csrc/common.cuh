@@ -23,6 +23,25 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) {
     return (unsigned)__cvta_generic_to_shared(p);
 }
 
+// True in one lane of the (converged) warp, the same one every time.  Code under
+// it stays warp-uniform for the compiler, so that the operands of a single-thread
+// instruction (tcgen05.mma) are formed in uniform registers; under
+// `if (lane == 0)` each is moved there one by one before every instruction.
+__device__ __forceinline__ bool elect_one() {
+    unsigned p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
+
+// A value that is the same in all lanes, known to the compiler as such.
+__device__ __forceinline__ unsigned warp_uniform(unsigned v) {
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
                  : "memory");

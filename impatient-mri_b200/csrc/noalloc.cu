@@ -103,7 +103,7 @@ extern "C" imp_status imp_parallel_ift_noalloc(
     const size_t b_data = up(sizeof(float2) * (size_t)p.G * p.Mpad * p.CG);
     const size_t fixed = b_err + b_kgeo + b_vgeo + b_sens + b_data;
     imp::NuLaunch l = imp::nu_default_launch(p, true);
-    imp::nu_tuned_lookup(p, true, &l);
+    imp::nu_tuned_lookup(p, true, &l);  // never the FP16 kernel: the plan has no image
     // the partial sums must fit what is left: fewer splits if needed
     while (fixed + up(imp::nu_adj_partial_bytes(p, l)) > kNoAllocBytes && l.split > 1) l.split /= 2;
     if (fixed + up(imp::nu_adj_partial_bytes(p, l)) > kNoAllocBytes) {

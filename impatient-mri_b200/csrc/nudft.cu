@@ -373,9 +373,12 @@ cudaError_t launch_cg_pt_batch(const NuPlan &p, int split, int S, int max_ours,
 
 template <bool ADJ>
 cudaError_t launch_nudft_batch(const NuPlan &p, const NuLaunch &l, int S, int max_ours,
-                               const NuSlice *sl, const double4 *ours, const double4 *theirs,
+                               size_t elems, const NuSlice *sl, const double4 *ours, const double4 *theirs,
                                const float2 *tdata, float2 *out, unsigned *err,
                                cudaStream_t st) {
+    if (l.tc == 2)
+        return nu_partials_h_batch(p, l, ADJ, S, max_ours, elems, sl, ours, theirs, tdata, out, err,
+                                   st);
     if (l.tc)
         return nu_partials_tc_batch(p, l, ADJ, S, max_ours, sl, ours, theirs, tdata, out, err,
                                     st);
@@ -400,6 +403,7 @@ cudaError_t launch_nudft_batch(const NuPlan &p, const NuLaunch &l, int S, int ma
 template <bool ADJ>
 cudaError_t launch_nudft(const NuPlan &p, const NuLaunch &l, const float2 *tdata, float2 *out,
                          unsigned *err, cudaStream_t st) {
+    if (l.tc == 2) return nu_partials_h(p, l, ADJ, tdata, out, err, st);
     if (l.tc) return nu_partials_tc(p, l, ADJ, tdata, out, err, st);
     const double4 *ours = ADJ ? p.vgeo : p.kgeo;
     const double4 *theirs = ADJ ? p.kgeo : p.vgeo;
@@ -463,7 +467,7 @@ NuLaunch nu_default_launch(const NuPlan &p, bool adj) {
     const bool simt = nu_shape_supported(p.CG, p.CG >= 8 ? 2 : 4);
     if ((nu_tc_forced() || !simt) && nu_tc_supported(p.CG) && n_ours % nu_tc_rows(p.CG) == 0) {
         // one block per SM: about eight waves of blocks, whole tiles per split
-        l.tc = 1;
+        l.tc = p.img_bytes ? 2 : 1;
         const long blocks = (long)(n_ours / nu_tc_rows(p.CG)) * p.G;
         int split = 1;
         while (blocks * split < 148L * 8 && split < 64 && nu_split_ok(n_theirs, split * 2) &&
@@ -513,9 +517,23 @@ cudaError_t nu_plan_create(NuPlan &p, const float *kx, const float *ky, const fl
     if ((e = cudaMalloc(&p.vgeo, sizeof(double4) * p.Npad)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&p.sens, sizeof(float2) * (size_t)p.G * p.Npad * p.CG)) != cudaSuccess)
         return e;
+    if (p.CG > 8 || nu_tc_forced()) nu_plan_reserve_image(p);
     p.fwd = nu_default_launch(p, false);
     p.adj = nu_default_launch(p, true);
     return pack_geometry(p, kx, ky, kz, t, ix, iy, iz, fm, sensi_r, sensi_i, dev_err, st);
+}
+
+void nu_plan_reserve_image(NuPlan &p) {
+    const size_t need = nu_image_bytes(p.CG, (size_t)p.G * std::max(p.Mpad, p.Npad));
+    if (need <= p.img_bytes || !nu_tc_enabled()) return;
+    if (p.img) cudaFree(p.img);
+    p.img = nullptr;
+    p.img_bytes = 0;
+    if (cudaMalloc(&p.img, need) == cudaSuccess) p.img_bytes = need;
+    else {
+        cudaGetLastError();
+        p.img = nullptr;
+    }
 }
 
 cudaError_t nu_plan_repack(NuPlan &p, const float *kx, const float *ky, const float *kz,
@@ -558,6 +576,9 @@ void nu_plan_destroy(NuPlan &p) {
     if (p.kgeo) cudaFree(p.kgeo);
     if (p.vgeo) cudaFree(p.vgeo);
     if (p.sens) cudaFree(p.sens);
+    if (p.img) cudaFree(p.img);
+    p.img = nullptr;
+    p.img_bytes = 0;
     p.kgeo = nullptr;
     p.vgeo = nullptr;
     p.sens = nullptr;
@@ -594,13 +615,13 @@ cudaError_t nu_adjoint_partials(const NuPlan &p, const NuLaunch &l, const float2
 }
 
 cudaError_t nu_partials_batch(const NuPlan &p, const NuLaunch &l, bool adj, int S, int max_ours,
-                              const NuSlice *d_slices, const double4 *ours,
+                              size_t elems, const NuSlice *d_slices, const double4 *ours,
                               const double4 *theirs, const float2 *tdata, float2 *part,
                               unsigned *dev_err, cudaStream_t st) {
     if (S < 1 || !d_slices) return cudaErrorInvalidValue;
-    return adj ? launch_nudft_batch<true>(p, l, S, max_ours, d_slices, ours, theirs, tdata, part,
+    return adj ? launch_nudft_batch<true>(p, l, S, max_ours, elems, d_slices, ours, theirs, tdata, part,
                                           dev_err, st)
-               : launch_nudft_batch<false>(p, l, S, max_ours, d_slices, ours, theirs, tdata,
+               : launch_nudft_batch<false>(p, l, S, max_ours, elems, d_slices, ours, theirs, tdata,
                                            part, dev_err, st);
 }
 

@@ -26,7 +26,8 @@ struct NuLaunch {
     int pt = 4;     // "ours" elements per thread
     int split = 1;  // partitions of the "theirs" range (partial sums)
     int occ = 4;    // blocks per SM the register budget is sized for (4 or 6)
-    int tc = 0;     // 1: tensor-core kernel (nudft_tc.cu; pt and occ unused)
+    int tc = 0;     // tensor-core kernel (pt and occ unused): 1 TF32 (nudft_tc.cu), 2 FP16
+                    // head / tail (nudft_h.cu, needs the plan's image)
 };
 
 struct NuPlan {
@@ -37,6 +38,9 @@ struct NuPlan {
     double4 *kgeo = nullptr;     // [Mpad]  (kx, ky, kz, t)        turns / s
     double4 *vgeo = nullptr;     // [Npad]  (x, y, z, omega/2pi)   FOV / Hz
     float2 *sens = nullptr;      // [G][Npad][CG] coil sensitivities (zero padded)
+    // B operand image of the FP16 tensor-core kernel (no bytes: that kernel is not used)
+    unsigned char *img = nullptr;
+    size_t img_bytes = 0;
     NuLaunch fwd, adj;
 };
 
@@ -64,6 +68,9 @@ cudaError_t nu_plan_place(NuPlan &p, double4 *kgeo, double4 *vgeo, float2 *sens,
 // Replaces only the field map (per-slice) of an existing plan.
 cudaError_t nu_plan_set_fm(NuPlan &p, const float *fm, unsigned *dev_err, cudaStream_t st);
 void nu_plan_destroy(NuPlan &p);
+// Gives the plan the FP16 tensor-core kernel's image for both directions (of
+// the plan's own sizes).  Without the memory the plan goes on without it.
+void nu_plan_reserve_image(NuPlan &p);
 
 // Heuristic launch shape (replaced by the autotuner when enabled).
 NuLaunch nu_default_launch(const NuPlan &p, bool adj);
@@ -98,9 +105,10 @@ struct NuSlice {
 // S * G); `p` supplies C, CG, G, use_z and the shared sensitivities, `l` the
 // launch shape (its split must cut every slice's "theirs" range into whole
 // tiles).  Per-slice layouts are those of nu_forward_partials /
-// nu_adjoint_partials at the slice's offsets.
+// nu_adjoint_partials at the slice's offsets.  `elems`: "theirs" elements of
+// tdata over all slices and coil groups.
 cudaError_t nu_partials_batch(const NuPlan &p, const NuLaunch &l, bool adj, int S, int max_ours,
-                              const NuSlice *d_slices, const double4 *ours,
+                              size_t elems, const NuSlice *d_slices, const double4 *ours,
                               const double4 *theirs, const float2 *tdata, float2 *part,
                               unsigned *dev_err, cudaStream_t st);
 
@@ -136,6 +144,16 @@ cudaError_t nu_partials_tc_batch(const NuPlan &p, const NuLaunch &l, bool adj, i
                                  int max_ours, const NuSlice *d_slices, const double4 *ours,
                                  const double4 *theirs, const float2 *tdata, float2 *out,
                                  unsigned *dev_err, cudaStream_t st);
+
+// FP16 head / tail tensor-core kernel (nudft_h.cu), same layouts; p.img holds
+// nu_image_bytes of the launch's "theirs" elements (all slices and coil groups).
+size_t nu_image_bytes(int CG, size_t elems);
+cudaError_t nu_partials_h(const NuPlan &p, const NuLaunch &l, bool adj, const float2 *tdata,
+                          float2 *out, unsigned *err, cudaStream_t st);
+cudaError_t nu_partials_h_batch(const NuPlan &p, const NuLaunch &l, bool adj, int S, int max_ours,
+                                size_t elems, const NuSlice *d_slices, const double4 *ours,
+                                const double4 *theirs, const float2 *tdata, float2 *out,
+                                unsigned *err, cudaStream_t st);
 
 // Autotuner (tune.cu): times every supported (pt, occ, split) of one direction
 // and the tensor-core kernel's splits

@@ -6,7 +6,7 @@
 // (split), and the tensor-core kernel at every split -- with CUDA events on
 // the launching stream, and keeps the fastest.
 // Results are cached per shape in memory and persisted as text lines
-//     v2 <adj> <CG> <G> <use_z> <Mpad> <Npad> <pt> <occ> <split> <tc> <ms>
+//     v3 <adj> <CG> <G> <use_z> <Mpad> <Npad> <pt> <occ> <split> <tc> <ms>
 // and, for batched launches (the split only, timed by the batch itself),
 //     b1 <adj> <CG> <G> <use_z> <S> <Npad> <max Mpad> <sum Mpad> <tc> <pt> <occ> <split> <ms>
 // in $IMP_TUNE_CACHE (default ~/.cache/impatient_b200/nudft_tune.txt), so a
@@ -72,7 +72,7 @@ void load_locked() {
             if (ok && split >= 1 && split <= 64) g_bcache[bkey_of(b)] = l;
             continue;
         }
-        if (std::sscanf(line, "v2 %d %d %d %d %d %d %d %d %d %d %lf", &a, &cg, &g, &z, &mp, &np,
+        if (std::sscanf(line, "v3 %d %d %d %d %d %d %d %d %d %d %lf", &a, &cg, &g, &z, &mp, &np,
                         &pt, &occ, &split, &tc, &ms) != 11)
             continue;  // other versions are re-tuned
         NuLaunch l;
@@ -94,7 +94,7 @@ void persist(const Key &k, const NuLaunch &l, double ms) {
         if (path[i] == '/') mkdir(path.substr(0, i).c_str(), 0755);
     FILE *f = std::fopen(path.c_str(), "a");
     if (!f) return;  // the cache is an optimisation; failure to write is not an error
-    std::fprintf(f, "v2 %d %d %d %d %d %d %d %d %d %d %.4f\n", std::get<0>(k), std::get<1>(k),
+    std::fprintf(f, "v3 %d %d %d %d %d %d %d %d %d %d %.4f\n", std::get<0>(k), std::get<1>(k),
                  std::get<2>(k), std::get<3>(k), std::get<4>(k), std::get<5>(k), l.pt, l.occ,
                  l.split, l.tc, ms);
     std::fclose(f);
@@ -170,6 +170,7 @@ bool nu_tuned_lookup(const NuPlan &p, bool adj, NuLaunch *out) {
     auto it = g_cache.find(key_of(p, adj));
     if (it == g_cache.end()) return false;
     if (it->second.tc && !nu_tc_enabled()) return false;
+    if (it->second.tc == 2 && !p.img_bytes) return false;
     *out = it->second;
     return true;
 }
@@ -207,7 +208,7 @@ cudaError_t nu_autotune(const NuPlan &p, bool adj, const float2 *tdata, float2 *
     if (nu_tc_enabled() && nu_tc_supported(p.CG) && n_ours % nu_tc_rows(p.CG) == 0)
         for (int s = 1; s <= kMaxSplit; s *= 2) {
             NuLaunch l;
-            l.tc = 1;
+            l.tc = p.img_bytes ? 2 : 1;
             l.split = s;
             cands.push_back(l);
         }
