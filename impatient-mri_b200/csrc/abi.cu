@@ -47,11 +47,11 @@ imp_status begin(imp_context *ctx) {
 
 // Synchronizes and turns device error bits into a status.
 imp_status finish(imp_context *ctx) {
-    unsigned h = 0;
-    IMP_CUDA(cudaMemcpyAsync(&h, ctx->dev_err, sizeof(unsigned), cudaMemcpyDeviceToHost,
+    IMP_CUDA(cudaMemcpyAsync(ctx->host_err, ctx->dev_err, sizeof(unsigned), cudaMemcpyDeviceToHost,
                              ctx->stream),
              "read error word");
     IMP_CUDA(cudaStreamSynchronize(ctx->stream), "stream synchronize");
+    const unsigned h = *ctx->host_err;
     if (h & imp::DEV_ERR_RANGE)
         return fail(IMP_ERR_RANGE,
                     "input outside the fixed-point phase range (|k| <= 32768 cycles/FOV, "
@@ -100,11 +100,6 @@ imp_status scratch(imp_context *ctx, size_t bytes, void **p) {
     return IMP_OK;
 }
 
-struct PlanGuard {
-    imp::NuPlan p;
-    ~PlanGuard() { imp::nu_plan_destroy(p); }
-};
-
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 imp_status check_op_args(const void *out_r, const void *out_i, const void *in_r,
@@ -120,6 +115,50 @@ imp_status check_op_args(const void *out_r, const void *out_i, const void *in_r,
     return IMP_OK;
 }
 
+// Plan, packed input and partial sums of one operator call, all in the
+// context's grow-only scratch: nothing is allocated from the second call of a
+// size on (three allocations and frees had cost more than a small apply).
+struct OpWork {
+    imp::NuPlan p;
+    imp::NuLaunch l;
+    float2 *packed = nullptr, *part = nullptr;
+};
+
+imp_status op_work(imp_context *ctx, int M, int N, int C, bool use_z, bool adj, OpWork &w) {
+    imp::nu_plan_dims(w.p, M, N, C, use_z);
+    imp::NuPlan &p = w.p;
+    const size_t theirs = (size_t)p.G * (adj ? p.Mpad : p.Npad);
+    size_t image = imp::nu_tc_enabled() ? imp::nu_image_bytes(p.CG, theirs) : 0;
+    for (;;) {
+        p.img_bytes = image;
+        w.l = imp::nu_default_launch(p, adj);
+        imp::nu_tuned_lookup(p, adj, &w.l);
+        if (w.l.tc != 2) p.img_bytes = image = 0;
+        const size_t b_k = align256(sizeof(double4) * (size_t)p.Mpad);
+        const size_t b_v = align256(sizeof(double4) * (size_t)p.Npad);
+        const size_t b_s = adj ? align256(sizeof(float2) * (size_t)p.G * p.Npad * p.CG) : 0;
+        const size_t b_d = align256(sizeof(float2) * theirs * p.CG);
+        const size_t b_p = align256(adj ? imp::nu_adj_partial_bytes(p, w.l)
+                                        : imp::nu_fwd_partial_bytes(p, w.l));
+        void *base = nullptr;
+        const imp_status s = scratch(ctx, b_k + b_v + b_s + b_d + b_p + align256(image), &base);
+        if (s == IMP_ERR_NOMEM && image) {  // the kernel that needs no image
+            cudaGetLastError();
+            image = 0;
+            continue;
+        }
+        if (s != IMP_OK) return s;
+        char *at = (char *)base;
+        p.kgeo = (double4 *)at;
+        p.vgeo = (double4 *)(at += b_k);
+        p.sens = (float2 *)(at += b_v);
+        w.packed = (float2 *)(at += b_s);
+        w.part = (float2 *)(at += b_d);
+        p.img = image ? (unsigned char *)(at + b_p) : nullptr;
+        return IMP_OK;
+    }
+}
+
 imp_status run_forward(imp_context *ctx, float *yr, float *yi, const float *xr, const float *xi,
                        const float *kx, const float *ky, const float *kz, const float *ix,
                        const float *iy, const float *iz, const float *fm, const float *t,
@@ -129,21 +168,14 @@ imp_status run_forward(imp_context *ctx, float *yr, float *yi, const float *xr, 
     if (C <= 0) return fail(IMP_ERR_INVALID_ARG, "num_coil must be > 0");
     if (C > 1 && (!sr || !si)) return fail(IMP_ERR_INVALID_ARG, "sensi needed for num_coil > 1");
     if ((s = begin(ctx)) != IMP_OK) return s;
-    PlanGuard g;
-    IMP_CUDA(imp::nu_plan_create(g.p, kx, ky, kz, t, ix, iy, iz, fm, sr, si, M, N, C,
-                                 use_z != 0, ctx->dev_err, ctx->stream),
-             "plan");
-    imp::nu_tuned_lookup(g.p, false, &g.p.fwd);
-    const size_t xs_b = align256(sizeof(float2) * (size_t)g.p.G * g.p.Npad * g.p.CG);
-    const size_t pf_b = align256(imp::nu_fwd_partial_bytes(g.p, g.p.fwd));
-    void *w = nullptr;
-    if ((s = scratch(ctx, xs_b + pf_b, &w)) != IMP_OK) return s;
-    float2 *xs = (float2 *)w;
-    float2 *pf = (float2 *)((char *)w + xs_b);
-    IMP_CUDA(imp::nu_pack_image_soa(g.p, xr, xi, xs, ctx->stream), "pack image");
-    IMP_CUDA(imp::nu_forward_partials(g.p, g.p.fwd, xs, pf, ctx->dev_err, ctx->stream), "F");
-    IMP_CUDA(imp::nu_forward_finish_soa(g.p, g.p.fwd, pf, yr, yi, ctx->stream), "F finish");
-    ctx->launches = 6;
+    OpWork w;
+    if ((s = op_work(ctx, M, N, C, use_z != 0, false, w)) != IMP_OK) return s;
+    IMP_CUDA(imp::nu_pack_op(w.p, false, kx, ky, kz, t, ix, iy, iz, fm, sr, si, xr, xi, w.packed,
+                             ctx->dev_err, ctx->stream),
+             "pack");
+    IMP_CUDA(imp::nu_forward_partials(w.p, w.l, w.packed, w.part, ctx->dev_err, ctx->stream), "F");
+    IMP_CUDA(imp::nu_forward_finish_soa(w.p, w.l, w.part, yr, yi, ctx->stream), "F finish");
+    ctx->launches = 3;
     return finish(ctx);
 }
 
@@ -156,21 +188,14 @@ imp_status run_adjoint(imp_context *ctx, float *xr, float *xi, const float *dr, 
     if (C <= 0) return fail(IMP_ERR_INVALID_ARG, "num_coil must be > 0");
     if (C > 1 && (!sr || !si)) return fail(IMP_ERR_INVALID_ARG, "sensi needed for num_coil > 1");
     if ((s = begin(ctx)) != IMP_OK) return s;
-    PlanGuard g;
-    IMP_CUDA(imp::nu_plan_create(g.p, kx, ky, kz, t, ix, iy, iz, fm, sr, si, M, N, C,
-                                 use_z != 0, ctx->dev_err, ctx->stream),
-             "plan");
-    imp::nu_tuned_lookup(g.p, true, &g.p.adj);
-    const size_t dp_b = align256(sizeof(float2) * (size_t)g.p.G * g.p.Mpad * g.p.CG);
-    const size_t pa_b = align256(imp::nu_adj_partial_bytes(g.p, g.p.adj));
-    void *w = nullptr;
-    if ((s = scratch(ctx, dp_b + pa_b, &w)) != IMP_OK) return s;
-    float2 *dp = (float2 *)w;
-    float2 *pa = (float2 *)((char *)w + dp_b);
-    IMP_CUDA(imp::nu_pack_kdata(g.p, dr, di, dp, ctx->stream), "pack kdata");
-    IMP_CUDA(imp::nu_adjoint_partials(g.p, g.p.adj, dp, pa, ctx->dev_err, ctx->stream), "F^H");
-    IMP_CUDA(imp::nu_adjoint_finish_soa(g.p, g.p.adj, pa, xr, xi, ctx->stream), "F^H finish");
-    ctx->launches = 6;
+    OpWork w;
+    if ((s = op_work(ctx, M, N, C, use_z != 0, true, w)) != IMP_OK) return s;
+    IMP_CUDA(imp::nu_pack_op(w.p, true, kx, ky, kz, t, ix, iy, iz, fm, sr, si, dr, di, w.packed,
+                             ctx->dev_err, ctx->stream),
+             "pack");
+    IMP_CUDA(imp::nu_adjoint_partials(w.p, w.l, w.packed, w.part, ctx->dev_err, ctx->stream), "F^H");
+    IMP_CUDA(imp::nu_adjoint_finish_soa(w.p, w.l, w.part, xr, xi, ctx->stream), "F^H finish");
+    ctx->launches = 3;
     return finish(ctx);
 }
 
@@ -317,6 +342,11 @@ imp_status imp_context_create(int device, imp_context **out) {
     IMP_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamDefault), "stream");
     IMP_CUDA(cudaMalloc(&c->dev_err, sizeof(unsigned)), "error word");
     IMP_CUDA(cudaMemset(c->dev_err, 0, sizeof(unsigned)), "error word");
+    IMP_CUDA(cudaMallocHost(&c->host_err, sizeof(unsigned)), "error word");
+    // small operator calls then allocate nothing, the first one included
+    const size_t first = (size_t)8 << 20;
+    IMP_CUDA(cudaMalloc(&c->scratch, first), "scratch");
+    c->scratch_bytes = first;
     *out = c.release();
     return IMP_OK;
 }
@@ -333,6 +363,7 @@ imp_status imp_context_destroy(imp_context *ctx) {
     ctx->stage.clear();
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->dev_err) cudaFree(ctx->dev_err);
+    if (ctx->host_err) cudaFreeHost(ctx->host_err);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return IMP_OK;

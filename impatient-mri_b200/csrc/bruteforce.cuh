@@ -114,6 +114,11 @@ private:
     cudaError_t tune_shapes(bool adj);
 
     BfConfig cfg_;
+    cudaError_t place_inputs(const float *kx, const float *ky, const float *kz, const float *t,
+                             const float *ix, const float *iy, const float *iz, const float *fm,
+                             const float *sensi_r, const float *sensi_i);
+    bool ready_ = false;   // set up in full: a like call packs its inputs only
+    int switches_ = 0;     // kernel-choice switches of that set-up
     unsigned char *img_ = nullptr;  // B operand image of the FP16 tensor-core kernel
     NuPlan plan_;          // C, CG, G, Npad, use_z and the shared sensitivities
     NuLaunch fwd_, adj_;   // one launch shape for all slices

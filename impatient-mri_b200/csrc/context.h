@@ -18,6 +18,7 @@ struct imp_context {
     int device = 0;
     cudaStream_t stream = nullptr;
     unsigned *dev_err = nullptr;  // device error word (imp::DEV_ERR_*)
+    unsigned *host_err = nullptr;  // pinned word it is read back into
     long launches = 0;
     void *scratch = nullptr;      // grow-only work memory of the operator calls
     size_t scratch_bytes = 0;

@@ -198,10 +198,9 @@ __global__ void __launch_bounds__(kNT, OCC)
 
 // ------------------------------ packing ------------------------------------
 
-__global__ void k_pack_kgeo(double4 *kgeo, const float *kx, const float *ky, const float *kz,
-                            const float *t, int M, int Mpad, int use_z, unsigned *err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Mpad) return;
+__device__ __forceinline__ double4 kgeo_at(const float *kx, const float *ky, const float *kz,
+                                           const float *t, int i, int M, int use_z,
+                                           unsigned *err) {
     double4 q = make_double4(0.0, 0.0, 0.0, 0.0);
     if (i < M) {
         q.x = (double)kx[i];
@@ -213,13 +212,12 @@ __global__ void k_pack_kgeo(double4 *kgeo, const float *kx, const float *ky, con
               fabs(q.w) <= 16.0))
             atomicOr(err, DEV_ERR_RANGE);
     }
-    kgeo[i] = q;
+    return q;
 }
 
-__global__ void k_pack_vgeo(double4 *vgeo, const float *ix, const float *iy, const float *iz,
-                            const float *fm, int N, int Npad, int use_z, unsigned *err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Npad) return;
+__device__ __forceinline__ double4 vgeo_at(const float *ix, const float *iy, const float *iz,
+                                           const float *fm, int i, int N, int use_z,
+                                           unsigned *err) {
     double4 q = make_double4(0.0, 0.0, 0.0, 0.0);
     if (i < N) {
         q.x = (double)ix[i];
@@ -230,7 +228,19 @@ __global__ void k_pack_vgeo(double4 *vgeo, const float *ix, const float *iy, con
         if (!(fabs(q.x) <= 2.0 && fabs(q.y) <= 2.0 && fabs(q.z) <= 2.0 && fabs(q.w) <= 8192.0))
             atomicOr(err, DEV_ERR_RANGE);
     }
-    vgeo[i] = q;
+    return q;
+}
+
+__global__ void k_pack_kgeo(double4 *kgeo, const float *kx, const float *ky, const float *kz,
+                            const float *t, int M, int Mpad, int use_z, unsigned *err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < Mpad) kgeo[i] = kgeo_at(kx, ky, kz, t, i, M, use_z, err);
+}
+
+__global__ void k_pack_vgeo(double4 *vgeo, const float *ix, const float *iy, const float *iz,
+                            const float *fm, int N, int Npad, int use_z, unsigned *err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < Npad) vgeo[i] = vgeo_at(ix, iy, iz, fm, i, N, use_z, err);
 }
 
 __global__ void k_set_fm(double4 *vgeo, const float *fm, int N, int Npad, unsigned *err) {
@@ -272,17 +282,6 @@ __global__ void k_pack_image(float2 *xs, const float2 *x, const float2 *sens, in
     }
 }
 
-__global__ void k_pack_image_soa(float2 *xs, const float *xr, const float *xi,
-                                 const float2 *sens, int N, int Npad, int CG, int G) {
-    const size_t n = (size_t)G * Npad * CG;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)((i / CG) % Npad);
-        const float2 x = r < N ? make_float2(xr[r], xi[r]) : make_float2(0.f, 0.f);
-        xs[i] = cmul(sens[i], x);
-    }
-}
-
 __global__ void k_pack_kdata(float2 *packed, const float *dr, const float *di, int M, int Mpad,
                              int C, int CG, int G) {
     const size_t n = (size_t)G * Mpad * CG;
@@ -305,6 +304,7 @@ __global__ void k_fwd_finish_soa(float *yr, float *yi, const float2 *part, int M
         const int c = (int)(i / M), k = (int)(i % M);
         const int g = c / CG, cg = c % CG;
         float sr = 0.f, si = 0.f;
+#pragma unroll 8
         for (int s = 0; s < S; ++s) {
             const float2 v = part[(((size_t)s * G + g) * Mpad + k) * CG + cg];
             sr += v.x;
@@ -319,6 +319,7 @@ __global__ void k_adj_finish_soa(float *xr, float *xi, const float2 *part, int N
                                  int SG) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < N; r += gridDim.x * blockDim.x) {
         float sr = 0.f, si = 0.f;
+#pragma unroll 8
         for (int s = 0; s < SG; ++s) {
             const float2 v = part[(size_t)s * Npad + r];
             sr += v.x;
@@ -326,6 +327,64 @@ __global__ void k_adj_finish_soa(float *xr, float *xi, const float2 *part, int N
         }
         xr[r] = sr;
         xi[r] = si;
+    }
+}
+
+// Everything one operator call packs, in one launch (each array alone is a few
+// microseconds of launch and fill): the sample and voxel geometry, then for F
+// xs = S x (the sensitivities themselves are not read again) and for F^H the
+// sensitivities and the k-space data.
+struct PackOp {
+    double4 *kgeo, *vgeo;
+    float2 *sens, *packed;
+    const float *kx, *ky, *kz, *t, *ix, *iy, *iz, *fm, *sr, *si, *in_r, *in_i;
+    int M, N, Mpad, Npad, C, CG, G, use_z;
+    unsigned *err;
+};
+
+__device__ __forceinline__ float2 sens_at(const PackOp &a, int c, int r) {
+    if (c >= a.C || r >= a.N) return make_float2(0.f, 0.f);
+    if (!a.sr) return make_float2(1.f, 0.f);
+    const size_t o = (size_t)c * a.N + r;
+    return make_float2(a.sr[o], a.si ? a.si[o] : 0.f);
+}
+
+template <bool ADJ>
+__global__ void k_pack_op(const PackOp a) {
+    const size_t ns = (size_t)a.G * a.Npad * a.CG, nd = ADJ ? (size_t)a.G * a.Mpad * a.CG : 0;
+    const size_t n = (size_t)a.Mpad + a.Npad + ns + nd;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+         i += (size_t)gridDim.x * blockDim.x) {
+        size_t j = i;
+        if (j < (size_t)a.Mpad) {
+            a.kgeo[j] = kgeo_at(a.kx, a.ky, a.kz, a.t, (int)j, a.M, a.use_z, a.err);
+            continue;
+        }
+        j -= a.Mpad;
+        if (j < (size_t)a.Npad) {
+            a.vgeo[j] = vgeo_at(a.ix, a.iy, a.iz, a.fm, (int)j, a.N, a.use_z, a.err);
+            continue;
+        }
+        j -= a.Npad;
+        const int cg = (int)(j % a.CG);
+        const size_t gr = j / a.CG;
+        if (j < ns) {
+            const int r = (int)(gr % a.Npad);
+            const float2 s = sens_at(a, (int)(gr / a.Npad) * a.CG + cg, r);
+            if (ADJ) {
+                a.sens[j] = s;
+            } else {
+                const float2 x = r < a.N ? make_float2(a.in_r[r], a.in_i[r]) : make_float2(0.f, 0.f);
+                a.packed[j] = cmul(s, x);
+            }
+            continue;
+        }
+        j -= ns;
+        const size_t gk = j / a.CG;
+        const int k = (int)(gk % a.Mpad), c = (int)(gk / a.Mpad) * a.CG + (int)(j % a.CG);
+        const size_t o = (size_t)c * a.M + k;
+        a.packed[j] = (c < a.C && k < a.M) ? make_float2(a.in_r[o], a.in_i[o])
+                                           : make_float2(0.f, 0.f);
     }
 }
 
@@ -482,6 +541,8 @@ NuLaunch nu_default_launch(const NuPlan &p, bool adj) {
     while (blocks * split < target && split < 64 && nu_split_ok(n_theirs, split * 2) &&
            n_theirs / (split * 2) >= 4 * kTile)
         split *= 2;
+    // a problem that leaves SMs without a block splits down to single tiles
+    while (blocks * split < 148L * 4 && split < 64 && nu_split_ok(n_theirs, split * 2)) split *= 2;
     l.split = split;
     return l;
 }
@@ -597,10 +658,18 @@ cudaError_t nu_pack_image(const NuPlan &p, const float2 *x, float2 *xs, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t nu_pack_image_soa(const NuPlan &p, const float *xr, const float *xi, float2 *xs,
-                              cudaStream_t st) {
-    k_pack_image_soa<<<grid_for((size_t)p.G * p.Npad * p.CG), 256, 0, st>>>(
-        xs, xr, xi, p.sens, p.N, p.Npad, p.CG, p.G);
+cudaError_t nu_pack_op(const NuPlan &p, bool adj, const float *kx, const float *ky,
+                       const float *kz, const float *t, const float *ix, const float *iy,
+                       const float *iz, const float *fm, const float *sensi_r,
+                       const float *sensi_i, const float *in_r, const float *in_i, float2 *packed,
+                       unsigned *dev_err, cudaStream_t st) {
+    const PackOp a{p.kgeo, p.vgeo, p.sens,  packed,  kx,   ky,   kz,  t,   ix,  iy,
+                   iz,     fm,     sensi_r, sensi_i, in_r, in_i, p.M, p.N, p.Mpad, p.Npad,
+                   p.C,    p.CG,   p.G,     p.use_z ? 1 : 0, dev_err};
+    const size_t n = (size_t)p.Mpad + p.Npad +
+                     (size_t)p.G * p.CG * (p.Npad + (adj ? (size_t)p.Mpad : 0));
+    if (adj) k_pack_op<true><<<grid_for(n), 256, 0, st>>>(a);
+    else k_pack_op<false><<<grid_for(n), 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 

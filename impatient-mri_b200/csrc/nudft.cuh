@@ -81,9 +81,14 @@ size_t nu_adj_partial_bytes(const NuPlan &p, const NuLaunch &l);
 
 // xs[g][r][cg] = S[g][r][cg] * x[r]   (x interleaved complex, [Npad])
 cudaError_t nu_pack_image(const NuPlan &p, const float2 *x, float2 *xs, cudaStream_t st);
-// Same from SoA x (operator API).
-cudaError_t nu_pack_image_soa(const NuPlan &p, const float *xr, const float *xi, float2 *xs,
-                              cudaStream_t st);
+// Operator calls: geometry (and, adjoint, sensitivities) of a plan whose arrays
+// are placed, and the packed input: xs from SoA x (forward; p.sens is not
+// written) or [G][Mpad][CG] from SoA k-space data (adjoint), one launch.
+cudaError_t nu_pack_op(const NuPlan &p, bool adj, const float *kx, const float *ky,
+                       const float *kz, const float *t, const float *ix, const float *iy,
+                       const float *iz, const float *fm, const float *sensi_r,
+                       const float *sensi_i, const float *in_r, const float *in_i, float2 *packed,
+                       unsigned *dev_err, cudaStream_t st);
 
 // Forward partials: part[split][g][Mpad][CG].
 cudaError_t nu_forward_partials(const NuPlan &p, const NuLaunch &l, const float2 *xs,
