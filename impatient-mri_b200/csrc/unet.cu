@@ -541,6 +541,24 @@ __device__ __forceinline__ uint64_t umma_desc_sw(unsigned saddr, unsigned sbo, u
     return umma_desc(saddr, 16, sbo, layout);
 }
 
+// D (+)= A B, issued by one thread; its commit arrives on `bar` when this and
+// the thread's earlier MMAs are done.
+__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc,
+                                          uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+        "l"(da), "l"(db), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint64_t *bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+            smem_u32(bar))
+        : "memory");
+}
+
 // Swizzle layout code of a tile whose rows hold c BF16 channels (c * 2 bytes).
 __host__ __device__ constexpr unsigned sw_layout(int c) {
     return c == 64 ? 2u : (c == 32 ? 4u : 6u);
@@ -711,7 +729,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(const __grid_constant__ 
     __shared__ uint32_t tmem_sh;
     // Stage tiles start on 1024-byte boundaries (the swizzle pattern's period).
     unsigned char *sm = smraw + ((1024u - (smem_u32(smraw) & 1023u)) & 1023u);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int n_nt = (a.cout + NT - 1) / NT;
     const int n_tiles = n_nt * tiles_x * tiles_y * a.B;
     const int cpt = a.cin / CK;  // channel chunks per tap
@@ -742,7 +760,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(const __grid_constant__ 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_sh;
+    const uint32_t tmem = warp_uniform(tmem_sh);
 
     if (warp == 4) {
         if (lane == 0) {  // TMA producer
@@ -766,49 +784,36 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(const __grid_constant__ 
         }
         __syncwarp();
     } else if (warp == 5) {
-        if (lane == 0) {  // MMA issuer
-            bool ok = true;
-            int g = 0, it = 0;
-            for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
-                const int ab = it & 1;
-                const unsigned au = (unsigned)(it >> 1);
-                // the epilogue has drained this accumulator's previous tile
-                if (it >= 2 && !mbar_wait_tc(&acc_empty[ab], (au - 1) & 1)) ok = false;
+        // MMA issuer: the whole warp runs the loop, one lane issues
+        bool ok = true;
+        int g = 0, it = 0;
+        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
+            const int ab = it & 1;
+            const unsigned au = (unsigned)(it >> 1);
+            // the epilogue has drained this accumulator's previous tile
+            if (it >= 2 && !mbar_wait_tc(&acc_empty[ab], (au - 1) & 1)) ok = false;
+            tc_fence_after();
+            const uint32_t dacc = tmem + (uint32_t)(ab * ACOLS);
+            for (int k = 0; k < nk; ++k, ++g) {
+                const int s = g % S;
+                const unsigned u = (unsigned)(g / S);
+                if (!mbar_wait_tc(&full[s], u & 1)) ok = false;
                 tc_fence_after();
-                const uint32_t dacc = tmem + (uint32_t)(ab * ACOLS);
-                for (int k = 0; k < nk; ++k, ++g) {
-                    const int s = g % S;
-                    const unsigned u = (unsigned)(g / S);
-                    if (!mbar_wait_tc(&full[s], u & 1)) ok = false;
-                    tc_fence_after();
-                    const unsigned sa = smem_u32(sm + s * STAGE);
-                    const unsigned sb = sa + A_BYTES;
+                const unsigned sa = smem_u32(sm + s * STAGE);
+                const unsigned sb = sa + A_BYTES;
+                if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < CK / 16; ++kk) {
-                        const uint64_t da = umma_desc_sw(sa + kk * 32, SBO, LAYOUT);
-                        const uint64_t db = umma_desc_sw(sb + kk * 32, SBO, LAYOUT);
-                        const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\t"
-                            "setp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(
-                                dacc),
-                            "l"(da), "l"(db), "r"(IDESC), "r"(acc)
-                            : "memory");
-                    }
-                    asm volatile(
-                        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
-                        "[%0];" ::"r"(smem_u32(&empty[s]))
-                        : "memory");
+                    for (int kk = 0; kk < CK / 16; ++kk)
+                        umma_bf16(dacc, umma_desc_sw(sa + kk * 32, SBO, LAYOUT),
+                                  umma_desc_sw(sb + kk * 32, SBO, LAYOUT), IDESC,
+                                  (k > 0 || kk > 0) ? 1u : 0u);
+                    umma_commit(&empty[s]);
+                    if (k == nk - 1) umma_commit(&acc_full[ab]);
                 }
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
-                    "[%0];" ::"r"(smem_u32(&acc_full[ab]))
-                    : "memory");
+                __syncwarp();
             }
-            if (!ok && err) atomicOr(err, DEV_ERR_TIMEOUT);
         }
-        __syncwarp();
+        if (!ok && err && lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
     } else {  // epilogue: warp w reads accumulator lanes (rows) 32w .. 32w + 31
         int it = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
@@ -958,7 +963,7 @@ __global__ void __launch_bounds__(kTcThreads) k_wgrad_tc(const __grid_constant__
     __shared__ __align__(8) uint64_t full[S], empty[S], done;
     __shared__ uint32_t tmem_sh;
     unsigned char *sm = smraw + ((1024u - (smem_u32(smraw) & 1023u)) & 1023u);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int u = blockIdx.x;
     const int m0 = (u % n_mt) * kTcM, n0 = ((u / n_mt) % n_nt) * NT;
     const int q0 = (u / (n_mt * n_nt)) * per;
@@ -988,7 +993,7 @@ __global__ void __launch_bounds__(kTcThreads) k_wgrad_tc(const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_sh;
+    const uint32_t tmem = warp_uniform(tmem_sh);
 
     if (warp == 4) {
         if (lane == 0) {  // TMA producer
@@ -1016,39 +1021,27 @@ __global__ void __launch_bounds__(kTcThreads) k_wgrad_tc(const __grid_constant__
         }
         __syncwarp();
     } else if (warp == 5) {
-        if (lane == 0) {  // MMA issuer
-            bool ok = true;
-            for (int k = 0; k < nk; ++k) {
-                const int s = k % S;
-                if (!mbar_wait_tc(&full[s], (unsigned)(k / S) & 1)) ok = false;
-                tc_fence_after();
-                const unsigned sa = smem_u32(sm + s * STAGE);
-                const unsigned sb = sa + A_BYTES;
+        // MMA issuer: the whole warp runs the loop, one lane issues
+        bool ok = true;
+        for (int k = 0; k < nk; ++k) {
+            const int s = k % S;
+            if (!mbar_wait_tc(&full[s], (unsigned)(k / S) & 1)) ok = false;
+            tc_fence_after();
+            const unsigned sa = smem_u32(sm + s * STAGE);
+            const unsigned sb = sa + A_BYTES;
+            if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < kTcM / 16; ++kk) {  // 16 pixel rows per MMA
-                    const uint64_t da = umma_desc(sa + kk * 2 * SBOA, REGA, SBOA, sw_layout(CA));
-                    const uint64_t db = umma_desc(sb + kk * 2 * SBOB, REGB, SBOB, sw_layout(CB));
-                    const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(
-                            tmem),
-                        "l"(da), "l"(db), "r"(IDESC), "r"(acc)
-                        : "memory");
-                }
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
-                    "[%0];" ::"r"(smem_u32(&empty[s]))
-                    : "memory");
+                for (int kk = 0; kk < kTcM / 16; ++kk)  // 16 pixel rows per MMA
+                    umma_bf16(tmem, umma_desc(sa + kk * 2 * SBOA, REGA, SBOA, sw_layout(CA)),
+                              umma_desc(sb + kk * 2 * SBOB, REGB, SBOB, sw_layout(CB)), IDESC,
+                              (k > 0 || kk > 0) ? 1u : 0u);
+                umma_commit(&empty[s]);
             }
-            asm volatile(
-                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                    smem_u32(&done))
-                : "memory");
-            if (!ok && err) atomicOr(err, DEV_ERR_TIMEOUT);
+            __syncwarp();
         }
+        if (elect_one()) umma_commit(&done);
         __syncwarp();
+        if (!ok && err && lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
     } else {  // epilogue: accumulator row r = GEMM row m0 + r
         if (!mbar_wait_tc(&done, 0)) {
             if (err && lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
@@ -1212,7 +1205,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_strip(const __grid_constant
     unsigned char *sm = smraw + ((1024u - (smem_u32(smraw) & 1023u)) & 1023u);
     unsigned char *sw = sm;                 // weights [tap][WTAP]
     unsigned char *sst = sm + 9 * WTAP;     // stages [S][dy][REG]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int n_tiles = strips_x * a.H * a.B;
     auto tile_of = [&](int t) {
         TcTile T;
@@ -1249,7 +1242,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_strip(const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_sh;
+    const uint32_t tmem = warp_uniform(tmem_sh);
 
     if (warp == 4) {
         if (lane == 0) {  // TMA producer: the weights once, then three strips per tile
@@ -1272,50 +1265,37 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_strip(const __grid_constant
         }
         __syncwarp();
     } else if (warp == 5) {
-        if (lane == 0) {  // MMA issuer: nine taps per tile
-            bool ok = mbar_wait_tc(&wbar, 0);
-            int it = 0;
-            for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
-                const int ab = it & 1;
-                const unsigned au = (unsigned)(it >> 1);
-                if (it >= 2 && !mbar_wait_tc(&acc_empty[ab], (au - 1) & 1)) ok = false;
-                const int s = it % S;
-                if (!mbar_wait_tc(&full[s], (unsigned)(it / S) & 1)) ok = false;
-                tc_fence_after();
-                const uint32_t dacc = tmem + (uint32_t)(ab * ACOLS);
-                const unsigned st = smem_u32(sst + s * STAGE);
-                const unsigned sb = smem_u32(sw);
+        // MMA issuer, nine taps per tile: the whole warp runs the loop, one lane issues
+        bool ok = mbar_wait_tc(&wbar, 0);
+        int it = 0;
+        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
+            const int ab = it & 1;
+            const unsigned au = (unsigned)(it >> 1);
+            if (it >= 2 && !mbar_wait_tc(&acc_empty[ab], (au - 1) & 1)) ok = false;
+            const int s = it % S;
+            if (!mbar_wait_tc(&full[s], (unsigned)(it / S) & 1)) ok = false;
+            tc_fence_after();
+            const uint32_t dacc = tmem + (uint32_t)(ab * ACOLS);
+            const unsigned st = smem_u32(sst + s * STAGE);
+            const unsigned sb = smem_u32(sw);
+            if (elect_one()) {
 #pragma unroll
                 for (int tap = 0; tap < 9; ++tap) {
                     // output pixel i reads strip (tap / 3) at row i + tap % 3
                     const unsigned av = st + (tap / 3) * REG + (tap % 3) * ROWB;
                     const unsigned bv = sb + tap * WTAP;
 #pragma unroll
-                    for (int kk = 0; kk < CK / 16; ++kk) {
-                        const uint64_t da = umma_desc_sw(av + kk * 32, SBO, LAYOUT);
-                        const uint64_t db = umma_desc_sw(bv + kk * 32, SBO, LAYOUT);
-                        const uint32_t acc = (tap > 0 || kk > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\t"
-                            "setp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(
-                                dacc),
-                            "l"(da), "l"(db), "r"(IDESC), "r"(acc)
-                            : "memory");
-                    }
+                    for (int kk = 0; kk < CK / 16; ++kk)
+                        umma_bf16(dacc, umma_desc_sw(av + kk * 32, SBO, LAYOUT),
+                                  umma_desc_sw(bv + kk * 32, SBO, LAYOUT), IDESC,
+                                  (tap > 0 || kk > 0) ? 1u : 0u);
                 }
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
-                    "[%0];" ::"r"(smem_u32(&empty[s]))
-                    : "memory");
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
-                    "[%0];" ::"r"(smem_u32(&acc_full[ab]))
-                    : "memory");
+                umma_commit(&empty[s]);
+                umma_commit(&acc_full[ab]);
             }
-            if (!ok && err) atomicOr(err, DEV_ERR_TIMEOUT);
+            __syncwarp();
         }
-        __syncwarp();
+        if (!ok && err && lane == 0) atomicOr(err, DEV_ERR_TIMEOUT);
     } else {  // epilogue
         int it = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++it) {
