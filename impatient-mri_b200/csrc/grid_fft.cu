@@ -404,19 +404,20 @@ void grid_fft_destroy(GridFft *f) {
 }
 
 cudaError_t grid_fft_exec(const GridFft &f, float2 *data, bool inverse, cudaStream_t st) {
-    return grid_fft_exec_cropped(f, data, inverse, nullptr, st, f.batch);
+    return grid_fft_exec_cropped(f, data, inverse, nullptr, nullptr, st, f.batch);
 }
 
 cudaError_t grid_fft_exec_cropped(const GridFft &f, float2 *data, bool inverse,
-                                  const int keep_half[3], cudaStream_t st, int batch) {
+                                  const int keep_lo[3], const int keep_hi[3], cudaStream_t st,
+                                  int batch) {
     if (batch < 1 || batch % f.batch) return cudaErrorInvalidValue;
     // kept output range per axis: [0, lo) and [n - hi, n)
     int klo[3], khi[3];
     for (int a = 0; a < 3; ++a) {
-        const int h = keep_half ? keep_half[a] : 0;
-        if (h > 0 && 2 * h <= f.n[a]) {
-            klo[a] = h;
-            khi[a] = h;
+        const int lo = keep_lo ? keep_lo[a] : 0, hi = keep_hi ? keep_hi[a] : 0;
+        if (lo > 0 && hi > 0 && lo + hi <= f.n[a]) {
+            klo[a] = lo;
+            khi[a] = hi;
         } else {
             klo[a] = f.n[a];
             khi[a] = 0;

@@ -47,11 +47,12 @@ void grid_fft_destroy(GridFft *f);
 cudaError_t grid_fft_exec(const GridFft &f, float2 *data, bool inverse, cudaStream_t st);
 
 // The same transform when only a crop of the output is read afterwards: along
-// axis a, outputs j < keep_half[a] and j >= n[a] - keep_half[a] (0: all).  Each
+// axis a, outputs j < keep_lo[a] and j >= n[a] - keep_hi[a] (either 0: all).  Each
 // axis pass (fastest first) transforms only the lines whose faster coordinates
 // are kept and stores only its kept outputs; everything else of `data` is left
 // undefined.  `batch` (a multiple of f.batch) is the number of grids in `data`.
 cudaError_t grid_fft_exec_cropped(const GridFft &f, float2 *data, bool inverse,
-                                  const int keep_half[3], cudaStream_t st, int batch);
+                                  const int keep_lo[3], const int keep_hi[3], cudaStream_t st,
+                                  int batch);
 
 }  // namespace imp

@@ -115,7 +115,9 @@ __device__ __forceinline__ float kb_transform(float u, float beta) {
 // is added into the ifftshifted position (X + gs/2) mod gs of every cell X it
 // covers (ready for the inverse FFT), for a batch of grids at once: segments
 // [l0, l0 + nl) x coils [0, nc) of dr / di, grid (l - l0) nc + c at
-// `cells` elements each.  A sample's footprint, indices and KB weights are
+// `cells` elements each.  Without data (Q: the samples' real window values) a
+// grid holds two segments, 2 m in the real and 2 m + 1 in the imaginary part
+// (l0 even, nc 1, L1 segments in all).  A sample's footprint, indices and KB weights are
 // formed once for the (at most two) segments whose Hanning window covers it
 // and for all coils, whose values the lanes load in parallel; one launch per
 // (segment, coil) had recomputed them each time and was too short to fill the
@@ -123,14 +125,15 @@ __device__ __forceinline__ float kb_transform(float u, float beta) {
 // the cells of the footprint's two fastest-varying axes (z and y in 3-D, y and
 // x in 2-D; up to 9 x 9 at OS 2), so one atomic instruction of the warp updates
 // a few contiguous runs of a grid instead of 32 scattered cells, and the outer
-// axis is looped.  Bound by the L2's atomic rate (about 3e12 cells per second).
+// axis is looped.  Bound by the L2's rate of atomic sector updates (about 5e11
+// cells per second).
 constexpr int kGridWarps = 8;
 constexpr int kGridCoils = 32;  // coils per launch at most
 
 __global__ void __launch_bounds__(kGridWarps * 32)
     k_grid_w(float2 *grid, size_t cells, const float *kx, const float *ky, const float *kz,
              const float *t, const float *dr, const float *di, int M, GridSpec g, float tau,
-             float t0, int l0, int nl, int nc) {
+             float t0, int l0, int nl, int nc, int L1) {
     __shared__ float wsh[kGridWarps][3][kMaxTaps];
     __shared__ float2 vsh[kGridWarps][kGridCoils];
     if (!(tau > 0.f)) return;  // every window is empty
@@ -146,12 +149,15 @@ __global__ void __launch_bounds__(kGridWarps * 32)
         const float xs = (ts - t0) / tau;
         if (!(xs > (float)l0 - 2.f && xs < (float)(l0 + nl) + 1.f)) continue;
         const int lf = (int)floorf(xs);
-        const int la = max(l0, lf - 1), lb = min(l0 + nl, lf + 3);
+        // Q: step m stands for the segments 2 m and 2 m + 1 (real and imaginary part)
+        const int la = dr ? max(l0, lf - 1) : max(l0, lf - 1) >> 1;
+        const int lb = dr ? min(l0 + nl, lf + 3) : (min(l0 + nl, lf + 3) + 1) >> 1;
         bool ready = false;
         int lo[3], cnt[3];
         for (int l = la; l < lb; ++l) {
-            const float h = hanning(ts, tau, l, t0);
-            if (h == 0.f) continue;
+            const float h = hanning(ts, tau, dr ? l : 2 * l, t0);
+            const float h1 = !dr && 2 * l + 1 < L1 ? hanning(ts, tau, 2 * l + 1, t0) : 0.f;
+            if (h == 0.f && h1 == 0.f) continue;
             __syncwarp();  // the previous segment's values have been read
             if (dr)
                 for (int c = lane; c < nc; c += 32) {
@@ -159,7 +165,7 @@ __global__ void __launch_bounds__(kGridWarps * 32)
                     vs[c] = make_float2(h * __ldg(&dr[i]), h * (di ? __ldg(&di[i]) : 0.f));
                 }
             else if (lane == 0)
-                vs[0] = make_float2(h, 0.f);
+                vs[0] = make_float2(h, h1);
             if (!ready) {
                 ready = true;
                 const float k3[3] = {__ldg(&kx[s]), __ldg(&ky[s]), g.is3d ? __ldg(&kz[s]) : 0.f};
@@ -194,8 +200,10 @@ __global__ void __launch_bounds__(kGridWarps * 32)
             __syncwarp();
             // Shifted index lo + j + gs / 2 of a covered cell is below 2 gs: it wraps
             // at most once (one conditional subtraction, no division per cell).  The
-            // loop axis steps by a fixed stride and wraps once.
-            float2 *gl = grid + (size_t)(l - l0) * nc * cells;
+            // loop axis steps by a fixed stride and wraps once.  (Aligned pairs of
+            // cells as 16-byte atomics measured no faster: 5.32 against 5.22 ms for Q of
+            // 128x128x32 when a grid held one segment.)
+            float2 *gl = grid + (size_t)(l - (dr ? l0 : l0 >> 1)) * nc * cells;
             const int nbc = cnt[B] * cnt[Cc];
             int a0 = g.is3d ? lo[A] + g.gs[A] / 2 : 0;
             if (a0 >= g.gs[A]) a0 -= g.gs[A];
@@ -236,34 +244,51 @@ struct NV {
     int v[3];
 };
 
-// Voxel coordinates (x, y, z) of a voxel-order index (2-D [x][y], 3-D [y][x][z]).
-__device__ __forceinline__ void vox_xyz(size_t q, const int nv[3], bool is3d, int &x, int &y,
-                                        int &z) {
+// Voxel coordinates (x, y, z) of a voxel-order index (2-D [x][y], 3-D
+// [y][x][z]); indices below 2^32 with 32-bit divisions, which cost a fraction
+// of a 64-bit one.
+template <typename U>
+__device__ __forceinline__ void vox_xyz_u(U q, const int nv[3], bool is3d, int &x, int &y, int &z) {
     if (!is3d) {
-        x = (int)(q / nv[1]);
-        y = (int)(q % nv[1]);
+        const U c = q / (unsigned)nv[1];
+        x = (int)c;
+        y = (int)(q - c * (unsigned)nv[1]);
         z = 0;
     } else {
-        z = (int)(q % nv[2]);
-        x = (int)((q / nv[2]) % nv[1]);
-        y = (int)(q / ((size_t)nv[2] * nv[1]));
+        const U yx = q / (unsigned)nv[2], r = yx / (unsigned)nv[1];
+        z = (int)(q - yx * (unsigned)nv[2]);
+        y = (int)r;
+        x = (int)(yx - r * (unsigned)nv[1]);
     }
+}
+__device__ __forceinline__ void vox_xyz(size_t q, const int nv[3], bool is3d, int &x, int &y,
+                                        int &z) {
+    if (q >> 32) vox_xyz_u<unsigned long long>(q, nv, is3d, x, y, z);
+    else vox_xyz_u<unsigned>((unsigned)q, nv, is3d, x, y, z);
+}
+
+// (i + n / 2) mod n of an even n, i < n
+__device__ __forceinline__ int half_turn(int i, int n) {
+    return i < n / 2 ? i + n / 2 : i - n / 2;
 }
 
 // Where image voxel (x, y, z) of a gridding problem sits after the inverse FFT
-// (fftshift and crop of the centre), and its deapodisation factor.
+// (fftshift and crop of the centre), where its negative does, and its
+// deapodisation factor.
 struct GridAt {
-    size_t idx;
+    size_t idx, neg;
     float s;
 };
 __device__ __forceinline__ GridAt grid_at(const GridSpec &g, int x, int y, int z) {
     const int c[3] = {x, y, z};
-    GridAt r{0, 1.f};
+    GridAt r{0, 0, 1.f};
     float kern = 1.f;
     for (int a = 0; a < 3; ++a) {
-        const int off = g.gs[a] / 2 - g.img[a] / 2;
-        const int j = (c[a] + off + g.gs[a] / 2) % g.gs[a];
+        // c + gs/2 - img/2 + gs/2, below 2 gs
+        int j = c[a] + 2 * (g.gs[a] / 2) - g.img[a] / 2;
+        if (j >= g.gs[a]) j -= g.gs[a];
         r.idx = r.idx * g.gs[a] + j;
+        r.neg = r.neg * g.gs[a] + (j ? g.gs[a] - j : 0);
         if (a < 2 || g.is3d)
             kern *= kb_transform(((float)c[a] - 0.5f * (float)g.img[a]) / (float)g.img[a], g.beta);
     }
@@ -272,8 +297,11 @@ __device__ __forceinline__ GridAt grid_at(const GridSpec &g, int x, int y, int z
     return r;
 }
 
-// Q_l of nl segments from the inverse-FFT'd grids, in the reference layout; a
-// voxel's index and deapodisation (sinh per axis) serve all of them.
+// Q_l of nl segments from the inverse-FFT'd grids of two segments each, in the
+// reference layout.  The gridded windows are real, so each segment's transform
+// F is Hermitian and G = F_0 + i F_1 separates into F_0 = (G(r) + conj G(-r)) / 2
+// and F_1 = (G(r) - conj G(-r)) / 2i: half the transforms and scatters.  A
+// voxel's indices and deapodisation (sinh per axis) serve all segments.
 __global__ void k_q_post(const float2 *A, size_t cells, GridSpec g, NV n2, float *qr, float *qi,
                          size_t G2, int nl) {
     // n2: the 2N grid in voxel axis order
@@ -283,10 +311,16 @@ __global__ void k_q_post(const float2 *A, size_t cells, GridSpec g, NV n2, float
         int x, y, z;
         vox_xyz(q, nv, g.is3d, x, y, z);
         const GridAt at = grid_at(g, x, y, z);
-        for (int l = 0; l < nl; ++l) {
-            const float2 v = A[(size_t)l * cells + at.idx];
-            qr[(size_t)l * G2 + q] = v.x * at.s;
-            qi[(size_t)l * G2 + q] = v.y * at.s;
+        const float s = 0.5f * at.s;
+        for (int l = 0; l < nl; l += 2) {
+            const float2 *Al = A + (size_t)(l >> 1) * cells;
+            const float2 v = Al[at.idx], m = Al[at.neg];
+            qr[(size_t)l * G2 + q] = (v.x + m.x) * s;
+            qi[(size_t)l * G2 + q] = (v.y - m.y) * s;
+            if (l + 1 < nl) {
+                qr[(size_t)(l + 1) * G2 + q] = (v.y + m.y) * s;
+                qi[(size_t)(l + 1) * G2 + q] = (m.x - v.x) * s;
+            }
         }
     }
 }
@@ -301,10 +335,10 @@ __global__ void k_q_shift(const float *qr, const float *qi, NV n2, bool is3d, fl
         vox_xyz(q, nv, is3d, x, y, z);
         size_t o;
         if (!is3d)
-            o = (size_t)((x + nv[0] / 2) % nv[0]) * nv[1] + (y + nv[1] / 2) % nv[1];
+            o = (size_t)half_turn(x, nv[0]) * nv[1] + half_turn(y, nv[1]);
         else
-            o = ((size_t)((y + nv[0] / 2) % nv[0]) * nv[1] + (x + nv[1] / 2) % nv[1]) * nv[2] +
-                (z + nv[2] / 2) % nv[2];
+            o = ((size_t)half_turn(y, nv[0]) * nv[1] + half_turn(x, nv[1])) * nv[2] +
+                half_turn(z, nv[2]);
         fftbuf[o] = make_float2(qr[q], qi[q]);
     }
 }
@@ -594,11 +628,19 @@ float beatty_beta(float os) {
 // gridding grid, as half-lengths per FFT axis (grid_image_value: along each
 // axis the image's img/2 cells on either side of index 0).
 struct Crop {
-    int v[3];
+    int lo[3], hi[3];
 };
-static Crop crop_of(const GridSpec &g) {
-    if (g.is3d) return Crop{{g.img[0] / 2, g.img[1] / 2, g.img[2] / 2}};
-    return Crop{{0, g.img[0] / 2, g.img[1] / 2}};
+// negatives: the crop's negatives are read too (index img/2 joins; eight, so
+// that the kept runs stay multiples of the transform's column groups).
+static Crop crop_of(const GridSpec &g, bool negatives) {
+    Crop c{{0, 0, 0}, {0, 0, 0}};
+    const int first = g.is3d ? 0 : 1;
+    for (int a = first; a < 3; ++a) {
+        const int h = g.img[a - first] / 2;
+        c.lo[a] = negatives ? h + 8 : h;
+        c.hi[a] = h;
+    }
+    return c;
 }
 
 // Blocks of the warp-per-sample gridding: resident blocks of 8 warps on every
@@ -798,17 +840,19 @@ cudaError_t ToepSolver::compute_q(const float *kx, const float *ky, const float 
     const bool is3d = cfg_.nz > 1;
     const int img[3] = {2 * cfg_.nx, 2 * cfg_.ny, is3d ? 2 * cfg_.nz : 1};
     const GridSpec g = grid_spec(img, cfg_.os_q, true, 2.0f);
-    const int nb = (int)std::min<size_t>(grid_batch(g), L_ + 1);
+    // two segments per grid
+    const int nb = (int)std::min<size_t>(grid_batch(g), L_ / 2 + 1);
     T_TRY(ensure_grid_plan(g, &gfq_, nb));
     const NV n2d{{n2[0], n2[1], n2[2]}};
-    for (int l = 0; l <= L_; l += nb) {
-        const int nl = std::min(nb, L_ + 1 - l);
-        T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells() * nl, st_));
+    const Crop crop = crop_of(g, true);
+    for (int l = 0; l <= L_; l += 2 * nb) {
+        const int nl = std::min(2 * nb, L_ + 1 - l), ng = (nl + 1) / 2;
+        T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells() * ng, st_));
         k_grid_w<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(grid_, g.cells(), kx, ky, kz, t_,
                                                              nullptr, nullptr, cfg_.M, g, tau_,
-                                                             t0_, l, nl, 1);
+                                                             t0_, l, nl, 1, L_ + 1);
         T_TRY(cudaGetLastError());
-        T_TRY(grid_fft_exec_cropped(gfq_, grid_, true, crop_of(g).v, st_, nl));
+        T_TRY(grid_fft_exec_cropped(gfq_, grid_, true, crop.lo, crop.hi, st_, ng));
         k_q_post<<<gridn(G2_), kVB, 0, st_>>>(grid_, g.cells(), g, n2d, q_out_r + (size_t)l * G2_,
                                              q_out_i + (size_t)l * G2_, G2_, nl);
         T_TRY(cudaGetLastError());
@@ -822,7 +866,7 @@ cudaError_t ToepSolver::load_q(const float *q_r, const float *q_i) {
         for (int l = 0; l <= L_; l += qf_segs_) {
             const int nl = std::min(qf_segs_, L_ + 1 - l);
             T_TRY(toep_rows_embed(rp_, qf_, q_r + (size_t)l * G2_, q_i + (size_t)l * G2_, nl, st_));
-            T_TRY(grid_fft_exec_cropped(gf1_, qf_, false, nullptr, st_, nl));
+            T_TRY(grid_fft_exec_cropped(gf1_, qf_, false, nullptr, nullptr, st_, nl));
             T_TRY(toep_rows_qf(rp_, qf2_ + (size_t)l * rp_.q_elems(), qf_,
                                1.0f / (float)rp_.q_elems(), nl, st_));
             launches_ += 2 + gf1_.passes();
@@ -856,6 +900,7 @@ cudaError_t ToepSolver::compute_fhd(const float *kx, const float *ky, const floa
     const int nl_b = (int)std::min<size_t>(std::max<size_t>(room / nc_b, 1), L_ + 1);
     T_TRY(ensure_grid_plan(g, &gff_, nc_b * nl_b));
     const NV nvd{{nv[0], nv[1], nv[2]}};
+    const Crop crop = crop_of(g, false);
     T_TRY(cudaMemsetAsync(fhd_, 0, sizeof(float2) * N_, st_));
     for (int c = 0; c < cfg_.C; c += nc_b)
         for (int l = 0; l <= L_; l += nl_b) {
@@ -863,9 +908,9 @@ cudaError_t ToepSolver::compute_fhd(const float *kx, const float *ky, const floa
             T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells() * nc * nl, st_));
             k_grid_w<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(
                 grid_, g.cells(), kx, ky, kz, t_, kd_r + (size_t)c * cfg_.M,
-                kd_i + (size_t)c * cfg_.M, cfg_.M, g, tau_, t0_, l, nl, nc);
+                kd_i + (size_t)c * cfg_.M, cfg_.M, g, tau_, t0_, l, nl, nc, L_ + 1);
             T_TRY(cudaGetLastError());
-            T_TRY(grid_fft_exec_cropped(gff_, grid_, true, crop_of(g).v, st_, nc * nl));
+            T_TRY(grid_fft_exec_cropped(gff_, grid_, true, crop.lo, crop.hi, st_, nc * nl));
             k_fh_post<<<gridn(N_), kVB, 0, st_>>>(grid_, g.cells(), g, nvd, N_,
                                                  sens_ + (size_t)c * N_, eph_ + (size_t)l * N_,
                                                  fhd_, nl, nc);

@@ -460,3 +460,23 @@ def test_fhd_batches_match_oracle(pkg, ctx, dims, C, L, M):
     # a phase of pi / os per cell at the image's edge
     tol = max(TOL_OP, np.pi * max(nx, ny) * 2.0 ** -25)
     assert rel(got, np.asarray(want).reshape(-1)) < tol
+
+
+@pytest.mark.parametrize("dims,L,os", [((24, 20, 1), 0, 1.0), ((24, 20, 1), 1, 1.5),
+                                       ((16, 40, 1), 6, 2.0), ((10, 14, 6), 3, 1.25),
+                                       ((16, 16, 8), 2, 1.5), ((8, 8, 2), 1, 2.0)])
+def test_q_segment_pairs_match_oracle(pkg, ctx, dims, L, os):
+    """Q with odd and even segment counts (two real segments share a grid; the last may be
+    alone), uncropped (oversampling 1) and cropped transforms."""
+    rng = np.random.default_rng(L + dims[0])
+    nx, ny, nz = dims
+    M = 300
+    c = dict(dims=dims, L=L, cg=1, fdp=1e-2, tv_num=0, os_q=os, os_fh=1.5,
+             t=np.sort(rng.uniform(0.0, 0.01, M)).astype(np.float32),
+             kx=rng.uniform(-nx / 2, nx / 2 - 0.1, M).astype(np.float32),
+             ky=rng.uniform(-ny / 2, ny / 2 - 0.1, M).astype(np.float32),
+             kz=(rng.uniform(-nz / 2, nz / 2 - 0.1, M) if nz > 1 else np.zeros(M)).astype(np.float32))
+    got = gpu_q(pkg, ctx, opts_of(pkg, c), c)
+    want = np.asarray(T.compute_q(c["kx"], c["ky"], c["kz"], c["t"], dims, L, os))
+    for l in range(L + 1):
+        assert rel(got.reshape(L + 1, -1)[l], want.reshape(L + 1, -1)[l]) < 2 * TOL_OP
