@@ -40,7 +40,7 @@ struct ConvArgs {
     bf16 *y;                // BF16 output or null
     int ldy, yoff;
     float *yf;              // FP32 output or null
-    int ldyf, yfoff, accumulate;
+    int ldyf, yfoff;
     int B, H, W, cin, cout, ks, relu;
     int up2;                // BF16 output written to the 2 x 2 block of an image of size 2H x 2W
 };
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kCT) k_conv_fwd(ConvArgs a) {
         if (a.y) a.y[(size_t)p * a.ldy + a.yoff + co] = __float2bfloat16(v);
         if (a.yf) {
             float *d = a.yf + (size_t)p * a.ldyf + a.yfoff + co;
-            *d = a.accumulate ? *d + v : v;
+            *d = v;
         }
     }
 }
@@ -285,38 +285,24 @@ __device__ __forceinline__ uint4 f32_to_bf16x8(const float *f) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// db[co] += sum_p dz[p][co].  Thread = 8 channels x a pixel lane (cout / 8
-// divides the block); lanes are summed in shared memory, then one atomic per
-// channel and block.
-__global__ void k_bgrad(float *db, const bf16 *dz, int P, int cout) {
+// dz[p][co] = g[p][goff + co] * (relu ? (y[p][yoff + co] > 0) : 1), as BF16, and
+// the bias gradient db[co] += sum_p dz[p][co] (of the rounded values).  Thread =
+// 8 channels x a pixel lane (cout / 8 divides the block; cout, ldg, goff, ldy,
+// yoff multiples of 8); lanes are summed in shared memory, then one atomic per
+// channel and block.  Memory bound: one pass, 4 + 2 bytes in and 2 out per
+// value (a second kernel had read dz back for the sum: 0.59 + 0.42 ms of the
+// 7.97 ms of a batch of eight at 512x512).
+__global__ void __launch_bounds__(256) k_dz(bf16 *dz, const float *g, int ldg, int goff,
+                                            const bf16 *y, int ldy, int yoff, int P, int cout,
+                                            int relu, float *db) {
     __shared__ float acc[256];
     const int groups = cout >> 3, lanes = blockDim.x / groups;
-    const int cg = threadIdx.x % groups, pl = threadIdx.x / groups;
-    for (int c = threadIdx.x; c < cout; c += blockDim.x) acc[c] = 0.f;
+    const int cg = threadIdx.x % groups, pl = threadIdx.x / groups, c = cg * 8;
+    for (int i = threadIdx.x; i < cout; i += blockDim.x) acc[i] = 0.f;
     __syncthreads();
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int p = blockIdx.x * lanes + pl; p < P; p += gridDim.x * lanes) {
-        float f[8];
-        bf16x8_to_f32(*reinterpret_cast<const uint4 *>(dz + (size_t)p * cout + cg * 8), f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s[j] += f[j];
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(&acc[cg * 8 + j], s[j]);
-    __syncthreads();
-    for (int c = threadIdx.x; c < cout; c += blockDim.x) atomicAdd(&db[c], acc[c]);
-}
-
-// dz[p][co] = g[p][goff + co] * (relu ? (y[p][yoff + co] > 0) : 1), as BF16;
-// 8 channels per thread (cout, ldg, goff, ldy, yoff multiples of 8).
-__global__ void k_dz(bf16 *dz, const float *g, int ldg, int goff, const bf16 *y, int ldy, int yoff,
-                     int P, int cout, int relu) {
-    const int groups = cout >> 3;
-    const size_t n = (size_t)P * groups;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const size_t p = i / groups;
-        const int c = (int)(i - p * groups) * 8;
+#pragma unroll 2
+    for (size_t p = blockIdx.x * (size_t)lanes + pl; p < (size_t)P; p += (size_t)gridDim.x * lanes) {
         const float4 *gp = reinterpret_cast<const float4 *>(g + p * ldg + goff + c);
         const float4 g0 = gp[0], g1 = gp[1];
         float v[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
@@ -327,8 +313,16 @@ __global__ void k_dz(bf16 *dz, const float *g, int ldg, int goff, const bf16 *y,
             for (int j = 0; j < 8; ++j)
                 if (!(yv[j] > 0.f)) v[j] = 0.f;
         }
-        *reinterpret_cast<uint4 *>(dz + p * cout + c) = f32_to_bf16x8(v);
+        const uint4 r = f32_to_bf16x8(v);
+        *reinterpret_cast<uint4 *>(dz + p * cout + c) = r;
+        bf16x8_to_f32(r, v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += v[j];
     }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) atomicAdd(&acc[c + j], s[j]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < cout; i += blockDim.x) atomicAdd(&db[i], acc[i]);
 }
 
 // wt[ci][taps - 1 - t][co] = w[co][t][ci]
@@ -415,7 +409,7 @@ __global__ void k_up_fwd(bf16 *out, int ldo, int ooff, const bf16 *in, int B, in
     }
 }
 
-// gin[b][i][j][c] += sum of the 2 x 2 block of gout[..][goff + c]  (H, W: input
+// gin[b][i][j][c] = sum of the 2 x 2 block of gout[..][goff + c]  (H, W: input
 // size); 4 channels per thread.
 __global__ void k_up_bwd(float *gin, const float *gout, int ldg, int goff, int B, int H, int W,
                          int C) {
@@ -426,7 +420,7 @@ __global__ void k_up_bwd(float *gin, const float *gout, int ldg, int goff, int B
         const int c = (int)(i % G) * 4;
         const size_t p = i / G;
         const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((size_t)W * H));
-        float4 s = *reinterpret_cast<const float4 *>(gin + p * C + c);
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int d = 0; d < 4; ++d) {
             const size_t po = ((size_t)b * 2 * H + 2 * y + (d >> 1)) * (2 * W) + 2 * x + (d & 1);
@@ -632,7 +626,7 @@ __device__ __forceinline__ TcTile tc_tile(int t, int n_nt, int tiles_x, int tile
 // NT columns from tensor memory at tacc, + bias, ReLU, then 16 channels per
 // vector group to the BF16 output (at the pixel, or with up2 at the 2 x 2
 // block of the pixel in an image of twice the size: nearest up-sampling)
-// and / or the FP32 output (optionally accumulated).
+// and / or the FP32 output.
 // STRIP: the tile is 128 consecutive pixels of one image row (x0 .. x0+127
 // of row y0) instead of an 8 x 16 patch.
 template <int NT, bool STRIP = false>
@@ -692,15 +686,7 @@ __device__ __forceinline__ void conv_tc_store(const ConvArgs &a, const TcTile &T
             float4 *d = reinterpret_cast<float4 *>(a.yf + p * a.ldyf + a.yfoff + co);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                float4 o = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-                if (a.accumulate) {
-                    const float4 g = d[j];
-                    o.x += g.x;
-                    o.y += g.y;
-                    o.z += g.z;
-                    o.w += g.w;
-                }
-                d[j] = o;
+                d[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
             }
         }
     }
@@ -1561,14 +1547,16 @@ cudaError_t UNet::run_conv(const ConvArgs &a, int P) {
 
 // Gradients of layer li whose output is out[..][out_off, +cout) with gradient
 // out.g: weights, bias, and (when in.g is set and li > 0) the input gradient
-// in.g[..][in_off, +cin) += ...
+// in.g[..][in_off, +cin), written: the convolution is the first to contribute to
+// its input's gradient (the max-pool of a skip connection adds to it later).
 cudaError_t UNet::conv_bwd(int li, Act &in, int in_off, Act &out, int out_off) {
     const ConvLayer &L = layers_[li];
     const int P = B_ * in.H * in.W;
     const bool is_out = &out == &acts_[A_OUT];
-    k_dz<<<gridn_u((size_t)P * L.cout / 8), 256, 0, st_>>>(
-        dz_, is_out ? outg_ : out.g, out.C, is_out ? 0 : out_off, out.v, out.C,
-        out_off, P, L.cout, L.relu ? 1 : 0);
+    const int lanes = 256 / (L.cout / 8);  // pixel lanes of a k_dz block
+    k_dz<<<std::min((P + lanes - 1) / lanes, 148 * 8), 256, 0, st_>>>(
+        dz_, is_out ? outg_ : out.g, out.C, is_out ? 0 : out_off, out.v, out.C, out_off, P, L.cout,
+        L.relu ? 1 : 0, grad_ + L.b_off);
     WgArgs w{};
     w.dz = dz_;
     w.x = in.v;
@@ -1589,10 +1577,7 @@ cudaError_t UNet::conv_bwd(int li, Act &in, int in_off, Act &out, int out_off) {
         k_wgrad<<<dim3((L.cout + 63) / 64, (L.cin + 63) / 64, L.ks * L.ks * w.splits), kCT, 0,
                    st_>>>(w);
     }
-    const int lanes = 256 / (L.cout / 8);  // pixel lanes of a k_bgrad block
-    k_bgrad<<<std::min((P + lanes - 1) / lanes, 148 * 4), 256, 0, st_>>>(grad_ + L.b_off, dz_, P,
-                                                                         L.cout);
-    launches_ += 3;
+    launches_ += 2;
     if (li > 0 && in.g) {
         ConvArgs a{};
         a.x = dz_;
@@ -1604,7 +1589,6 @@ cudaError_t UNet::conv_bwd(int li, Act &in, int in_off, Act &out, int out_off) {
         a.yf = in.g;
         a.ldyf = in.C;
         a.yfoff = in_off;
-        a.accumulate = 1;
         a.B = B_;
         a.H = in.H;
         a.W = in.W;
@@ -1700,10 +1684,6 @@ cudaError_t UNet::gradients(const float *x, const float *target, float *loss) {
     U_TRY(cudaMemsetAsync(og, 0, (size_t)B_ * H_ * W_ * 16 * sizeof(float), st_));
     k_loss<<<kLossBlocks, 256, 0, st_>>>(og, scratch_, A[A_OUT].g, target, B_, H_ * W_);
     ++launches_;
-    for (int i = 0; i < A_COUNT; ++i)
-        if (i != A_OUT)
-            U_TRY(cudaMemsetAsync(A[i].g, 0, (size_t)B_ * A[i].H * A[i].W * A[i].C * sizeof(float),
-                                  st_));
     U_TRY(cudaMemsetAsync(grad_, 0, n_params_ * sizeof(float), st_));
     auto pool_bwd = [&](int dst, int lvl, int src) {  // gradient of pool(dst) -> dst.g
         Act &d = A[dst];
