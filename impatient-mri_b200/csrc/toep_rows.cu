@@ -1,4 +1,4 @@
-// Pruned F^H F engine of 2-D images on mixed-radix lengths.
+// Pruned F^H F engine of 2-D and 3-D images on mixed-radix lengths.
 //
 // Along each axis of length n the zero-padded 2n-point transform splits by
 // output parity a into two n-point transforms of x[j] w_2n^{a j}; the inverse
@@ -7,11 +7,14 @@
 // k = k2 + R2 k1, an n-point line is an R2-point register DFT per j1, the
 // twiddle w_2n^{j1 (2 k2 + a)} (it carries the parity's j1 part; the rest,
 // w_{2 R2}^{a j2}, is a compile-time constant) and an R1-point register DFT
-// per k2.  Three kernels per chunk of (segment, coil) transforms:
+// per k2.  An image is [s][m][f] (2-D: one m).  Kernels per chunk of (segment,
+// coil) transforms:
 //   k_row_fwd  rows along f: forms S_c e_l x from global memory in registers,
-//              both parities, writes [s][a][k];
+//              both parities, writes [s][m][a][kf];
+//   k_mid_fwd  3-D: columns along m, both parities, writes [s][a][km][...];
 //   k_col      columns along s, in place: both parities forward, x Qf_l,
 //              inverse, parity sum;
+//   k_mid_inv  3-D: columns along m: inverse, parity sum;
 //   k_row_inv  rows along f: inverse, parity sum, conj(e_l S_c), summed over the
 //              block's transforms in registers and over the cluster's blocks in
 //              distributed shared memory.
@@ -19,6 +22,12 @@
 // one writes it from registers, so a row kernel makes one trip through shared
 // memory and the column kernel two.  The inverse transforms run as forward
 // ones on values with real and imaginary parts exchanged.
+//
+// What bounds it: issue and latency at 16 to 24 warps per SM (the register DFTs
+// take 64 registers for 32 points), not memory (15 to 60 % of DRAM).  512x512 x 32
+// coils, one application: rows forward 49 us, columns 151, rows inverse 96 (a plane
+// engine of line passes in shared memory: 74, 174, 112).  256x256x32 x 4 coils, one
+// segment: 54, 89 (middle forward), 257, 77, 73 us (plane engine 176, 273, 202).
 //
 // Sides that are no length of the table run on the next one: rows and columns
 // past the image are zero on input and dropped on output, Q_l sits at its
@@ -225,18 +234,25 @@ struct ColShape {
     static constexpr size_t smem = sizeof(float2) * (size_t)2 * R1 * P * W;
 };
 
-// Columns [blockIdx.x W, + W) of the transform blockIdx.y, in place.
+// Block = (column group, transform).  Columns [cg W, + W) of the transform, in
+// place.  `jobs_x`: the transform is the faster block index, so that the coils of
+// a segment read the same columns of Qf_l close in time (3-D, where Qf_l exceeds
+// the L2; in 2-D the neighbouring columns first are faster, 6.51 against 6.62 ms
+// for 20 updates at 512x512 x 32 coils).
 template <int R1, int R2>
-__global__ void __launch_bounds__(ColShape<R1, R2>::T, cmax(1, 512 / ColShape<R1, R2>::T))
+__global__ void __launch_bounds__(ColShape<R1, R2>::T, cmax(1, (R1 == 16 ? 768 : 512) / ColShape<R1, R2>::T))
     k_col(float2 *__restrict__ b1, const float2 *__restrict__ qf2, int ns, int ncol, int C,
-          int job0, const float2 *__restrict__ tw, const int *__restrict__ done) {
+          int job0, int jobs_x, const float2 *__restrict__ tw, const int *__restrict__ done) {
     using S = ColShape<R1, R2>;
     constexpr int W = S::W, P = S::P, n = S::n;
     extern __shared__ float2 sm[];
     if (done && *done) return;
-    const int l = (job0 + blockIdx.y) / C;
+    const unsigned cgrp = jobs_x ? blockIdx.y : blockIdx.x;
+    const int job = (int)(jobs_x ? blockIdx.x : blockIdx.y);
+    const int l = (job0 + job) / C;
     const int w = threadIdx.x % W, tj = threadIdx.x / W;
-    float2 *col = b1 + (size_t)blockIdx.y * ns * ncol + blockIdx.x * W + w;
+    const size_t col0 = (size_t)cgrp * W + w;
+    float2 *col = b1 + (size_t)job * ns * ncol + col0;
     const float2 *twB = tw + 2 * n;
     if (tj < R1) {
         const int j1 = tj;
@@ -267,8 +283,7 @@ __global__ void __launch_bounds__(ColShape<R1, R2>::T, cmax(1, 512 / ColShape<R1
 #pragma unroll
         for (int q = 0; q < R1; ++q) z[q] = p[q * P * W];
         fftr::dft<R1>(z);
-        const float2 *qc = qf2 + (size_t)l * 2 * n * ncol + (size_t)(a * n + k2) * ncol +
-                           blockIdx.x * W + w;
+        const float2 *qc = qf2 + (size_t)l * 2 * n * ncol + (size_t)(a * n + k2) * ncol + col0;
 #pragma unroll
         for (int q = 0; q < R1; ++q)
             z[q] = fftr::swap_ri(cmul(z[q], __ldg(&qc[(size_t)(R2 * q) * ncol])), true);
@@ -299,33 +314,137 @@ __global__ void __launch_bounds__(ColShape<R1, R2>::T, cmax(1, 512 / ColShape<R1
     }
 }
 
-__global__ void k_embed(float2 *__restrict__ buf, const float *__restrict__ qr,
-                        const float *__restrict__ qi, int ns, int nf, int es, int ef) {
-    const size_t G = (size_t)4 * ns * nf;
-    buf += (size_t)blockIdx.y * 4 * es * ef;
-    qr += blockIdx.y * G;
-    qi += blockIdx.y * G;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < G;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i / (2 * nf)), y = (int)(i % (2 * nf));
-        const int dx = x - ns, dy = y - nf;  // displacement
-        const size_t o = (size_t)(dx < 0 ? dx + 2 * es : dx) * (2 * ef) + (dy < 0 ? dy + 2 * ef : dy);
-        buf[o] = make_float2(qr[i], qi[i]);
+// Columns along m of one s-plane: in [m][w] (row stride ncol) -> both parities
+// [a][km][w].  blockIdx.x = column group, .y = s, .z = transform.
+template <int R1, int R2>
+__global__ void __launch_bounds__(ColShape<R1, R2>::T)
+    k_mid_fwd(float2 *__restrict__ b1, const float2 *__restrict__ b0, int nm, int ncol,
+              const float2 *__restrict__ tw, const int *__restrict__ done) {
+    using S = ColShape<R1, R2>;
+    constexpr int W = S::W, P = S::P, n = S::n;
+    extern __shared__ float2 sm[];
+    if (done && *done) return;
+    const int w = threadIdx.x % W, tj = threadIdx.x / W;
+    const size_t plane = (size_t)blockIdx.z * gridDim.y + blockIdx.y;
+    if (tj < R1) {
+        const int j1 = tj;
+        const float2 *src = b0 + plane * nm * ncol + blockIdx.x * W + w;
+        float2 v[R2], t[R2];
+#pragma unroll
+        for (int q = 0; q < R2; ++q) {
+            v[q] = make_float2(0.f, 0.f);
+            if (j1 + R1 * q < nm) v[q] = src[(size_t)(j1 + R1 * q) * ncol];
+        }
+        float2 *dst = sm + j1 * P * W + w;
+#pragma unroll
+        for (int q = 0; q < R2; ++q) t[q] = v[q];
+        fftr::dft<R2>(t);
+        dst[0] = t[0];
+#pragma unroll
+        for (int q = 1; q < R2; ++q) dst[q * W] = cmul(t[q], __ldg(&tw[q * R1 + j1]));
+        half_twist<R2, 1>(v);
+        fftr::dft<R2>(v);
+        dst += R1 * P * W;
+#pragma unroll
+        for (int q = 0; q < R2; ++q) dst[q * W] = cmul(v[q], __ldg(&tw[(R2 + q) * R1 + j1]));
+    }
+    __syncthreads();
+    if (tj < 2 * R2) {
+        const int a = tj / R2, k2 = tj - a * R2;
+        const float2 *src = sm + (a * R1 * P + k2) * W + w;
+        float2 z[R1];
+#pragma unroll
+        for (int q = 0; q < R1; ++q) z[q] = src[q * P * W];
+        fftr::dft<R1>(z);
+        float2 *dst = b1 + (plane * 2 * n + (size_t)a * n + k2) * ncol + blockIdx.x * W + w;
+#pragma unroll
+        for (int q = 0; q < R1; ++q) dst[(size_t)(R2 * q) * ncol] = z[q];
     }
 }
 
-// [2es][2ef] natural order -> row (as es + ks), column (af ef + kf), scaled
-__global__ void k_qf_parity(float2 *__restrict__ qf2, const float2 *__restrict__ qf, int es,
-                            int ef, float scale) {
-    const size_t G = (size_t)4 * es * ef;
-    qf2 += blockIdx.y * G;
-    qf += blockIdx.y * G;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < G;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const int ks = (int)(i / (2 * ef)), kf = (int)(i % (2 * ef));
+// The inverse of k_mid_fwd: both parities back to the nm rows of the image.
+template <int R1, int R2>
+__global__ void __launch_bounds__(ColShape<R1, R2>::T)
+    k_mid_inv(float2 *__restrict__ b0, const float2 *__restrict__ b1, int nm, int ncol,
+              const float2 *__restrict__ tw, const int *__restrict__ done) {
+    using S = ColShape<R1, R2>;
+    constexpr int W = S::W, P = S::P, n = S::n;
+    extern __shared__ float2 sm[];
+    if (done && *done) return;
+    const int w = threadIdx.x % W, tj = threadIdx.x / W;
+    const size_t plane = (size_t)blockIdx.z * gridDim.y + blockIdx.y;
+    const float2 *twB = tw + 2 * n;
+    if (tj < 2 * R2) {
+        const int a = tj / R2, k2 = tj - a * R2;
+        const float2 *src = b1 + (plane * 2 * n + (size_t)a * n + k2) * ncol + blockIdx.x * W + w;
+        float2 z[R1];
+#pragma unroll
+        for (int q = 0; q < R1; ++q) z[q] = src[(size_t)(R2 * q) * ncol];
+#pragma unroll
+        for (int q = 0; q < R1; ++q) z[q] = fftr::swap_ri(z[q], true);
+        fftr::dft<R1>(z);
+        float2 *dst = sm + (a * R1 * P + k2) * W + w;
+        dst[0] = z[0];
+#pragma unroll
+        for (int q = 1; q < R1; ++q)
+            dst[q * P * W] = cmul(z[q], __ldg(&twB[(q * 2 + a) * R2 + k2]));
+    }
+    __syncthreads();
+    if (tj < R1) {
+        const int j1 = tj;
+        const float2 *src = sm + j1 * P * W + w;
+        float2 t[R2], u[R2];
+#pragma unroll
+        for (int q = 0; q < R2; ++q) t[q] = src[q * W];
+        fftr::dft<R2>(t);
+        src += R1 * P * W;
+#pragma unroll
+        for (int q = 0; q < R2; ++q) u[q] = src[q * W];
+        fftr::dft<R2>(u);
+        half_twist<R2, 1>(u);
+        float2 *dst = b0 + plane * nm * ncol + blockIdx.x * W + w;
+#pragma unroll
+        for (int q = 0; q < R2; ++q)
+            if (j1 + R1 * q < nm)
+                dst[(size_t)(j1 + R1 * q) * ncol] = make_float2(t[q].y + u[q].y, t[q].x + u[q].x);
+    }
+}
+
+// Sizes of a doubled grid and of the one it is placed on (2-D: middle sizes 1).
+struct Grids {
+    int n0, n1, n2;  // image axes doubled
+    int e0, e1, e2;  // engine lengths doubled
+};
+
+// blockIdx.y = index along the slowest axis, .z = segment
+__global__ void k_embed(float2 *__restrict__ buf, const float *__restrict__ qr,
+                        const float *__restrict__ qi, Grids g) {
+    const unsigned plane = (unsigned)g.n1 * g.n2;
+    const size_t src = ((size_t)blockIdx.z * g.n0 + blockIdx.y) * plane;
+    auto place = [](int i, int n, int e) {  // displacement i - n / 2 modulo e
+        return n == 1 ? 0 : (i < n / 2 ? i - n / 2 + e : i - n / 2);
+    };
+    buf += ((size_t)blockIdx.z * g.e0 + place((int)blockIdx.y, g.n0, g.e0)) * g.e1 * g.e2;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane;
+         i += gridDim.x * blockDim.x) {
+        const unsigned m = i / (unsigned)g.n2, f = i - m * g.n2;
+        buf[(size_t)place((int)m, g.n1, g.e1) * g.e2 + place((int)f, g.n2, g.e2)] =
+            make_float2(qr[src + i], qi[src + i]);
+    }
+}
+
+// Natural order -> parity-major along every axis (index (k & 1) e + (k >> 1)), scaled.
+__global__ void k_qf_parity(float2 *__restrict__ qf2, const float2 *__restrict__ qf, Grids g,
+                            float scale) {
+    const unsigned plane = (unsigned)g.e1 * g.e2;
+    auto par = [](unsigned k, int e) { return e == 1 ? 0u : (k & 1u) * (e / 2) + (k >> 1); };
+    qf += ((size_t)blockIdx.z * g.e0 + blockIdx.y) * plane;
+    qf2 += ((size_t)blockIdx.z * g.e0 + par(blockIdx.y, g.e0)) * plane;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane;
+         i += gridDim.x * blockDim.x) {
+        const unsigned m = i / (unsigned)g.e2, f = i - m * g.e2;
         const float2 v = qf[i];
-        qf2[(size_t)((ks & 1) * es + (ks >> 1)) * (2 * ef) + (kf & 1) * ef + (kf >> 1)] =
-            make_float2(v.x * scale, v.y * scale);
+        qf2[(size_t)par(m, g.e1) * g.e2 + par(f, g.e2)] = make_float2(v.x * scale, v.y * scale);
     }
 }
 
@@ -336,15 +455,19 @@ struct Entry {
     decltype(&k_row_fwd<8, 4>) fwd;
     decltype(&k_row_inv<8, 4>) inv;
     decltype(&k_col<8, 4>) col;
+    decltype(&k_mid_fwd<8, 4>) mid_fwd;
+    decltype(&k_mid_inv<8, 4>) mid_inv;
 };
 
 #define ER(A, B)                                                                              \
     {A * B, A, B, RowShape<A, B>::PS, RowShape<A, B>::T, ColShape<A, B>::T, RowShape<A, B>::smem, \
-     ColShape<A, B>::smem, k_row_fwd<A, B>, k_row_inv<A, B>, k_col<A, B>}
-// Lengths at most a fifth apart; R1 about 2 R2, so that the R1 threads of a line
+     ColShape<A, B>::smem, k_row_fwd<A, B>, k_row_inv<A, B>, k_col<A, B>, k_mid_fwd<A, B>,        \
+     k_mid_inv<A, B>}
+// Lengths at most a fifth apart (from 20); R1 about 2 R2, so that the R1 threads of a line
 // in the one pass and the 2 R2 of the other keep the same block busy.
 const Entry kTable[] = {
-    ER(4, 4),   ER(8, 4),   ER(8, 6),   ER(8, 8),   ER(10, 8),  ER(12, 8),  ER(14, 8),
+    ER(2, 2),   ER(4, 2),   ER(4, 3),   ER(4, 4),   ER(5, 4),   ER(6, 4),   ER(7, 4),
+    ER(8, 4),   ER(10, 4),  ER(8, 6),   ER(14, 4),  ER(8, 8),   ER(10, 8),  ER(12, 8),  ER(14, 8),
     ER(16, 8),  ER(16, 9),  ER(16, 10), ER(16, 12), ER(20, 10), ER(20, 12), ER(16, 16),
     ER(24, 12), ER(20, 16), ER(24, 14), ER(24, 16), ER(25, 16), ER(28, 16), ER(30, 16),
     ER(32, 16), ER(32, 18), ER(32, 20), ER(32, 24), ER(32, 28), ER(32, 32),
@@ -368,6 +491,10 @@ cudaError_t smem_opt(const Entry &e) {
     if (r == cudaSuccess)
         r = cudaFuncSetAttribute((const void *)e.col, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)e.sm_col);
+    for (const void *k : {(const void *)e.mid_fwd, (const void *)e.mid_inv})
+        if (r == cudaSuccess)
+            r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)e.sm_col);
     return r;
 }
 
@@ -388,72 +515,111 @@ cudaError_t twiddles(const Entry &e, float2 **tw) {
     return cudaMemcpy(*tw, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice);
 }
 
-unsigned blocks_for(size_t n) { return (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16); }
+Grids grids(const ToepRowsPlan &p) {
+    const bool three = p.nm > 1;
+    return Grids{2 * p.ns, three ? 2 * p.nm : 1, 2 * p.nf, 2 * p.es, three ? 2 * p.em : 1, 2 * p.ef};
+}
+
+// blocks along x for a plane of n elements, rows x segs planes
+dim3 plane_grid(size_t n, int rows, int segs) {
+    const size_t want = 148 * 16, planes = (size_t)rows * segs;
+    const size_t x = std::max<size_t>(1, std::min((n + 255) / 256, want / planes + 1));
+    return dim3((unsigned)x, rows, segs);
+}
 
 }  // namespace
 
-bool toep_rows_plan(int ns, int nf, int C, int L1, ToepRowsPlan *plan) {
+bool toep_rows_plan(int ns, int nm, int nf, int C, int L1, ToepRowsPlan *plan) {
     ToepRowsPlan p;
     p.ns = ns;
+    p.nm = nm;
     p.nf = nf;
     p.C = C;
     p.L1 = L1;
     p.e_s = entry_for(ns);
+    p.e_m = nm > 1 ? entry_for(nm) : 0;
     p.e_f = entry_for(nf);
-    if (ns < 1 || nf < 1 || C < 1 || L1 < 1 || p.e_s < 0 || p.e_f < 0) return false;
+    if (ns < 1 || nm < 1 || nf < 1 || C < 1 || L1 < 1 || L1 > 65535 || p.e_s < 0 || p.e_m < 0 ||
+        p.e_f < 0)
+        return false;
     p.es = kTable[p.e_s].n;
+    p.em = nm > 1 ? kTable[p.e_m].n : 1;
     p.ef = kTable[p.e_f].n;
-    // Half spectra of at most 256 MB: the kernels are bound by issue and latency, not by
+    // Half spectra of at most 320 MB: the kernels are bound by issue and latency, not by
     // memory, so chunks that fit the L2 only add launches and tails (512x512 x 32 coils, 20
     // updates: 6.54 ms in one chunk of 134 MB, 6.90 in 64 MB chunks, 7.33 in 32 MB ones).
-    const size_t job = sizeof(float2) * (size_t)ns * 2 * p.ef;
-    const size_t fit = std::max<size_t>(1, ((size_t)256 << 20) / job);
+    // A whole number of coil sets where they fit, for the reuse of Qf_l in k_col.
+    const size_t job = sizeof(float2) * p.job_elems();
+    const size_t fit = std::max<size_t>(1, ((size_t)320 << 20) / job);
     const size_t jobs = (size_t)L1 * C;
     const size_t parts = (jobs + fit - 1) / fit;
-    p.chunk = (int)std::min<size_t>((jobs + parts - 1) / parts, 65535);
-    if (smem_opt(kTable[p.e_s]) != cudaSuccess || smem_opt(kTable[p.e_f]) != cudaSuccess)
-        return false;
+    size_t chunk = (jobs + parts - 1) / parts;
+    if (chunk > (size_t)C) chunk = std::min(fit / C * C, (chunk + C - 1) / C * C);
+    else if (fit >= (size_t)C) chunk = C;
+    p.chunk = (int)std::min<size_t>(std::max<size_t>(chunk, 1), 65535);
+    for (int e : {p.e_s, p.e_m, p.e_f})
+        if (smem_opt(kTable[e]) != cudaSuccess) return false;
     *plan = p;
     return true;
 }
 
-cudaError_t toep_rows_twiddles(const ToepRowsPlan &p, float2 **tw_s, float2 **tw_f) {
-    const cudaError_t e = twiddles(kTable[p.e_s], tw_s);
-    return e != cudaSuccess ? e : twiddles(kTable[p.e_f], tw_f);
+cudaError_t toep_rows_twiddles(const ToepRowsPlan &p, float2 *tw[3]) {
+    const int e[3] = {p.e_s, p.e_m, p.e_f};
+    for (int a = 0; a < 3; ++a)
+        if (a != 1 || p.nm > 1) {
+            const cudaError_t r = twiddles(kTable[e[a]], &tw[a]);
+            if (r != cudaSuccess) return r;
+        }
+    return cudaSuccess;
 }
 
 cudaError_t toep_rows_embed(const ToepRowsPlan &p, float2 *fftbuf, const float *q_r,
                             const float *q_i, int nl, cudaStream_t st) {
-    if (p.es != p.ns || p.ef != p.nf) {
+    if (p.es != p.ns || p.em != p.nm || p.ef != p.nf) {
         const cudaError_t e = cudaMemsetAsync(fftbuf, 0, sizeof(float2) * p.q_elems() * nl, st);
         if (e != cudaSuccess) return e;
     }
-    k_embed<<<dim3(blocks_for((size_t)4 * p.ns * p.nf), nl), 256, 0, st>>>(
-        fftbuf, q_r, q_i, p.ns, p.nf, p.es, p.ef);
+    const Grids g = grids(p);
+    k_embed<<<plane_grid((size_t)g.n1 * g.n2, g.n0, nl), 256, 0, st>>>(fftbuf, q_r, q_i, g);
     return cudaGetLastError();
 }
 
 cudaError_t toep_rows_qf(const ToepRowsPlan &p, float2 *qf2, const float2 *qf, float scale, int nl,
                          cudaStream_t st) {
-    k_qf_parity<<<dim3(blocks_for(p.q_elems()), nl), 256, 0, st>>>(qf2, qf, p.es, p.ef, scale);
+    const Grids g = grids(p);
+    k_qf_parity<<<plane_grid((size_t)g.e1 * g.e2, g.e0, nl), 256, 0, st>>>(qf2, qf, g, scale);
     return cudaGetLastError();
 }
 
 cudaError_t toep_rows_apply(const ToepRowsPlan &p, float2 *q, const float2 *x, const float2 *sens,
-                            const float2 *eph, float2 *b1, const float2 *qf2, const int *done,
-                            const float2 *tw_s, const float2 *tw_f, cudaStream_t st) {
-    const Entry &es = kTable[p.e_s], &ef = kTable[p.e_f];
-    const unsigned groups = (unsigned)((p.ns + ef.ps - 1) / ef.ps);
+                            const float2 *eph, float2 *b0, float2 *b1, const float2 *qf2,
+                            const int *done, float2 *const tw[3], cudaStream_t st) {
+    const Entry &es = kTable[p.e_s], &em = kTable[p.e_m], &ef = kTable[p.e_f];
+    const bool three = p.nm > 1;
+    const int rows = p.ns * p.nm, cols = 2 * p.ef, ncol = (three ? 2 * p.em : 1) * cols;
+    const unsigned groups = (unsigned)((rows + ef.ps - 1) / ef.ps);
+    float2 *rbuf = three ? b0 : b1;  // the rows' spectra
     const int jobs = p.L1 * p.C;
     for (int j0 = 0; j0 < jobs; j0 += p.chunk) {
         const int nj = std::min(p.chunk, jobs - j0);
-        ef.fwd<<<dim3(groups, nj), ef.t_row, ef.sm_row, st>>>(b1, x, sens, eph, p.ns, p.nf, p.C,
-                                                             j0, tw_f, done);
-        es.col<<<dim3(2 * p.ef / kColW, nj), es.t_col, es.sm_col, st>>>(
-            b1, qf2, p.ns, 2 * p.ef, p.C, j0, tw_s, done);
-        // cluster over the transforms: as many ranks as give every one the same
-        // number of them (at most 8, the portable cluster size)
-        const int rounds = (nj + 7) / 8, cs = (nj + rounds - 1) / rounds;
+        ef.fwd<<<dim3(groups, nj), ef.t_row, ef.sm_row, st>>>(rbuf, x, sens, eph, rows, p.nf, p.C,
+                                                             j0, tw[2], done);
+        const dim3 mid(cols / kColW, p.ns, nj);
+        if (three)
+            em.mid_fwd<<<mid, em.t_col, em.sm_col, st>>>(b1, b0, p.nm, cols, tw[1], done);
+        const bool jobs_x = three && ncol / kColW <= 65535;
+        const dim3 gc = jobs_x ? dim3(nj, ncol / kColW) : dim3(ncol / kColW, nj);
+        es.col<<<gc, es.t_col, es.sm_col, st>>>(b1, qf2, p.ns, ncol, p.C, j0, jobs_x ? 1 : 0,
+                                               tw[0], done);
+        if (three)
+            em.mid_inv<<<mid, em.t_col, em.sm_col, st>>>(b0, b1, p.nm, cols, tw[1], done);
+        // cluster over the transforms: enough ranks for some sixteen blocks per SM (at
+        // most 8, the portable cluster size), as many as give every one the same number
+        // of transforms; a block of a 3-D image takes them all (256x256x32 x 4: 96 us
+        // per launch with one each, for the cluster's barriers and the exchange)
+        const int want = std::min(8, std::max(1, (int)((148 * 16 + groups - 1) / groups)));
+        const int most = std::min(want, nj);
+        const int rounds = (nj + most - 1) / most, cs = (nj + rounds - 1) / rounds;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(groups, cs);
         cfg.blockDim = dim3(ef.t_row);
@@ -466,9 +632,9 @@ cudaError_t toep_rows_apply(const ToepRowsPlan &p, float2 *q, const float2 *x, c
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const cudaError_t e =
-            cudaLaunchKernelEx(&cfg, ef.inv, q, (const float2 *)b1, sens, eph, p.ns, p.nf, p.C, j0,
-                               nj, j0 == 0 ? 1 : 0, tw_f, done);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, ef.inv, q, (const float2 *)rbuf, sens, eph,
+                                                 rows, p.nf, p.C, j0, nj, j0 == 0 ? 1 : 0,
+                                                 (const float2 *)tw[2], done);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();

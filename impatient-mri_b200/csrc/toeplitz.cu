@@ -17,10 +17,9 @@
 //   cells the post kernels read;
 // * every shift / crop / deapodisation / phase / SENSE step is an index map
 //   fused into the kernels around the FFTs; the FFTs are this library's own
-//   (the pruned F^H F engine of toep_fft.cu for power-of-two images, the
-//   mixed-radix grid transform of grid_fft.cu for the gridding grids, Qf_l
-//   and the zero-padded chain of other sizes, all coils batched in one
-//   transform);
+//   (the pruned mixed-radix F^H F engine of toep_rows.cu, the mixed-radix grid
+//   transform of grid_fft.cu for the gridding grids, Qf_l and the zero-padded
+//   chain of sides longer than the engine's longest length);
 // * Qf_l, sensitivities and phase factors stay resident in HBM; one CG
 //   iteration (FFT chain + FP64 CG scalars, best-iterate tracking and the
 //   tolerance stop all on the device) is captured once as a CUDA graph.
@@ -685,12 +684,12 @@ void ToepSolver::release() {
     }
     reg_.release();
     void *bufs[] = {sens_, eph_, fm_, qf_, big_, x_, r_, p_, q_, best_, fhd_, w_, dots_,
-                    t_, grid_, qf2_, b1_, tw_, tw_f_};
+                    t_, grid_, qf2_, b0_, b1_, tw_[0], tw_[1], tw_[2]};
     for (void *b : bufs)
         if (b) cudaFree(b);
     sens_ = eph_ = qf_ = big_ = x_ = r_ = p_ = q_ = best_ = fhd_ = grid_ = nullptr;
-    qf2_ = b1_ = tw_ = tw_f_ = nullptr;
-    fast_ = rows_ = false;
+    qf2_ = b0_ = b1_ = tw_[0] = tw_[1] = tw_[2] = nullptr;
+    rows_ = false;
     fm_ = w_ = t_ = nullptr;
     dots_ = nullptr;
     grid_cells_ = 0;
@@ -767,25 +766,20 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     if (cfg.q_only) return cudaSuccess;
     T_TRY(cudaMalloc(&sens_, sizeof(float2) * C * N_));
     T_TRY(cudaMalloc(&eph_, sizeof(float2) * L1 * N_));
-    // 2-D images run on the mixed-radix row engine (sides up to its longest
-    // length), 3-D images of power-of-two sides on the plane engine; other sizes
-    // (and IMP_TOEP_PADDED=1) use the zero-padded chain on the grid transform.
+    // Sides up to the engine's longest length run on the pruned mixed-radix
+    // engine; others (and IMP_TOEP_PADDED=1) use the zero-padded chain on the
+    // grid transform.
     const char *force_padded = std::getenv("IMP_TOEP_PADDED");
     const bool pruned = !(force_padded && force_padded[0] == '1');
-    rows_ = pruned && !is3d && toep_rows_plan(nv[0], nv[1], C, L1, &rp_);
-    fast_ = pruned && is3d && toep_fft_plan(nv[0], nv[1], nv[2], C, &fp_);
+    rows_ = pruned && toep_rows_plan(nv[0], is3d ? nv[1] : 1, is3d ? nv[2] : nv[1], C, L1, &rp_);
     if (rows_) {
         qf_segs_ = (int)std::min<size_t>(
             L1, std::max<size_t>(1, ((size_t)128 << 20) / (sizeof(float2) * rp_.q_elems())));
         T_TRY(cudaMalloc(&qf_, sizeof(float2) * rp_.q_elems() * qf_segs_));
         T_TRY(cudaMalloc(&qf2_, sizeof(float2) * rp_.q_elems() * L1));
+        if (rp_.b0_elems()) T_TRY(cudaMalloc(&b0_, sizeof(float2) * rp_.b0_elems()));
         T_TRY(cudaMalloc(&b1_, sizeof(float2) * rp_.b1_elems()));
-        T_TRY(toep_rows_twiddles(rp_, &tw_, &tw_f_));
-    } else if (fast_) {
-        T_TRY(cudaMalloc(&qf_, sizeof(float2) * G2_));  // one segment, before permutation
-        T_TRY(cudaMalloc(&qf2_, sizeof(float2) * L1 * G2_));
-        T_TRY(cudaMalloc(&b1_, sizeof(float2) * fp_.b1_elems()));
-        T_TRY(toep_fft_twiddles(&tw_));
+        T_TRY(toep_rows_twiddles(rp_, tw_));
     } else {
         T_TRY(cudaMalloc(&qf_, sizeof(float2) * L1 * G2_));
         T_TRY(cudaMalloc(&big_, sizeof(float2) * C * G2_));
@@ -801,11 +795,14 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     // for Qf_l (2-D grids are [n2[0]][n2[1]], 3-D [n2[0]][n2[1]][n2[2]])
     int d0 = is3d ? n2[0] : 1, d1 = is3d ? n2[1] : n2[0], d2 = is3d ? n2[2] : n2[1];
     if (rows_) {  // the engine's lengths; a doubled side that no grid takes stays refused
-        if (!grid_fft_length_ok(d1) || !grid_fft_length_ok(d2)) return cudaErrorInvalidValue;
-        d1 = 2 * rp_.es;
+        for (int d : {d0, d1, d2})
+            if (!grid_fft_length_ok(d)) return cudaErrorInvalidValue;
+        d0 = is3d ? 2 * rp_.es : 1;
+        d1 = is3d ? 2 * rp_.em : 2 * rp_.es;
         d2 = 2 * rp_.ef;
+    } else {
+        T_TRY(grid_fft_create(&gf2_, d0, d1, d2, C));
     }
-    if (!fast_ && !rows_) T_TRY(grid_fft_create(&gf2_, d0, d1, d2, C));
     T_TRY(grid_fft_create(&gf1_, d0, d1, d2, 1));
     launches_ = 2;
     return set_reg();
@@ -875,16 +872,12 @@ cudaError_t ToepSolver::load_q(const float *q_r, const float *q_i) {
     }
     const NV n2d{{n2[0], n2[1], n2[2]}};
     for (int l = 0; l <= L_; ++l) {
-        float2 *qf_l = fast_ ? qf_ : qf_ + (size_t)l * G2_;
+        float2 *qf_l = qf_ + (size_t)l * G2_;
         k_q_shift<<<gridn(G2_), kVB, 0, st_>>>(q_r + (size_t)l * G2_, q_i + (size_t)l * G2_, n2d,
                                               cfg_.nz > 1, qf_l, G2_);
         T_TRY(cudaGetLastError());
         T_TRY(grid_fft_exec(gf1_, qf_l, false, st_));
         launches_ += 1 + gf1_.passes();
-        if (fast_) {
-            T_TRY(toep_fft_qf(fp_, qf2_ + (size_t)l * G2_, qf_l, 1.0f / (float)G2_, st_));
-            ++launches_;
-        }
     }
     return cudaStreamSynchronize(st_);
 }
@@ -933,16 +926,7 @@ cudaError_t ToepSolver::apply_aha(const float2 *p, float2 *q) {
     const float scale = 1.0f / (float)G2_;
     const double *dots = dots_;
     if (rows_)
-        return toep_rows_apply(rp_, q, p, sens_, eph_, b1_, qf2_, done_flag(), tw_, tw_f_, st_);
-    if (fast_) {
-        const int *done = reinterpret_cast<const int *>(
-            reinterpret_cast<const char *>(dots_ + T_SCAL * kTBlocks) + offsetof(TScal, done));
-        for (int l = 0; l <= L_; ++l)
-            T_TRY(toep_fft_apply_l(fp_, q, p, sens_, eph_ + (size_t)l * N_, b1_,
-                                   qf2_ + (size_t)l * G2_, l == 0 ? 1 : 0, done, tw_, err_,
-                                   st_));
-        return cudaSuccess;
-    }
+        return toep_rows_apply(rp_, q, p, sens_, eph_, b0_, b1_, qf2_, done_flag(), tw_, st_);
     for (int l = 0; l <= L_; ++l) {
         const float2 *eph_l = eph_ + (size_t)l * N_;
         T_TRY(cudaMemsetAsync(big_, 0, sizeof(float2) * C * G2_, st_));

@@ -8,7 +8,6 @@
 
 #include "grid_fft.cuh"
 #include "sparse_reg.cuh"
-#include "toep_fft.cuh"
 #include "toep_rows.cuh"
 
 namespace imp {
@@ -104,7 +103,7 @@ private:
     float2 *sens_ = nullptr;   // [C][N]
     float2 *eph_ = nullptr;    // [(L+1)][N] exp(-i fm (tau l + t0))
     float *fm_ = nullptr;      // [N]
-    float2 *qf_ = nullptr;     // [(L+1)][G2] (one segment of scratch with the engine)
+    float2 *qf_ = nullptr;     // [(L+1)][G2] (qf_segs_ segments of scratch with the engine)
     float2 *big_ = nullptr;    // [C][G2] zero-padded chain (sizes the engine does not take)
     float2 *x_ = nullptr, *r_ = nullptr, *p_ = nullptr, *q_ = nullptr, *best_ = nullptr;
     float2 *fhd_ = nullptr;
@@ -118,18 +117,18 @@ private:
     size_t grid_cells_ = 0;
     cudaGraphExec_t g_iter_ = nullptr;
     long launches_ = 0;
-    // pruned FFT engine (power-of-two sizes); the zero-padded chain otherwise
-    bool fast_ = false;
-    ToepFftPlan fp_;
-    float2 *qf2_ = nullptr;    // [(L+1)][G2] Qf_l in parity-major order, scaled 1/G2
-    float2 *b1_ = nullptr;     // [C][half spectrum] engine scratch
-    float2 *tw_ = nullptr;     // twiddle table (rows_: of the slow axis)
-    // 2-D: mixed-radix row engine
+    // pruned mixed-radix engine (sides up to its longest length); the
+    // zero-padded chain otherwise
     bool rows_ = false;
     ToepRowsPlan rp_;
     int qf_segs_ = 1;          // segments of qf_ scratch
-    float2 *tw_f_ = nullptr;   // twiddle table of the fast axis
-    int aha_launches() const { return rows_ ? rp_.launches() : 3 * (L_ + 1); }
+    float2 *qf2_ = nullptr;    // [(L+1)] Qf_l in parity-major order, scaled
+    float2 *b0_ = nullptr;     // row spectra of a chunk (3-D)
+    float2 *b1_ = nullptr;     // half spectra of a chunk
+    float2 *tw_[3] = {nullptr, nullptr, nullptr};  // twiddle tables per axis
+    int aha_launches() const {
+        return rows_ ? rp_.launches() : (L_ + 1) * (3 + 2 * gf2_.passes());
+    }
 };
 
 }  // namespace imp

@@ -1,4 +1,4 @@
-"""The 2-D mixed-radix F^H F engine (toep_rows.cu): one A^H A (+ lambda D^H D) application
+"""The mixed-radix F^H F engine (toep_rows.cu): one A^H A (+ lambda D^H D) application
 against the FP64 oracle over the lengths of its table, the sides between them (which run on the
 next length), uneven coil counts and several segments; refused sizes stay refused."""
 import numpy as np
@@ -63,3 +63,25 @@ def test_sizes_past_the_table(pkg, ctx):
     c, Q, p = make((2 * 257, 4, 1), 1, 0, 6)
     with pytest.raises(pkg.ImpError):
         gpu_apply(pkg, ctx, opts_of(pkg, c), c, Q, p)
+
+
+# (x, y, z): y is the slow (column) axis, x the middle one, z the contiguous one
+SIZES_3D = [(2, 2, 2), (4, 6, 2), (10, 12, 4), (14, 18, 10), (40, 24, 12), (16, 34, 6), (34, 16, 18),
+            (20, 48, 24), (66, 10, 8), (10, 66, 8), (8, 12, 66), (24, 20, 30), (130, 6, 4),
+            (6, 130, 36), (4, 258, 2), (258, 4, 2), (4, 4, 258), (4, 1040, 2)]
+
+
+@pytest.mark.parametrize("nx,ny,nz", SIZES_3D)
+def test_3d_lengths_match_oracle(pkg, ctx, nx, ny, nz):
+    """3-D images over the table's lengths and between them (the last side is past the table:
+    the zero-padded chain)."""
+    c, Q, p = make((nx, ny, nz), 2, 1, nx * 7 + ny + 3 * nz)
+    got = gpu_apply(pkg, ctx, opts_of(pkg, c), c, Q, p)
+    assert rel(got, oracle_apply(c, Q, p, c["fdp"])) < TOL_OP
+
+
+@pytest.mark.parametrize("C,L", [(1, 0), (1, 3), (5, 2), (9, 1)])
+def test_3d_coils_and_segments_match_oracle(pkg, ctx, C, L):
+    c, Q, p = make((20, 14, 6), C, L, 10 * C + L)
+    got = gpu_apply(pkg, ctx, opts_of(pkg, c), c, Q, p)
+    assert rel(got, oracle_apply(c, Q, p, c["fdp"])) < TOL_OP
