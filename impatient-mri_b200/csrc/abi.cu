@@ -128,7 +128,7 @@ imp_status op_work(imp_context *ctx, int M, int N, int C, bool use_z, bool adj, 
     imp::nu_plan_dims(w.p, M, N, C, use_z);
     imp::NuPlan &p = w.p;
     const size_t theirs = (size_t)p.G * (adj ? p.Mpad : p.Npad);
-    size_t image = imp::nu_tc_enabled() ? imp::nu_image_bytes(p.CG, theirs) : 0;
+    size_t image = imp::nu_wants_image(p.CG) ? imp::nu_image_bytes(p.CG, theirs) : 0;
     for (;;) {
         p.img_bytes = image;
         w.l = imp::nu_default_launch(p, adj);

@@ -319,7 +319,6 @@ cudaError_t BfSolver::setup(const BfConfig &cfg, const float *kx, const float *k
     // field map is set per slice in solve()
     IMP_TRY(nu_plan_create(plan_, kx, ky, kz, t, ix, iy, iz, nullptr, sensi_r, sensi_i, cfg.M,
                            cfg.N, cfg.C, cfg.use_z, dev_err, st));
-    nu_plan_reserve_image(plan_);  // a tuning candidate at every coil count
     const size_t nk = (size_t)plan_.G * plan_.Mpad * plan_.CG;
     const size_t nxs = (size_t)plan_.G * plan_.Npad * plan_.CG;
     IMP_TRY(dalloc(&y_, nk));

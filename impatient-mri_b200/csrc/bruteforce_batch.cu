@@ -389,7 +389,7 @@ cudaError_t BfBatch::setup(const BfConfig &cfg, int S, const int *k_off, const f
     plan_.vgeo = vgeo_;
     plan_.sens = sens_;
     // B operand image of the FP16 tensor-core kernel (without the memory: the TF32 one)
-    if (nu_tc_enabled() && (CG > 8 || nu_tc_forced())) {
+    if (nu_wants_image(CG)) {
         const size_t need = nu_image_bytes(
             CG, (size_t)G * std::max<size_t>((size_t)mpad_total_, (size_t)S * Npad));
         if (cudaMalloc(&img_, need) == cudaSuccess) {

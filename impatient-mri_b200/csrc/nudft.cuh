@@ -153,6 +153,8 @@ cudaError_t nu_partials_tc_batch(const NuPlan &p, const NuLaunch &l, bool adj, i
 // FP16 head / tail tensor-core kernel (nudft_h.cu), same layouts; p.img holds
 // nu_image_bytes of the launch's "theirs" elements (all slices and coil groups).
 size_t nu_image_bytes(int CG, size_t elems);
+// Whether plans of this coil grouping use that kernel (more than 8 coils, or forced).
+bool nu_wants_image(int CG);
 cudaError_t nu_partials_h(const NuPlan &p, const NuLaunch &l, bool adj, const float2 *tdata,
                           float2 *out, unsigned *err, cudaStream_t st);
 cudaError_t nu_partials_h_batch(const NuPlan &p, const NuLaunch &l, bool adj, int S, int max_ours,
