@@ -885,10 +885,10 @@ def run_toeplitz(args, ws, rank, local):
         "gpu_launches": launches,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm,
-                     "traffic": ncu_traffic("toeplitz_apply_toep3d_256x256x32.md",
+                     "traffic": ncu_traffic("toeplitz_rows_toep3d_256x256x32.md",
                                             "traffic_bytes_per_apply:"),
-                     "traffic_source": "profiles/toeplitz_apply_toep3d_256x256x32.md: DRAM bytes "
-                                       "of the three engine kernels of one application (ncu)",
+                     "traffic_source": "profiles/toeplitz_rows_toep3d_256x256x32.md: DRAM bytes "
+                                       "of the five engine kernels of one application (ncu)",
                      "kernel": "A^H A application inside the CG (pruned FFT engine: k_row_fwd, k_mid_fwd, "
                                "k_col with x Qf_l, k_mid_inv, k_row_inv with the coil sum; CG update), "
                                "per application; bytes = the zero-padded FFT model",
@@ -1279,9 +1279,9 @@ def run_headline(args, ws, rank, local):
         "gpu_launches": launches,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm,
-                     "traffic": ncu_traffic("toeplitz_apply_warm512.md",
+                     "traffic": ncu_traffic("toeplitz_rows_warm512.md",
                                             "traffic_bytes_per_apply:"),
-                     "traffic_source": "profiles/toeplitz_apply_warm512.md: DRAM bytes of the "
+                     "traffic_source": "profiles/toeplitz_rows_warm512.md: DRAM bytes of the "
                                        "three engine kernels of one application (ncu)",
                      "kernel": "one CG update (A^H A application: k_row_fwd, k_col with x Qf, "
                                "k_row_inv with the coil sum; FD term; vector updates); bytes "
