@@ -24,10 +24,10 @@
 // ones on values with real and imaginary parts exchanged.
 //
 // What bounds it: issue and latency at 16 to 24 warps per SM (the register DFTs
-// take 64 registers for 32 points), not memory (15 to 60 % of DRAM).  512x512 x 32
-// coils, one application: rows forward 49 us, columns 151, rows inverse 96 (a plane
-// engine of line passes in shared memory: 74, 174, 112).  256x256x32 x 4 coils, one
-// segment: 54, 89 (middle forward), 257, 77, 73 us (plane engine 176, 273, 202).
+// take 64 registers for 32 points), not memory (20 to 60 % of DRAM).  512x512 x 32
+// coils, one application: rows forward 48 us, columns 143, rows inverse 80 (a plane
+// engine of line passes in shared memory: 75, 175, 114).  256x256x32 x 4 coils, one
+// segment: 56, 91 (middle forward), 259, 79, 71 us (plane engine 176, 273, 202).
 //
 // Sides that are no length of the table run on the next one: rows and columns
 // past the image are zero on input and dropped on output, Q_l sits at its

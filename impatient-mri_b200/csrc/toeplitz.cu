@@ -129,19 +129,25 @@ __device__ __forceinline__ float kb_transform(float u, float beta) {
 constexpr int kGridWarps = 8;
 constexpr int kGridCoils = 32;  // coils per launch at most
 
-__global__ void __launch_bounds__(kGridWarps * 32)
+// ONE: a single value per sample and step (nc 1), kept in registers (the coil
+// loop's shared-memory read per cell costs: Q of 128x128x32 3.41 -> 3.09 ms).
+// D3: a 3-D grid; the axes' roles are compile-time, their arrays in registers.
+// The samples are strided over kGridBlocks resident blocks per SM.
+constexpr int kGridBlocks = 6;
+template <bool ONE, bool D3>
+__global__ void __launch_bounds__(kGridWarps * 32, kGridBlocks)
     k_grid_w(float2 *grid, size_t cells, const float *kx, const float *ky, const float *kz,
              const float *t, const float *dr, const float *di, int M, GridSpec g, float tau,
              float t0, int l0, int nl, int nc, int L1) {
     __shared__ float wsh[kGridWarps][3][kMaxTaps];
-    __shared__ float2 vsh[kGridWarps][kGridCoils];
+    __shared__ float2 vsh[ONE ? 1 : kGridWarps][kGridCoils];
     if (!(tau > 0.f)) return;  // every window is empty
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float(&ws)[3][kMaxTaps] = wsh[wid];
-    float2(&vs)[kGridCoils] = vsh[wid];
+    float2(&vs)[kGridCoils] = vsh[ONE ? 0 : wid];
     const float inv_os = 1.0f / g.os;
     // loop axis A, lane axes B (slower) and Cc (faster)
-    const int A = g.is3d ? 0 : 2, B = g.is3d ? 1 : 0, Cc = g.is3d ? 2 : 1;
+    constexpr int A = D3 ? 0 : 2, B = D3 ? 1 : 0, Cc = D3 ? 2 : 1;
     for (int s = blockIdx.x * kGridWarps + wid; s < M; s += gridDim.x * kGridWarps) {
         // segments around t: every lane reads the same sample, so all of this is warp-uniform
         const float ts = __ldg(&t[s]);
@@ -157,21 +163,26 @@ __global__ void __launch_bounds__(kGridWarps * 32)
             const float h = hanning(ts, tau, dr ? l : 2 * l, t0);
             const float h1 = !dr && 2 * l + 1 < L1 ? hanning(ts, tau, 2 * l + 1, t0) : 0.f;
             if (h == 0.f && h1 == 0.f) continue;
-            __syncwarp();  // the previous segment's values have been read
-            if (dr)
+            float2 v1 = make_float2(h, h1);
+            if constexpr (ONE) {
+                if (dr) {
+                    v1 = make_float2(h * __ldg(&dr[s]), h * (di ? __ldg(&di[s]) : 0.f));
+                    if (v1.x == 0.f && v1.y == 0.f) continue;
+                }
+            } else {
+                __syncwarp();  // the previous segment's values have been read
                 for (int c = lane; c < nc; c += 32) {
                     const size_t i = (size_t)c * M + s;
                     vs[c] = make_float2(h * __ldg(&dr[i]), h * (di ? __ldg(&di[i]) : 0.f));
                 }
-            else if (lane == 0)
-                vs[0] = make_float2(h, h1);
+            }
             if (!ready) {
                 ready = true;
-                const float k3[3] = {__ldg(&kx[s]), __ldg(&ky[s]), g.is3d ? __ldg(&kz[s]) : 0.f};
+                const float k3[3] = {__ldg(&kx[s]), __ldg(&ky[s]), D3 ? __ldg(&kz[s]) : 0.f};
                 float cc[3];
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
-                    if (a == 2 && !g.is3d) {
+                    if (a == 2 && !D3) {
                         lo[2] = 0;
                         cnt[2] = 1;
                         cc[2] = 0.f;
@@ -190,7 +201,7 @@ __global__ void __launch_bounds__(kGridWarps * 32)
                 for (int q = lane; q < 3 * kMaxTaps; q += 32) {
                     const int a = q / kMaxTaps, j = q - a * kMaxTaps;
                     if (j < cnt[a])
-                        ws[a][j] = (a == 2 && !g.is3d)
+                        ws[a][j] = (a == 2 && !D3)
                                        ? 1.f
                                        : kb_weight(fabsf(cc[a] - (float)(lo[a] + j)) * inv_os,
                                                    g.beta);
@@ -204,11 +215,11 @@ __global__ void __launch_bounds__(kGridWarps * 32)
             // 128x128x32 when a grid held one segment.)
             float2 *gl = grid + (size_t)(l - (dr ? l0 : l0 >> 1)) * nc * cells;
             const int nbc = cnt[B] * cnt[Cc];
-            int a0 = g.is3d ? lo[A] + g.gs[A] / 2 : 0;
+            int a0 = D3 ? lo[A] + g.gs[A] / 2 : 0;
             if (a0 >= g.gs[A]) a0 -= g.gs[A];
-            const size_t astride = g.is3d ? (size_t)g.gs[1] * g.gs[2] : 0;
+            const size_t astride = D3 ? (size_t)g.gs[1] * g.gs[2] : 0;
             const size_t awrap = astride * g.gs[A];
-            const int rowlen = g.is3d ? g.gs[2] : g.gs[1];  // stride of axis B
+            const int rowlen = D3 ? g.gs[2] : g.gs[1];  // stride of axis B
             for (int p = lane; p < nbc; p += 32) {
                 const int jb = p / cnt[Cc], jc = p - jb * cnt[Cc];
                 const float wbc = ws[B][jb] * ws[Cc][jc];
@@ -221,12 +232,16 @@ __global__ void __launch_bounds__(kGridWarps * 32)
                 int ia = a0;
                 for (int ja = 0; ja < cnt[A]; ++ja) {
                     const float ww = wbc * ws[A][ja];
-                    if (ww != 0.f)
-                        for (int c = 0; c < nc; ++c) {
-                            const float2 v = vs[c];
-                            atomicAdd(&gl[(size_t)c * cells + cell],
-                                      make_float2(ww * v.x, ww * v.y));
-                        }
+                    if (ww != 0.f) {
+                        if constexpr (ONE)
+                            atomicAdd(&gl[cell], make_float2(ww * v1.x, ww * v1.y));
+                        else
+                            for (int c = 0; c < nc; ++c) {
+                                const float2 v = vs[c];
+                                atomicAdd(&gl[(size_t)c * cells + cell],
+                                          make_float2(ww * v.x, ww * v.y));
+                            }
+                    }
                     cell += astride;
                     if (++ia == g.gs[A]) {
                         ia = 0;
@@ -642,9 +657,8 @@ static Crop crop_of(const GridSpec &g, bool negatives) {
     return c;
 }
 
-// Blocks of the warp-per-sample gridding: resident blocks of 8 warps on every
-// SM a few times over (grid-stride over the samples).
-static unsigned grid_blocks() { return 148u * 8u; }
+// Blocks of the warp-per-sample gridding: one wave (grid-stride over the samples).
+static unsigned grid_blocks() { return 148u * kGridBlocks; }
 
 GridSpec grid_spec(const int img[3], float os, bool beta_after_rounding, float kscale) {
     GridSpec g;
@@ -845,9 +859,10 @@ cudaError_t ToepSolver::compute_q(const float *kx, const float *ky, const float 
     for (int l = 0; l <= L_; l += 2 * nb) {
         const int nl = std::min(2 * nb, L_ + 1 - l), ng = (nl + 1) / 2;
         T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells() * ng, st_));
-        k_grid_w<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(grid_, g.cells(), kx, ky, kz, t_,
-                                                             nullptr, nullptr, cfg_.M, g, tau_,
-                                                             t0_, l, nl, 1, L_ + 1);
+        auto scatter = g.is3d ? k_grid_w<true, true> : k_grid_w<true, false>;
+        scatter<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(
+            grid_, g.cells(), kx, ky, kz, t_, nullptr, nullptr, cfg_.M, g, tau_, t0_, l, nl, 1,
+            L_ + 1);
         T_TRY(cudaGetLastError());
         T_TRY(grid_fft_exec_cropped(gfq_, grid_, true, crop.lo, crop.hi, st_, ng));
         k_q_post<<<gridn(G2_), kVB, 0, st_>>>(grid_, g.cells(), g, n2d, q_out_r + (size_t)l * G2_,
@@ -899,7 +914,9 @@ cudaError_t ToepSolver::compute_fhd(const float *kx, const float *ky, const floa
         for (int l = 0; l <= L_; l += nl_b) {
             const int nc = std::min(nc_b, cfg_.C - c), nl = std::min(nl_b, L_ + 1 - l);
             T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells() * nc * nl, st_));
-            k_grid_w<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(
+            auto scatter = nc == 1 ? (g.is3d ? k_grid_w<true, true> : k_grid_w<true, false>)
+                                   : (g.is3d ? k_grid_w<false, true> : k_grid_w<false, false>);
+            scatter<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(
                 grid_, g.cells(), kx, ky, kz, t_, kd_r + (size_t)c * cfg_.M,
                 kd_i + (size_t)c * cfg_.M, cfg_.M, g, tau_, t0_, l, nl, nc, L_ + 1);
             T_TRY(cudaGetLastError());
