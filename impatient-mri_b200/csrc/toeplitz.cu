@@ -707,6 +707,7 @@ void ToepSolver::release() {
     fm_ = w_ = t_ = nullptr;
     dots_ = nullptr;
     grid_cells_ = 0;
+    ready_ = false;
 }
 
 cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float *fm,
@@ -714,10 +715,10 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
                               cudaStream_t st) {
     // Same sizes and stream: keep buffers, FFT plans and (same CG terms) the
     // captured iteration graph; only the per-call inputs are refreshed.
-    const bool same_shape = (cfg.q_only ? t_ != nullptr : dots_ != nullptr) && st == st_ &&
-                            cfg.q_only == cfg_.q_only && cfg.nx == cfg_.nx && cfg.ny == cfg_.ny &&
-                            cfg.nz == cfg_.nz && cfg.C == cfg_.C && cfg.M == cfg_.M &&
-                            (int)cfg.ntime_segs == L_;
+    const bool same_shape = ready_ && st == st_ && cfg.q_only == cfg_.q_only &&
+                            cfg.nx == cfg_.nx && cfg.ny == cfg_.ny && cfg.nz == cfg_.nz &&
+                            cfg.C == cfg_.C && cfg.M == cfg_.M && (int)cfg.ntime_segs == L_;
+    ready_ = false;  // until this set-up is complete
     if (same_shape) {
         if (g_iter_ && (cfg.fd != cfg_.fd || cfg.lambda != cfg_.lambda ||
                         cfg.use_graphs != cfg_.use_graphs)) {
@@ -735,15 +736,21 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
         const int L1 = L_ + 1, C = cfg.C;
         T_TRY(cudaMemcpyAsync(t_, t, sizeof(float) * cfg.M, cudaMemcpyDeviceToDevice, st));
         launches_ = 0;
-        if (cfg.q_only) return cudaSuccess;
-        k_pack_sens_c<<<gridn((size_t)C * N_), kVB, 0, st>>>(sens_, sensi_r, sensi_i,
-                                                            (size_t)C * N_);
-        k_eph<<<gridn((size_t)L1 * N_), kVB, 0, st>>>(eph_, fm, N_, L1, tau_, t0_);
-        launches_ = 2;
-        T_TRY(cudaGetLastError());
-        return set_reg();
+        if (!cfg.q_only) {
+            k_pack_sens_c<<<gridn((size_t)C * N_), kVB, 0, st>>>(sens_, sensi_r, sensi_i,
+                                                                (size_t)C * N_);
+            k_eph<<<gridn((size_t)L1 * N_), kVB, 0, st>>>(eph_, fm, N_, L1, tau_, t0_);
+            launches_ = 2;
+            T_TRY(cudaGetLastError());
+            T_TRY(set_reg());
+        }
+        ready_ = true;
+        return cudaSuccess;
     }
     release();
+    // a doubled side that no grid transform takes is refused, whatever the call
+    for (int d : {cfg.nx, cfg.ny, cfg.nz})
+        if (d > 1 && !grid_fft_length_ok(2 * d)) return cudaErrorInvalidValue;
     cfg_ = cfg;
     st_ = st;
     err_ = dev_err;
@@ -777,7 +784,10 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     T_TRY(cudaMalloc(&t_, sizeof(float) * cfg.M));
     T_TRY(cudaMemcpyAsync(t_, t, sizeof(float) * cfg.M, cudaMemcpyDeviceToDevice, st));
     launches_ = 0;
-    if (cfg.q_only) return cudaSuccess;
+    if (cfg.q_only) {
+        ready_ = true;
+        return cudaSuccess;
+    }
     T_TRY(cudaMalloc(&sens_, sizeof(float2) * C * N_));
     T_TRY(cudaMalloc(&eph_, sizeof(float2) * L1 * N_));
     // Sides up to the engine's longest length run on the pruned mixed-radix
@@ -808,9 +818,7 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     // the 2N grid: batched over the coils for the zero-padded chain, single
     // for Qf_l (2-D grids are [n2[0]][n2[1]], 3-D [n2[0]][n2[1]][n2[2]])
     int d0 = is3d ? n2[0] : 1, d1 = is3d ? n2[1] : n2[0], d2 = is3d ? n2[2] : n2[1];
-    if (rows_) {  // the engine's lengths; a doubled side that no grid takes stays refused
-        for (int d : {d0, d1, d2})
-            if (!grid_fft_length_ok(d)) return cudaErrorInvalidValue;
+    if (rows_) {  // the engine's lengths
         d0 = is3d ? 2 * rp_.es : 1;
         d1 = is3d ? 2 * rp_.em : 2 * rp_.es;
         d2 = 2 * rp_.ef;
@@ -819,7 +827,9 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     }
     T_TRY(grid_fft_create(&gf1_, d0, d1, d2, 1));
     launches_ = 2;
-    return set_reg();
+    T_TRY(set_reg());
+    ready_ = true;
+    return cudaSuccess;
 }
 
 // Plan of one grid and room for `batch` of them.

@@ -91,6 +91,7 @@ private:
     cudaError_t ensure_grid_plan(const GridSpec &g, GridFft *plan, int batch);
 
     ToepConfig cfg_;
+    bool ready_ = false;       // the last set-up was completed
     SparseReg reg_;            // -reg: C and C^T on the device
     cudaStream_t st_ = nullptr;
     unsigned *err_ = nullptr;

@@ -4,7 +4,8 @@ next length), uneven coil counts and several segments; refused sizes stay refuse
 import numpy as np
 import pytest
 
-from test_toeplitz_gpu import TOL_OP, gpu_apply, grid_elems, opts_of, oracle_apply, rel
+from test_toeplitz_gpu import (TOL_OP, gpu_apply, gpu_fhd, gpu_q, gpu_recon, grid_elems, opts_of,
+                               oracle_apply, rel)
 
 pytestmark = pytest.mark.gpu
 
@@ -63,6 +64,27 @@ def test_sizes_past_the_table(pkg, ctx):
     c, Q, p = make((2 * 257, 4, 1), 1, 0, 6)
     with pytest.raises(pkg.ImpError):
         gpu_apply(pkg, ctx, opts_of(pkg, c), c, Q, p)
+
+
+@pytest.mark.parametrize("dims", [(514, 4, 1), (4, 2 * 257, 2), (2, 4, 514)])
+@pytest.mark.parametrize("padded", ["0", "1"])
+def test_refused_size_is_refused_again(pkg, monkeypatch, dims, padded):
+    """A second call of a refused size on the same context is refused like the first, by every
+    entry point, and the context then serves another size."""
+    monkeypatch.setenv("IMP_TOEP_PADDED", padded)
+    c, Q, p = make(dims, 1, 1, 6)
+    c["ky"] = c["kz"] = c["kx"]
+    c["kdata"] = np.ones((1, c["kx"].size), np.complex64)
+    ok, Qok, pok = make((16, 18, 1), 2, 1, 7)
+    with pkg.Context(0) as one:
+        o = opts_of(pkg, c)
+        for call in (lambda: gpu_apply(pkg, one, o, c, Q, p), lambda: gpu_fhd(pkg, one, o, c),
+                     lambda: gpu_q(pkg, one, o, c), lambda: gpu_recon(pkg, one, o, c, Q, p)):
+            for _ in range(2):
+                with pytest.raises(pkg.ImpError):
+                    call()
+        got = gpu_apply(pkg, one, opts_of(pkg, ok), ok, Qok, pok)
+        assert rel(got, oracle_apply(ok, Qok, pok, ok["fdp"])) < TOL_OP
 
 
 # (x, y, z): y is the slow (column) axis, x the middle one, z the contiguous one
