@@ -57,3 +57,12 @@ def test_batch_solver_reuse(pkg, synth):
         for a in runs:
             with pkg.Context(0) as fresh:
                 assert np.array_equal(call(one, *a), call(fresh, *a))
+
+
+def test_new_context_takes_no_work_memory(pkg):
+    """A context's work memory comes with the calls that need it."""
+    import torch
+    pkg.Context(0).close()
+    before = torch.cuda.mem_get_info()[0]
+    with pkg.Context(0):
+        assert before - torch.cuda.mem_get_info()[0] < 4 << 20
