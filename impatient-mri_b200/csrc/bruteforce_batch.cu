@@ -455,11 +455,13 @@ cudaError_t BfBatch::place_inputs(const float *kx, const float *ky, const float 
     return cudaSuccess;
 }
 
-// Per-slice table of one direction for a given split (see NuSlice).
+// Per-slice table of one direction for a given split (see NuSlice), which has to cut
+// every slice's "theirs" range into whole tiles: the kernels drop what is left over.
 cudaError_t BfBatch::set_table(bool adj, int split) {
     const int S = S_, G = plan_.G, CG = plan_.CG, Npad = plan_.Npad;
     std::vector<NuSlice> tab(S);
     for (int s = 0; s < S; ++s) {
+        if (!nu_split_ok(adj ? mpad_[s] : Npad, split)) return cudaErrorInvalidValue;
         const long long ko = koff_pad_[s];
         tab[s] = adj ? NuSlice{(long long)s * Npad, ko, (long long)G * CG * ko,
                                (long long)s * split * G * Npad, Npad, mpad_[s], mpad_[s] / split}
@@ -484,13 +486,20 @@ cudaError_t BfBatch::tune_shapes(bool adj) {
     const int G = plan_.G, CG = plan_.CG, Npad = plan_.Npad;
     const NuBatchKey key{adj ? 1 : 0, CG, G, plan_.use_z ? 1 : 0, S_, Npad, max_mpad_,
                          mpad_total_, l.tc};
+    const std::vector<int> ranges = adj ? mpad_ : std::vector<int>{Npad};
     NuLaunch cached;
     if (nu_batch_lookup(key, &cached)) {
-        l = cached;
-        return cudaSuccess;
+        // The key holds the slices' largest and summed lengths only: a split found for
+        // other slices may not cut these into whole tiles.  Tuning again then stores a
+        // smaller split, which is a legal one for both.
+        bool ok = true;
+        for (int r : ranges) ok = ok && nu_split_ok(r, cached.split);
+        if (ok) {
+            l = cached;
+            return cudaSuccess;
+        }
     }
     if (!nu_tuning_enabled()) return cudaSuccess;
-    const std::vector<int> ranges = adj ? mpad_ : std::vector<int>{Npad};
     auto split_ok = [&](int sp) {
         for (int r : ranges)
             if (!nu_split_ok(r, sp) || r / sp < 2 * kTile) return false;

@@ -1,6 +1,10 @@
 """Brute-force CG on the GPU against the reference's FP64 recon (golden
 vectors) and the FP64 oracle.  Tolerance: 1e-4 relative L2 on the final
 image after the same iteration count and semantics (cg_num-1 updates)."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -466,3 +470,54 @@ def test_batch_tuned_shapes_are_cached(pkg, ctx, synth, monkeypatch, tmp_path):
         got = images[0][s * N:(s + 1) * N]
         ref = oracle.bf_cg(c, cg_num=6, tv=False, tv_num=1, eps=1e-6, use_z=0)
         assert oracle.rel_l2(got, ref) < TOL_IMG, s
+
+
+_OTHER_SLICES = """
+import os, sys
+sys.path[:0] = [{root!r}, {tests!r}]
+import numpy as np
+from __graft_entry__ import load_package
+pkg = load_package()
+C, n, counts = {C}, 16, (8192, 7168, 1024)
+rng = np.random.default_rng(C)
+f32 = lambda a: np.ascontiguousarray(a, np.float32)
+off = np.cumsum((0,) + counts)
+N, M, S = n * n, int(off[-1]), len(counts)
+g = f32((np.arange(n) - n / 2) / n)
+ix, iy = np.repeat(g, n), np.tile(g, n)
+kx, ky = (f32(rng.uniform(-n / 2, n / 2, M)) for _ in range(2))
+t, fm = f32(rng.uniform(0, 0.01, M)), f32(rng.uniform(-300, 300, S * N))
+d = [f32(rng.standard_normal(C * M)) for _ in range(2)]
+s = [f32(rng.standard_normal(C * N)) for _ in range(2)]
+out = []
+for tune in ("1", "0"):
+    os.environ["IMP_AUTOTUNE"] = tune
+    xr, xi = np.zeros(S * N, np.float32), np.zeros(S * N, np.float32)
+    with pkg.Context(0) as c:
+        pkg.bruteForceBatch(c, pkg.bf_options(cg_num=2, dims=(n, n, 1)), xr, xi, *d, kx, ky, 0 * kx,
+                            t, off, ix, iy, 0 * ix, fm, *s, N, C)
+    out.append(xr + 1j * xi)
+print("REL", np.linalg.norm(out[0] - out[1]) / np.linalg.norm(out[1]))
+"""
+
+
+@pytest.mark.parametrize("C,CG,tc", [(4, 4, 0), (12, 16, 2)])
+def test_batch_cached_split_of_other_slices(tmp_path, C, CG, tc):
+    """A cached split that was found for slices of the same number, largest and summed length,
+    but does not cut this batch's slices into whole tiles (8192, 7168 and 1024 samples by 32),
+    is not used: the image is that of the untuned shapes and the cache gets a legal split."""
+    from pathlib import Path
+    here = Path(__file__).resolve().parent
+    cache = tmp_path / "tune.txt"
+    cache.write_text(f"b1 1 {CG} 1 0 3 1024 8192 16384 {tc} {2 if tc else 4} 4 32 0.1\n")
+    env = dict(os.environ, IMP_TUNE_CACHE=str(cache))
+    env.pop("IMP_NUDFT_TC", None)
+    code = _OTHER_SLICES.format(root=str(here.parent), tests=str(here), C=C)
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    # the same sums in another order: one update, FP32
+    assert float(r.stdout.split("REL")[1]) < 1e-5
+    adj = [ln.split() for ln in cache.read_text().splitlines() if ln.startswith("b1 1 ")]
+    assert len(adj) == 2 and adj[0][1:10] == adj[1][1:10]  # the same problem, tuned again
+    assert all(m % (64 * int(adj[1][12])) == 0 for m in (8192, 7168, 1024))
