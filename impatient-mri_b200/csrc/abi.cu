@@ -29,6 +29,7 @@ imp_status fail(imp_status s, const std::string &msg) {
 
 imp_status from_cuda(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return IMP_OK;
+    cudaGetLastError();  // reported here: not by the next call's first launch
     const imp_status s = e == cudaErrorMemoryAllocation ? IMP_ERR_NOMEM : IMP_ERR_CUDA;
     return fail(s, std::string(what) + ": " + cudaGetErrorString(e));
 }

@@ -277,6 +277,7 @@ cudaError_t BfSolver::profile_collect(double ms[2], long count[2]) {
 }
 
 void BfSolver::release() {
+    ready_ = false;
     if (g_iter_) cudaGraphExecDestroy(g_iter_);
     if (g_init_) cudaGraphExecDestroy(g_init_);
     g_iter_ = g_init_ = nullptr;
@@ -295,10 +296,11 @@ cudaError_t BfSolver::setup(const BfConfig &cfg, const float *kx, const float *k
                             const float *kz, const float *t, const float *ix, const float *iy,
                             const float *iz, const float *sensi_r, const float *sensi_i,
                             unsigned *dev_err, cudaStream_t st) {
-    const bool same_shape = plan_.kgeo && st == st_ && dev_err == err_ && cfg.M == cfg_.M &&
+    const bool same_shape = ready_ && st == st_ && dev_err == err_ && cfg.M == cfg_.M &&
                             cfg.N == cfg_.N && cfg.C == cfg_.C && cfg.use_z == cfg_.use_z &&
                             cfg.n0 == cfg_.n0 && cfg.n1 == cfg_.n1 && cfg.n2 == cfg_.n2 &&
                             cfg.autotune == cfg_.autotune;
+    ready_ = false;  // until this set-up is complete
     if (same_shape) {
         // keep buffers, tuned launch shapes and (if the captured scalars match) the graphs
         bool stale = cfg.fd != cfg_.fd || cfg.lambda != cfg_.lambda;
@@ -310,7 +312,9 @@ cudaError_t BfSolver::setup(const BfConfig &cfg, const float *kx, const float *k
             if (g_init_) cudaGraphExecDestroy(g_init_);
             g_iter_ = g_init_ = nullptr;
         }
-        return nu_plan_repack(plan_, kx, ky, kz, t, ix, iy, iz, sensi_r, sensi_i, dev_err, st);
+        IMP_TRY(nu_plan_repack(plan_, kx, ky, kz, t, ix, iy, iz, sensi_r, sensi_i, dev_err, st));
+        ready_ = true;
+        return cudaSuccess;
     }
     release();
     cfg_ = cfg;
@@ -349,7 +353,9 @@ cudaError_t BfSolver::setup(const BfConfig &cfg, const float *kx, const float *k
     IMP_TRY(cudaMemsetAsync(dots_, 0, sizeof(double) * 5 * kDotBlocks, st_));
     bool moved = false;
     IMP_TRY(set_reg(&moved));
-    return cudaGetLastError();
+    IMP_TRY(cudaGetLastError());
+    ready_ = true;
+    return cudaSuccess;
 }
 
 // Uploads (or drops) the -reg matrix of cfg_; *graphs_stale when the penalty

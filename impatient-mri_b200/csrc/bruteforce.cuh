@@ -64,6 +64,7 @@ private:
     cudaError_t set_reg(bool *graphs_stale);
 
     BfConfig cfg_;
+    bool ready_ = false;      // the last set-up was completed
     NuPlan plan_;
     SparseReg reg_;           // -reg: C and C^T on the device
     cudaStream_t st_ = nullptr;
