@@ -316,13 +316,29 @@ cudaError_t BfSolver::setup(const BfConfig &cfg, const float *kx, const float *k
         ready_ = true;
         return cudaSuccess;
     }
-    release();
     cfg_ = cfg;
     st_ = st;
     err_ = dev_err;
+    // The FP16 kernel's image is optional: where it leaves no room for the rest, the
+    // set-up is done without it (the TF32 kernel).
+    cudaError_t e = build(kx, ky, kz, t, ix, iy, iz, sensi_r, sensi_i, true);
+    if (e == cudaErrorMemoryAllocation && plan_.img_bytes) {
+        cudaGetLastError();
+        e = build(kx, ky, kz, t, ix, iy, iz, sensi_r, sensi_i, false);
+    }
+    ready_ = e == cudaSuccess;
+    return e;
+}
+
+// Plan, buffers and launch shapes of cfg_.
+cudaError_t BfSolver::build(const float *kx, const float *ky, const float *kz, const float *t,
+                            const float *ix, const float *iy, const float *iz,
+                            const float *sensi_r, const float *sensi_i, bool image) {
+    release();
+    const BfConfig &cfg = cfg_;
     // field map is set per slice in solve()
     IMP_TRY(nu_plan_create(plan_, kx, ky, kz, t, ix, iy, iz, nullptr, sensi_r, sensi_i, cfg.M,
-                           cfg.N, cfg.C, cfg.use_z, dev_err, st));
+                           cfg.N, cfg.C, cfg.use_z, image, err_, st_));
     const size_t nk = (size_t)plan_.G * plan_.Mpad * plan_.CG;
     const size_t nxs = (size_t)plan_.G * plan_.Npad * plan_.CG;
     IMP_TRY(dalloc(&y_, nk));
@@ -353,9 +369,8 @@ cudaError_t BfSolver::setup(const BfConfig &cfg, const float *kx, const float *k
     IMP_TRY(cudaMemsetAsync(dots_, 0, sizeof(double) * 5 * kDotBlocks, st_));
     bool moved = false;
     IMP_TRY(set_reg(&moved));
-    IMP_TRY(cudaGetLastError());
-    ready_ = true;
-    return cudaSuccess;
+    if (plan_.img_bytes && !nu_room_beside_image()) return cudaErrorMemoryAllocation;
+    return cudaGetLastError();
 }
 
 // Uploads (or drops) the -reg matrix of cfg_; *graphs_stale when the penalty

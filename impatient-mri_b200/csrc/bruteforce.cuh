@@ -62,6 +62,9 @@ private:
     size_t prof_used_ = 0;
 
     cudaError_t set_reg(bool *graphs_stale);
+    cudaError_t build(const float *kx, const float *ky, const float *kz, const float *t,
+                      const float *ix, const float *iy, const float *iz, const float *sensi_r,
+                      const float *sensi_i, bool image);
 
     BfConfig cfg_;
     bool ready_ = false;      // the last set-up was completed
@@ -113,6 +116,9 @@ private:
     cudaError_t run_iteration();
     cudaError_t set_table(bool adj, int split);
     cudaError_t tune_shapes(bool adj);
+    cudaError_t build(int S, const int *k_off, const float *kx, const float *ky, const float *kz,
+                      const float *t, const float *ix, const float *iy, const float *iz,
+                      const float *fm, const float *sensi_r, const float *sensi_i, bool image);
 
     BfConfig cfg_;
     cudaError_t place_inputs(const float *kx, const float *ky, const float *kz, const float *t,

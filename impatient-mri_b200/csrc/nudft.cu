@@ -568,7 +568,8 @@ static cudaError_t pack_geometry(NuPlan &p, const float *kx, const float *ky, co
 cudaError_t nu_plan_create(NuPlan &p, const float *kx, const float *ky, const float *kz,
                            const float *t, const float *ix, const float *iy, const float *iz,
                            const float *fm, const float *sensi_r, const float *sensi_i, int M,
-                           int N, int C, bool use_z, unsigned *dev_err, cudaStream_t st) {
+                           int N, int C, bool use_z, bool image, unsigned *dev_err,
+                           cudaStream_t st) {
     nu_plan_destroy(p);
     p.M = M;
     p.N = N;
@@ -583,7 +584,7 @@ cudaError_t nu_plan_create(NuPlan &p, const float *kx, const float *ky, const fl
     if ((e = cudaMalloc(&p.vgeo, sizeof(double4) * p.Npad)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&p.sens, sizeof(float2) * (size_t)p.G * p.Npad * p.CG)) != cudaSuccess)
         return e;
-    if (nu_wants_image(p.CG)) nu_plan_reserve_image(p);
+    if (image && nu_wants_image(p.CG)) nu_plan_reserve_image(p);
     p.fwd = nu_default_launch(p, false);
     p.adj = nu_default_launch(p, true);
     return pack_geometry(p, kx, ky, kz, t, ix, iy, iz, fm, sensi_r, sensi_i, dev_err, st);
@@ -600,6 +601,11 @@ void nu_plan_reserve_image(NuPlan &p) {
         cudaGetLastError();
         p.img = nullptr;
     }
+}
+
+bool nu_room_beside_image() {
+    size_t free_b = 0, total = 0;
+    return cudaMemGetInfo(&free_b, &total) == cudaSuccess && free_b >= ((size_t)64 << 20);
 }
 
 cudaError_t nu_plan_repack(NuPlan &p, const float *kx, const float *ky, const float *kz,

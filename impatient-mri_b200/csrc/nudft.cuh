@@ -45,11 +45,13 @@ struct NuPlan {
 };
 
 // Creates geometry and packed sensitivities from device SoA inputs.
-// sensi_r/sensi_i may be null (unit sensitivity, C must be 1).
+// sensi_r/sensi_i may be null (unit sensitivity, C must be 1).  `image`: with the FP16
+// tensor-core kernel's image where the coil grouping uses it and the memory is there.
 cudaError_t nu_plan_create(NuPlan &p, const float *kx, const float *ky, const float *kz,
                            const float *t, const float *ix, const float *iy, const float *iz,
                            const float *fm, const float *sensi_r, const float *sensi_i, int M,
-                           int N, int C, bool use_z, unsigned *dev_err, cudaStream_t st);
+                           int N, int C, bool use_z, bool image, unsigned *dev_err,
+                           cudaStream_t st);
 // Re-packs geometry and sensitivities of the same sizes into an existing plan.
 cudaError_t nu_plan_repack(NuPlan &p, const float *kx, const float *ky, const float *kz,
                            const float *t, const float *ix, const float *iy, const float *iz,
@@ -71,6 +73,9 @@ void nu_plan_destroy(NuPlan &p);
 // Gives the plan the FP16 tensor-core kernel's image for both directions (of
 // the plan's own sizes).  Without the memory the plan goes on without it.
 void nu_plan_reserve_image(NuPlan &p);
+// Whether a complete set-up that holds an image leaves room for what comes with the
+// first launches (code, graphs).
+bool nu_room_beside_image();
 
 // Heuristic launch shape (replaced by the autotuner when enabled).
 NuLaunch nu_default_launch(const NuPlan &p, bool adj);

@@ -170,7 +170,8 @@ bool nu_tuned_lookup(const NuPlan &p, bool adj, NuLaunch *out) {
     auto it = g_cache.find(key_of(p, adj));
     if (it == g_cache.end()) return false;
     if (it->second.tc && !nu_tc_enabled()) return false;
-    if (it->second.tc == 2 && !p.img_bytes) return false;
+    // the tensor-core kernel that this plan has: FP16 with the image, TF32 without
+    if (it->second.tc && (it->second.tc == 2) != (p.img_bytes != 0)) return false;
     *out = it->second;
     return true;
 }
@@ -241,6 +242,8 @@ cudaError_t nu_autotune(const NuPlan &p, bool adj, const float2 *tdata, float2 *
     cudaEventDestroy(e1);
     if (e != cudaSuccess) return e;
     *out = best_l;
+    // a shape found while the memory lacked the image is not kept for later plans
+    if (nu_wants_image(p.CG) && !p.img_bytes) return cudaSuccess;
     std::lock_guard<std::mutex> g(g_mu);
     load_locked();
     g_cache[key_of(p, adj)] = best_l;

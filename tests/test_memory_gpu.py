@@ -83,3 +83,25 @@ def test_failed_setup_is_done_again(pkg, what, C):
                     with pytest.raises(pkg.ImpError, match="(?i)memory"):
                         call(one)
         assert np.array_equal(call(one), want)
+
+
+@pytest.mark.parametrize("slices", [0, 2])
+def test_optional_image_gives_way(pkg, monkeypatch, slices):
+    """12 coils (the FP16 kernel and its image of the k-space data) with room for everything but
+    half of that image: the call is served, by the TF32 kernel."""
+    monkeypatch.setenv("IMP_AUTOTUNE", "0")
+    M = 1 << 19
+    image = M * 16 * 16  # bytes: 16 per sample and coil of the group
+    call = brute_force(pkg, 12, M // max(slices, 1), slices)
+    with pkg.Context(0) as ctx:
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        before = torch.cuda.mem_get_info()[0]
+        want = call(ctx)
+        torch.cuda.empty_cache()
+        used = before - torch.cuda.mem_get_info()[0]
+    assert used > 2 * image
+    with pkg.Context(0) as ctx, leave(used - image // 2):
+        got = call(ctx)
+    # one CG update of FP16- and TF32-split sums, both 22 bits
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < 1e-5
