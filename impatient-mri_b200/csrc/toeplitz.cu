@@ -111,7 +111,7 @@ __device__ __forceinline__ float kb_transform(float u, float beta) {
 }
 
 // Scatter gridding, one warp per sample: each sample's separable KB footprint
-// is added into the ifftshifted position (X + gs/2) mod gs of every cell X it
+// is added into the ifftshifted position (X - gs/2) mod gs of every cell X it
 // covers (ready for the inverse FFT), for a batch of grids at once: segments
 // [l0, l0 + nl) x coils [0, nc) of dr / di, grid (l - l0) nc + c at
 // `cells` elements each.  Without data (Q: the samples' real window values) a
@@ -208,14 +208,16 @@ __global__ void __launch_bounds__(kGridWarps * 32, kGridBlocks)
                 }
             }
             __syncwarp();
-            // Shifted index lo + j + gs / 2 of a covered cell is below 2 gs: it wraps
-            // at most once (one conditional subtraction, no division per cell).  The
-            // loop axis steps by a fixed stride and wraps once.  (Aligned pairs of
-            // cells as 16-byte atomics measured no faster: 5.32 against 5.22 ms for Q of
-            // 128x128x32 when a grid held one segment.)
+            // A covered cell's shifted index is lo + j - gs / 2 modulo gs; with + (gs + 1) / 2
+            // instead it is below 2 gs and wraps at most once (one conditional subtraction, no
+            // division per cell).  gs is odd where an axis' oversampled length, rounded up in
+            // FP32, passes the multiple of four it was made for (z: 61 for 38 at 1.5).  The loop
+            // axis steps by a fixed stride and wraps once.  (Aligned pairs of cells as 16-byte
+            // atomics measured no faster: 5.32 against 5.22 ms for Q of 128x128x32 when a grid
+            // held one segment.)
             float2 *gl = grid + (size_t)(l - (dr ? l0 : l0 >> 1)) * nc * cells;
             const int nbc = cnt[B] * cnt[Cc];
-            int a0 = D3 ? lo[A] + g.gs[A] / 2 : 0;
+            int a0 = D3 ? lo[A] + (g.gs[A] + 1) / 2 : 0;
             if (a0 >= g.gs[A]) a0 -= g.gs[A];
             const size_t astride = D3 ? (size_t)g.gs[1] * g.gs[2] : 0;
             const size_t awrap = astride * g.gs[A];
@@ -224,9 +226,9 @@ __global__ void __launch_bounds__(kGridWarps * 32, kGridBlocks)
                 const int jb = p / cnt[Cc], jc = p - jb * cnt[Cc];
                 const float wbc = ws[B][jb] * ws[Cc][jc];
                 if (wbc == 0.f) continue;
-                int ib = lo[B] + jb + g.gs[B] / 2;
+                int ib = lo[B] + jb + (g.gs[B] + 1) / 2;
                 if (ib >= g.gs[B]) ib -= g.gs[B];
-                int ic = lo[Cc] + jc + g.gs[Cc] / 2;
+                int ic = lo[Cc] + jc + (g.gs[Cc] + 1) / 2;
                 if (ic >= g.gs[Cc]) ic -= g.gs[Cc];
                 size_t cell = (size_t)a0 * astride + (size_t)ib * rowlen + ic;
                 int ia = a0;
@@ -298,9 +300,9 @@ __device__ __forceinline__ GridAt grid_at(const GridSpec &g, int x, int y, int z
     GridAt r{0, 0, 1.f};
     float kern = 1.f;
     for (int a = 0; a < 3; ++a) {
-        // c + gs/2 - img/2 + gs/2, below 2 gs
-        int j = c[a] + 2 * (g.gs[a] / 2) - g.img[a] / 2;
-        if (j >= g.gs[a]) j -= g.gs[a];
+        // the centred crop, shifted: c - img/2 modulo gs
+        int j = c[a] - g.img[a] / 2;
+        if (j < 0) j += g.gs[a];
         r.idx = r.idx * g.gs[a] + j;
         r.neg = r.neg * g.gs[a] + (j ? g.gs[a] - j : 0);
         if (a < 2 || g.is3d)

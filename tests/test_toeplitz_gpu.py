@@ -480,3 +480,32 @@ def test_q_segment_pairs_match_oracle(pkg, ctx, dims, L, os):
     want = np.asarray(T.compute_q(c["kx"], c["ky"], c["kz"], c["t"], dims, L, os))
     for l in range(L + 1):
         assert rel(got.reshape(L + 1, -1)[l], want.reshape(L + 1, -1)[l]) < 2 * TOL_OP
+
+
+@pytest.mark.parametrize("nz,os_fh", [(38, 1.5), (42, 1.125)])
+def test_odd_grids_match_oracle(pkg, ctx, nz, os_fh):
+    """The grid along z is rounded up from an FP32 product and can come out odd (61 for 38 at the
+    default oversampling 1.5, 49 for 42 at 1.125; Q's 97 for 84): shifts, crop and the pairs of
+    segments of such grids."""
+    dims, L, M, C = (12, 10, nz), 3, 300, 2
+    n_q = tuple(2 * v for v in dims)
+    assert T.grid_size(T.rounded_os(os_fh, dims), dims)[2] % 2 == 1
+    assert T.grid_size(T.rounded_os(1.125, (n_q[0], n_q[1], 84)), (n_q[0], n_q[1], 84))[2] == 97
+    rng = np.random.default_rng(nz)
+    nx, ny, _ = dims
+    N = nx * ny * nz
+    cplx = lambda *s: (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+    c = dict(dims=dims, L=L, cg=1, fdp=1e-2, tv_num=0, os_q=1.125, os_fh=os_fh,
+             t=np.sort(rng.uniform(0.0, 0.01, M)).astype(np.float32),
+             kx=rng.uniform(-nx / 2, nx / 2 - 0.1, M).astype(np.float32),
+             ky=rng.uniform(-ny / 2, ny / 2 - 0.1, M).astype(np.float32),
+             kz=rng.uniform(-nz / 2, nz / 2 - 0.1, M).astype(np.float32),
+             fm=rng.uniform(-300.0, 300.0, N).astype(np.float32), sens=cplx(C, N),
+             kdata=cplx(C, M))
+    want = T.compute_fhd(c["kx"], c["ky"], c["kz"], c["t"], dims, L, os_fh, c["kdata"], c["sens"],
+                         c["fm"])
+    assert rel(gpu_fhd(pkg, ctx, opts_of(pkg, c), c), np.asarray(want).reshape(-1)) < TOL_OP
+    got = gpu_q(pkg, ctx, opts_of(pkg, c), c)
+    want = np.asarray(T.compute_q(c["kx"], c["ky"], c["kz"], c["t"], dims, L, 1.125))
+    for l in range(L + 1):
+        assert rel(got[l], want.reshape(L + 1, -1)[l]) < 2 * TOL_OP
