@@ -691,25 +691,41 @@ GridSpec grid_spec(const int img[3], float os, bool beta_after_rounding, float k
 
 ToepSolver::~ToepSolver() { release(); }
 
+static void free_plan(GridFft *f) {
+    grid_fft_destroy(f);
+    *f = GridFft();
+}
+
 void ToepSolver::release() {
-    if (g_iter_) cudaGraphExecDestroy(g_iter_);
-    g_iter_ = nullptr;
-    for (GridFft *f : {&gf2_, &gf1_, &gfq_, &gff_}) {
-        grid_fft_destroy(f);
-        *f = GridFft();
-    }
-    reg_.release();
-    void *bufs[] = {sens_, eph_, fm_, qf_, big_, x_, r_, p_, q_, best_, fhd_, w_, dots_,
-                    t_, grid_, qf2_, b0_, b1_, tw_[0], tw_[1], tw_[2]};
-    for (void *b : bufs)
+    release_cg();
+    free_plan(&gfq_);
+    free_plan(&gff_);
+    for (void *b : {(void *)sens_, (void *)eph_, (void *)fm_, (void *)fhd_, (void *)t_,
+                    (void *)grid_})
         if (b) cudaFree(b);
-    sens_ = eph_ = qf_ = big_ = x_ = r_ = p_ = q_ = best_ = fhd_ = grid_ = nullptr;
-    qf2_ = b0_ = b1_ = tw_[0] = tw_[1] = tw_[2] = nullptr;
-    rows_ = false;
-    fm_ = w_ = t_ = nullptr;
-    dots_ = nullptr;
+    sens_ = eph_ = fhd_ = grid_ = nullptr;
+    fm_ = t_ = nullptr;
     grid_cells_ = 0;
     ready_ = false;
+}
+
+// What F^H F and the CG hold beside the set-up.
+void ToepSolver::release_cg() {
+    if (g_iter_) cudaGraphExecDestroy(g_iter_);
+    g_iter_ = nullptr;
+    free_plan(&gf2_);
+    free_plan(&gf1_);
+    reg_.release();
+    void *bufs[] = {qf_, big_, x_,  r_,  p_,  q_,     best_,  w_,
+                    dots_, qf2_, b0_, b1_, tw_[0], tw_[1], tw_[2]};
+    for (void *b : bufs)
+        if (b) cudaFree(b);
+    qf_ = big_ = x_ = r_ = p_ = q_ = best_ = nullptr;
+    qf2_ = b0_ = b1_ = tw_[0] = tw_[1] = tw_[2] = nullptr;
+    w_ = nullptr;
+    dots_ = nullptr;
+    rows_ = false;
+    cg_ready_ = false;
 }
 
 cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float *fm,
@@ -717,10 +733,12 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
                               cudaStream_t st) {
     // Same sizes and stream: keep buffers, FFT plans and (same CG terms) the
     // captured iteration graph; only the per-call inputs are refreshed.
-    const bool same_shape = ready_ && st == st_ && cfg.q_only == cfg_.q_only &&
-                            cfg.nx == cfg_.nx && cfg.ny == cfg_.ny && cfg.nz == cfg_.nz &&
-                            cfg.C == cfg_.C && cfg.M == cfg_.M && (int)cfg.ntime_segs == L_;
+    const bool like = st == st_ && cfg.q_only == cfg_.q_only && cfg.nx == cfg_.nx &&
+                      cfg.ny == cfg_.ny && cfg.nz == cfg_.nz && cfg.C == cfg_.C &&
+                      cfg.M == cfg_.M && (int)cfg.ntime_segs == L_;
+    const bool same_shape = ready_ && like;
     ready_ = false;  // until this set-up is complete
+    if (!like) lean_ = 0;
     if (same_shape) {
         if (g_iter_ && (cfg.fd != cfg_.fd || cfg.lambda != cfg_.lambda ||
                         cfg.use_graphs != cfg_.use_graphs)) {
@@ -744,8 +762,8 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
             k_eph<<<gridn((size_t)L1 * N_), kVB, 0, st>>>(eph_, fm, N_, L1, tau_, t0_);
             launches_ = 2;
             T_TRY(cudaGetLastError());
-            T_TRY(set_reg());
         }
+        if (cfg.cg) T_TRY(prepare_cg());
         ready_ = true;
         return cudaSuccess;
     }
@@ -792,14 +810,50 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     }
     T_TRY(cudaMalloc(&sens_, sizeof(float2) * C * N_));
     T_TRY(cudaMalloc(&eph_, sizeof(float2) * L1 * N_));
+    if (cfg.cg) T_TRY(prepare_cg());
+    T_TRY(cudaMalloc(&fhd_, sizeof(float2) * N_));
+    k_pack_sens_c<<<gridn((size_t)C * N_), kVB, 0, st>>>(sens_, sensi_r, sensi_i, (size_t)C * N_);
+    k_eph<<<gridn((size_t)L1 * N_), kVB, 0, st>>>(eph_, fm, N_, L1, tau_, t0_);
+    T_TRY(cudaGetLastError());
+    launches_ = 2;
+    ready_ = true;
+    return cudaSuccess;
+}
+
+// Buffers and plans of F^H F and the CG, and the -reg matrix of cfg_; kept from the first
+// call that needs them on (F^H d does not: 64x64 x 4 coils, first call 0.93 -> 0.53 ms).
+cudaError_t ToepSolver::prepare_cg() {
+    if (!cg_ready_) T_TRY(build_cg());
+    cg_ready_ = true;
+    return set_reg();
+}
+
+// After a call that ran out of memory: gives back what it can, so that the same call needs
+// less.  1: gridding grids one at a time, F^H F with one transform and one Qf_l at a time;
+// 2: F^H F on the zero-padded chain, whose transforms are no longer than the doubled image.
+bool ToepSolver::shrink() {
+    if (lean_ >= (cfg_.q_only ? 1 : 2)) return false;
+    ++lean_;
+    release_cg();
+    if (grid_) cudaFree(grid_);
+    grid_ = nullptr;
+    grid_cells_ = 0;
+    return true;
+}
+
+cudaError_t ToepSolver::build_cg() {
+    release_cg();
+    const bool is3d = cfg_.nz > 1;
+    const int L1 = L_ + 1, C = cfg_.C;
     // Sides up to the engine's longest length run on the pruned mixed-radix
     // engine; others (and IMP_TOEP_PADDED=1) use the zero-padded chain on the
     // grid transform.
     const char *force_padded = std::getenv("IMP_TOEP_PADDED");
-    const bool pruned = !(force_padded && force_padded[0] == '1');
+    const bool pruned = lean_ < 2 && !(force_padded && force_padded[0] == '1');
     rows_ = pruned && toep_rows_plan(nv[0], is3d ? nv[1] : 1, is3d ? nv[2] : nv[1], C, L1, &rp_);
     if (rows_) {
-        qf_segs_ = (int)std::min<size_t>(
+        if (lean_) rp_.chunk = 1;
+        qf_segs_ = lean_ ? 1 : (int)std::min<size_t>(
             L1, std::max<size_t>(1, ((size_t)128 << 20) / (sizeof(float2) * rp_.q_elems())));
         T_TRY(cudaMalloc(&qf_, sizeof(float2) * rp_.q_elems() * qf_segs_));
         T_TRY(cudaMalloc(&qf2_, sizeof(float2) * rp_.q_elems() * L1));
@@ -810,13 +864,10 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
         T_TRY(cudaMalloc(&qf_, sizeof(float2) * L1 * G2_));
         T_TRY(cudaMalloc(&big_, sizeof(float2) * C * G2_));
     }
-    for (float2 **b : {&x_, &r_, &p_, &q_, &best_, &fhd_}) T_TRY(cudaMalloc(b, sizeof(float2) * N_));
+    for (float2 **b : {&x_, &r_, &p_, &q_, &best_}) T_TRY(cudaMalloc(b, sizeof(float2) * N_));
     T_TRY(cudaMalloc(&w_, sizeof(float) * N_));
     T_TRY(cudaMalloc(&dots_, sizeof(double) * (T_SCAL * kTBlocks + 8)));
-    T_TRY(cudaMemsetAsync(dots_, 0, sizeof(double) * (T_SCAL * kTBlocks + 8), st));
-    k_pack_sens_c<<<gridn((size_t)C * N_), kVB, 0, st>>>(sens_, sensi_r, sensi_i, (size_t)C * N_);
-    k_eph<<<gridn((size_t)L1 * N_), kVB, 0, st>>>(eph_, fm, N_, L1, tau_, t0_);
-    T_TRY(cudaGetLastError());
+    T_TRY(cudaMemsetAsync(dots_, 0, sizeof(double) * (T_SCAL * kTBlocks + 8), st_));
     // the 2N grid: batched over the coils for the zero-padded chain, single
     // for Qf_l (2-D grids are [n2[0]][n2[1]], 3-D [n2[0]][n2[1]][n2[2]])
     int d0 = is3d ? n2[0] : 1, d1 = is3d ? n2[1] : n2[0], d2 = is3d ? n2[2] : n2[1];
@@ -828,9 +879,6 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
         T_TRY(grid_fft_create(&gf2_, d0, d1, d2, C));
     }
     T_TRY(grid_fft_create(&gf1_, d0, d1, d2, 1));
-    launches_ = 2;
-    T_TRY(set_reg());
-    ready_ = true;
     return cudaSuccess;
 }
 
@@ -854,8 +902,8 @@ cudaError_t ToepSolver::ensure_grid_plan(const GridSpec &g, GridFft *plan, int b
 
 // Gridding grids per batch: as many as half of the L2 holds (the scatter's
 // atomics, the transform and the crop then stay in L2), at least one.
-static size_t grid_batch(const GridSpec &g) {
-    return std::max<size_t>(1, ((size_t)64 << 20) / (sizeof(float2) * g.cells()));
+static size_t grid_batch(const GridSpec &g, bool lean) {
+    return lean ? 1 : std::max<size_t>(1, ((size_t)64 << 20) / (sizeof(float2) * g.cells()));
 }
 
 cudaError_t ToepSolver::compute_q(const float *kx, const float *ky, const float *kz,
@@ -864,7 +912,7 @@ cudaError_t ToepSolver::compute_q(const float *kx, const float *ky, const float 
     const int img[3] = {2 * cfg_.nx, 2 * cfg_.ny, is3d ? 2 * cfg_.nz : 1};
     const GridSpec g = grid_spec(img, cfg_.os_q, true, 2.0f);
     // two segments per grid
-    const int nb = (int)std::min<size_t>(grid_batch(g), L_ / 2 + 1);
+    const int nb = (int)std::min<size_t>(grid_batch(g, lean_ > 0), L_ / 2 + 1);
     T_TRY(ensure_grid_plan(g, &gfq_, nb));
     const NV n2d{{n2[0], n2[1], n2[2]}};
     const Crop crop = crop_of(g, true);
@@ -915,7 +963,7 @@ cudaError_t ToepSolver::compute_fhd(const float *kx, const float *ky, const floa
     const int img[3] = {cfg_.nx, cfg_.ny, cfg_.nz};
     const GridSpec g = grid_spec(img, cfg_.os_fh, false, 1.0f);
     // batches of coils x segments: the coils of a launch share each sample's weights
-    const size_t room = grid_batch(g);
+    const size_t room = grid_batch(g, lean_ > 0);
     const int nc_b = (int)std::min<size_t>(room, std::min(cfg_.C, kGridCoils));
     const int nl_b = (int)std::min<size_t>(std::max<size_t>(room / nc_b, 1), L_ + 1);
     T_TRY(ensure_grid_plan(g, &gff_, nc_b * nl_b));
@@ -1217,6 +1265,17 @@ imp::ToepSolver &solver_q_of(imp_context *ctx) {
     return *ctx->tp_q;
 }
 
+// Makes a call, and while it runs out of device memory, once more with less work memory
+// (nothing of a call's in- and outputs is written before its last allocation).
+template <class F>
+imp_status in_less_memory(imp_context *ctx, F call) {
+    imp_status s = call();
+    while (s == IMP_ERR_NOMEM &&
+           ((ctx->tp && ctx->tp->shrink()) || (ctx->tp_q && ctx->tp_q->shrink())))
+        s = call();
+    return s;
+}
+
 imp_status copy_out(imp_context *ctx, float *dst, const float *src, size_t n) {
     IMP_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream),
              "output D2H");
@@ -1245,32 +1304,34 @@ imp_status imp_toeplitz_q(imp_context *ctx, const imp_toeplitz_options *opt, flo
     if (s != IMP_OK) return s;
     if (!q_r || !q_i || !kx || !ky || !t || (nz > 1 && !kz))
         return fail(IMP_ERR_INVALID_ARG, "null array argument");
-    if ((s = imp::begin(ctx)) != IMP_OK) return s;
-    imp::stage_reset(ctx);
-    DevKeep keep;
-    const float *dkx, *dky, *dkz = nullptr, *dt;
-    if ((s = imp::to_device_staged(ctx, kx, num_k, &dkx, nullptr)) ||
-        (s = imp::to_device_staged(ctx, ky, num_k, &dky, nullptr)) ||
-        (s = imp::to_device_staged(ctx, kz, nz > 1 ? num_k : 0, &dkz, nullptr)) ||
-        (s = imp::to_device_staged(ctx, t, num_k, &dt, nullptr)))
+    return in_less_memory(ctx, [&]() -> imp_status {
+        if ((s = imp::begin(ctx)) != IMP_OK) return s;
+        imp::stage_reset(ctx);
+        DevKeep keep;
+        const float *dkx, *dky, *dkz = nullptr, *dt;
+        if ((s = imp::to_device_staged(ctx, kx, num_k, &dkx, nullptr)) ||
+            (s = imp::to_device_staged(ctx, ky, num_k, &dky, nullptr)) ||
+            (s = imp::to_device_staged(ctx, kz, nz > 1 ? num_k : 0, &dkz, nullptr)) ||
+            (s = imp::to_device_staged(ctx, t, num_k, &dt, nullptr)))
+            return s;
+        imp::ToepSolver &ts = solver_q_of(ctx);
+        imp::ToepConfig qcfg = toep_cfg_nopen(opt, nx, ny, nz, 1, num_k);
+        qcfg.q_only = true;
+        IMP_CUDA(ts.setup(qcfg, dt, nullptr, nullptr, nullptr, ctx->dev_err, ctx->stream),
+                 "toeplitz setup");
+        const size_t nq = (size_t)ts.segments() * ts.q_elems();
+        float *dqr, *dqi;
+        bool hr, hi;
+        if ((s = imp::out_device_staged(ctx, q_r, nq, &dqr, &hr)) ||
+            (s = imp::out_device_staged(ctx, q_i, nq, &dqi, &hi)))
+            return s;
+        IMP_CUDA(ts.compute_q(dkx, dky, dkz, dqr, dqi), "Q gridding");
+        if (hr && (s = copy_out(ctx, q_r, dqr, nq))) return s;
+        if (hi && (s = copy_out(ctx, q_i, dqi, nq))) return s;
+        s = imp::finish(ctx);
+        ctx->launches = ts.launches();
         return s;
-    imp::ToepSolver &ts = solver_q_of(ctx);
-    imp::ToepConfig qcfg = toep_cfg_nopen(opt, nx, ny, nz, 1, num_k);
-    qcfg.q_only = true;
-    IMP_CUDA(ts.setup(qcfg, dt, nullptr, nullptr, nullptr, ctx->dev_err, ctx->stream),
-             "toeplitz setup");
-    const size_t nq = (size_t)ts.segments() * ts.q_elems();
-    float *dqr, *dqi;
-    bool hr, hi;
-    if ((s = imp::out_device_staged(ctx, q_r, nq, &dqr, &hr)) ||
-        (s = imp::out_device_staged(ctx, q_i, nq, &dqi, &hi)))
-        return s;
-    IMP_CUDA(ts.compute_q(dkx, dky, dkz, dqr, dqi), "Q gridding");
-    if (hr && (s = copy_out(ctx, q_r, dqr, nq))) return s;
-    if (hi && (s = copy_out(ctx, q_i, dqi, nq))) return s;
-    s = imp::finish(ctx);
-    ctx->launches = ts.launches();
-    return s;
+    });
 }
 
 imp_status imp_toeplitz_fhd(imp_context *ctx, const imp_toeplitz_options *opt, float *fhd_r,
@@ -1284,37 +1345,39 @@ imp_status imp_toeplitz_fhd(imp_context *ctx, const imp_toeplitz_options *opt, f
         return fail(IMP_ERR_INVALID_ARG, "null array argument");
     if (num_coil <= 0 || (num_coil > 1 && (!sensi_r || !sensi_i)))
         return fail(IMP_ERR_INVALID_ARG, "num_coil > 0 and sensi for num_coil > 1");
-    if ((s = imp::begin(ctx)) != IMP_OK) return s;
-    imp::stage_reset(ctx);
-    const size_t N = (size_t)nx * ny * nz, M = num_k, C = num_coil;
-    DevKeep keep;
-    const float *dkx, *dky, *dkz = nullptr, *dt, *dfm = nullptr, *dsr = nullptr, *dsi = nullptr,
-                      *dkr, *dki;
-    if ((s = imp::to_device_staged(ctx, kx, M, &dkx, nullptr)) ||
-        (s = imp::to_device_staged(ctx, ky, M, &dky, nullptr)) ||
-        (s = imp::to_device_staged(ctx, kz, nz > 1 ? M : 0, &dkz, nullptr)) ||
-        (s = imp::to_device_staged(ctx, t, M, &dt, nullptr)) ||
-        (s = imp::to_device_staged(ctx, fm, N, &dfm, nullptr)) ||
-        (s = imp::to_device_staged(ctx, num_coil > 1 ? sensi_r : nullptr, C * N, &dsr, nullptr)) ||
-        (s = imp::to_device_staged(ctx, num_coil > 1 ? sensi_i : nullptr, C * N, &dsi, nullptr)) ||
-        (s = imp::to_device_staged(ctx, kdata_r, C * M, &dkr, nullptr)) ||
-        (s = imp::to_device_staged(ctx, kdata_i, C * M, &dki, nullptr)))
+    return in_less_memory(ctx, [&]() -> imp_status {
+        if ((s = imp::begin(ctx)) != IMP_OK) return s;
+        imp::stage_reset(ctx);
+        const size_t N = (size_t)nx * ny * nz, M = num_k, C = num_coil;
+        DevKeep keep;
+        const float *dkx, *dky, *dkz = nullptr, *dt, *dfm = nullptr, *dsr = nullptr;
+        const float *dsi = nullptr, *dkr, *dki;
+        if ((s = imp::to_device_staged(ctx, kx, M, &dkx, nullptr)) ||
+            (s = imp::to_device_staged(ctx, ky, M, &dky, nullptr)) ||
+            (s = imp::to_device_staged(ctx, kz, nz > 1 ? M : 0, &dkz, nullptr)) ||
+            (s = imp::to_device_staged(ctx, t, M, &dt, nullptr)) ||
+            (s = imp::to_device_staged(ctx, fm, N, &dfm, nullptr)) ||
+            (s = imp::to_device_staged(ctx, C > 1 ? sensi_r : nullptr, C * N, &dsr, nullptr)) ||
+            (s = imp::to_device_staged(ctx, C > 1 ? sensi_i : nullptr, C * N, &dsi, nullptr)) ||
+            (s = imp::to_device_staged(ctx, kdata_r, C * M, &dkr, nullptr)) ||
+            (s = imp::to_device_staged(ctx, kdata_i, C * M, &dki, nullptr)))
+            return s;
+        imp::ToepSolver &ts = solver_of(ctx);
+        IMP_CUDA(ts.setup(toep_cfg_nopen(opt, nx, ny, nz, num_coil, num_k), dt, dfm, dsr, dsi,
+                          ctx->dev_err, ctx->stream),
+                 "toeplitz setup");
+        float *dfr, *dfi;
+        bool hr, hi;
+        if ((s = imp::out_device_staged(ctx, fhd_r, N, &dfr, &hr)) ||
+            (s = imp::out_device_staged(ctx, fhd_i, N, &dfi, &hi)))
+            return s;
+        IMP_CUDA(ts.compute_fhd(dkx, dky, dkz, dkr, dki, dfr, dfi), "F^H d gridding");
+        if (hr && (s = copy_out(ctx, fhd_r, dfr, N))) return s;
+        if (hi && (s = copy_out(ctx, fhd_i, dfi, N))) return s;
+        s = imp::finish(ctx);
+        ctx->launches = ts.launches();
         return s;
-    imp::ToepSolver &ts = solver_of(ctx);
-    IMP_CUDA(ts.setup(toep_cfg_nopen(opt, nx, ny, nz, num_coil, num_k), dt, dfm, dsr, dsi,
-                      ctx->dev_err, ctx->stream),
-             "toeplitz setup");
-    float *dfr, *dfi;
-    bool hr, hi;
-    if ((s = imp::out_device_staged(ctx, fhd_r, N, &dfr, &hr)) ||
-        (s = imp::out_device_staged(ctx, fhd_i, N, &dfi, &hi)))
-        return s;
-    IMP_CUDA(ts.compute_fhd(dkx, dky, dkz, dkr, dki, dfr, dfi), "F^H d gridding");
-    if (hr && (s = copy_out(ctx, fhd_r, dfr, N))) return s;
-    if (hi && (s = copy_out(ctx, fhd_i, dfi, N))) return s;
-    s = imp::finish(ctx);
-    ctx->launches = ts.launches();
-    return s;
+    });
 }
 
 static imp_status toeplitz_common(imp_context *ctx, const imp_toeplitz_options *opt,
@@ -1337,8 +1400,9 @@ static imp_status toeplitz_common(imp_context *ctx, const imp_toeplitz_options *
         (s = imp::to_device_staged(ctx, num_coil > 1 ? sensi_i : nullptr, C * N, &dsi, nullptr)))
         return s;
     imp::ToepSolver &ts = solver_of(ctx);
-    IMP_CUDA(ts.setup(toep_cfg(opt, nx, ny, nz, num_coil, num_k), dt, dfm, dsr, dsi,
-                      ctx->dev_err, ctx->stream),
+    imp::ToepConfig cfg = toep_cfg(opt, nx, ny, nz, num_coil, num_k);
+    cfg.cg = true;
+    IMP_CUDA(ts.setup(cfg, dt, dfm, dsr, dsi, ctx->dev_err, ctx->stream),
              "toeplitz setup");
     const size_t nq = (size_t)ts.segments() * ts.q_elems();
     if ((s = imp::to_device_staged(ctx, q_r, nq, &dqr, nullptr)) ||
@@ -1355,26 +1419,28 @@ imp_status imp_toeplitz_recon(imp_context *ctx, const imp_toeplitz_options *opt,
                               const float *fm, const float *sensi_r, const float *sensi_i,
                               int num_coil, int nx, int ny, int nz) {
     if (!x_r || !x_i || !fhd_r || !fhd_i) return fail(IMP_ERR_INVALID_ARG, "null array argument");
-    DevKeep keep;
-    imp::ToepSolver *ts = nullptr;
-    imp_status s = toeplitz_common(ctx, opt, q_r, q_i, t, num_k, fm, sensi_r, sensi_i, num_coil,
-                                   nx, ny, nz, keep, &ts);
-    if (s != IMP_OK) return s;
-    const size_t N = (size_t)nx * ny * nz;
-    const float *dfr, *dfi;
-    float *dxr, *dxi;
-    bool hr, hi;
-    if ((s = imp::to_device_staged(ctx, fhd_r, N, &dfr, nullptr)) ||
-        (s = imp::to_device_staged(ctx, fhd_i, N, &dfi, nullptr)) ||
-        (s = imp::out_device_staged(ctx, x_r, N, &dxr, &hr)) ||
-        (s = imp::out_device_staged(ctx, x_i, N, &dxi, &hi)))
+    return in_less_memory(ctx, [&]() -> imp_status {
+        DevKeep keep;
+        imp::ToepSolver *ts = nullptr;
+        imp_status s = toeplitz_common(ctx, opt, q_r, q_i, t, num_k, fm, sensi_r, sensi_i, num_coil,
+                                       nx, ny, nz, keep, &ts);
+        if (s != IMP_OK) return s;
+        const size_t N = (size_t)nx * ny * nz;
+        const float *dfr, *dfi;
+        float *dxr, *dxi;
+        bool hr, hi;
+        if ((s = imp::to_device_staged(ctx, fhd_r, N, &dfr, nullptr)) ||
+            (s = imp::to_device_staged(ctx, fhd_i, N, &dfi, nullptr)) ||
+            (s = imp::out_device_staged(ctx, x_r, N, &dxr, &hr)) ||
+            (s = imp::out_device_staged(ctx, x_i, N, &dxi, &hi)))
+            return s;
+        IMP_CUDA(ts->solve(dfr, dfi, dxr, dxi), "toeplitz CG");
+        if (hr && (s = copy_out(ctx, x_r, dxr, N))) return s;
+        if (hi && (s = copy_out(ctx, x_i, dxi, N))) return s;
+        s = imp::finish(ctx);
+        ctx->launches = ts->launches();
         return s;
-    IMP_CUDA(ts->solve(dfr, dfi, dxr, dxi), "toeplitz CG");
-    if (hr && (s = copy_out(ctx, x_r, dxr, N))) return s;
-    if (hi && (s = copy_out(ctx, x_i, dxi, N))) return s;
-    s = imp::finish(ctx);
-    ctx->launches = ts->launches();
-    return s;
+    });
 }
 
 imp_status imp_toeplitz_cg(imp_context *ctx, const imp_toeplitz_options *opt, float *x_r,
@@ -1386,32 +1452,35 @@ imp_status imp_toeplitz_cg(imp_context *ctx, const imp_toeplitz_options *opt, fl
     if (max_iter < 0 || !(tol >= 0.0)) return fail(IMP_ERR_INVALID_ARG, "max_iter >= 0, tol >= 0");
     imp_toeplitz_options o = *opt;
     o.enable_tv = 0;  // one CG run, no reweighting passes
-    DevKeep keep;
-    imp::ToepSolver *ts = nullptr;
-    imp_status s = toeplitz_common(ctx, &o, q_r, q_i, t, num_k, fm, sensi_r, sensi_i, num_coil,
-                                   nx, ny, nz, keep, &ts);
-    if (s != IMP_OK) return s;
-    const size_t N = (size_t)nx * ny * nz;
-    const float *dfr, *dfi, *dx0r, *dx0i;
-    float *dxr, *dxi;
-    bool hr, hi;
-    if ((s = imp::to_device_staged(ctx, fhd_r, N, &dfr, nullptr)) ||
-        (s = imp::to_device_staged(ctx, fhd_i, N, &dfi, nullptr)) ||
-        (s = imp::to_device_staged(ctx, x_r, N, &dx0r, nullptr)) ||
-        (s = imp::to_device_staged(ctx, x_i, N, &dx0i, nullptr)) ||
-        (s = imp::out_device_staged(ctx, x_r, N, &dxr, &hr)) ||
-        (s = imp::out_device_staged(ctx, x_i, N, &dxi, &hi)))
+    return in_less_memory(ctx, [&]() -> imp_status {
+        DevKeep keep;
+        imp::ToepSolver *ts = nullptr;
+        imp_status s = toeplitz_common(ctx, &o, q_r, q_i, t, num_k, fm, sensi_r, sensi_i, num_coil,
+                                       nx, ny, nz, keep, &ts);
+        if (s != IMP_OK) return s;
+        const size_t N = (size_t)nx * ny * nz;
+        const float *dfr, *dfi, *dx0r, *dx0i;
+        float *dxr, *dxi;
+        bool hr, hi;
+        if ((s = imp::to_device_staged(ctx, fhd_r, N, &dfr, nullptr)) ||
+            (s = imp::to_device_staged(ctx, fhd_i, N, &dfi, nullptr)) ||
+            (s = imp::to_device_staged(ctx, x_r, N, &dx0r, nullptr)) ||
+            (s = imp::to_device_staged(ctx, x_i, N, &dx0i, nullptr)) ||
+            (s = imp::out_device_staged(ctx, x_r, N, &dxr, &hr)) ||
+            (s = imp::out_device_staged(ctx, x_i, N, &dxi, &hi)))
+            return s;
+        const cudaMemcpyKind d2d = cudaMemcpyDeviceToDevice;
+        if (hr) IMP_CUDA(cudaMemcpyAsync(dxr, dx0r, N * 4, d2d, ctx->stream), "x0");
+        if (hi) IMP_CUDA(cudaMemcpyAsync(dxi, dx0i, N * 4, d2d, ctx->stream), "x0");
+        int it = 0;
+        IMP_CUDA(ts->solve_from(dfr, dfi, dxr, dxi, tol, max_iter, &it), "toeplitz warm CG");
+        if (iterations) *iterations = it;
+        if (hr && (s = copy_out(ctx, x_r, dxr, N))) return s;
+        if (hi && (s = copy_out(ctx, x_i, dxi, N))) return s;
+        s = imp::finish(ctx);
+        ctx->launches = ts->launches();
         return s;
-    if (hr) IMP_CUDA(cudaMemcpyAsync(dxr, dx0r, N * 4, cudaMemcpyDeviceToDevice, ctx->stream), "x0");
-    if (hi) IMP_CUDA(cudaMemcpyAsync(dxi, dx0i, N * 4, cudaMemcpyDeviceToDevice, ctx->stream), "x0");
-    int it = 0;
-    IMP_CUDA(ts->solve_from(dfr, dfi, dxr, dxi, tol, max_iter, &it), "toeplitz warm CG");
-    if (iterations) *iterations = it;
-    if (hr && (s = copy_out(ctx, x_r, dxr, N))) return s;
-    if (hi && (s = copy_out(ctx, x_i, dxi, N))) return s;
-    s = imp::finish(ctx);
-    ctx->launches = ts->launches();
-    return s;
+    });
 }
 
 imp_status imp_grid_fft(imp_context *ctx, float *data_r, float *data_i, int n0, int n1, int n2,
@@ -1463,26 +1532,28 @@ imp_status imp_toeplitz_apply(imp_context *ctx, const imp_toeplitz_options *opt,
                               int num_coil, int nx, int ny, int nz) {
     if (!q_out_r || !q_out_i || !p_r || !p_i)
         return fail(IMP_ERR_INVALID_ARG, "null array argument");
-    DevKeep keep;
-    imp::ToepSolver *ts = nullptr;
-    imp_status s = toeplitz_common(ctx, opt, q_r, q_i, t, num_k, fm, sensi_r, sensi_i, num_coil,
-                                   nx, ny, nz, keep, &ts);
-    if (s != IMP_OK) return s;
-    const size_t N = (size_t)nx * ny * nz;
-    const float *dpr, *dpi;
-    float *dor, *doi;
-    bool hr, hi;
-    if ((s = imp::to_device_staged(ctx, p_r, N, &dpr, nullptr)) ||
-        (s = imp::to_device_staged(ctx, p_i, N, &dpi, nullptr)) ||
-        (s = imp::out_device_staged(ctx, q_out_r, N, &dor, &hr)) ||
-        (s = imp::out_device_staged(ctx, q_out_i, N, &doi, &hi)))
+    return in_less_memory(ctx, [&]() -> imp_status {
+        DevKeep keep;
+        imp::ToepSolver *ts = nullptr;
+        imp_status s = toeplitz_common(ctx, opt, q_r, q_i, t, num_k, fm, sensi_r, sensi_i, num_coil,
+                                       nx, ny, nz, keep, &ts);
+        if (s != IMP_OK) return s;
+        const size_t N = (size_t)nx * ny * nz;
+        const float *dpr, *dpi;
+        float *dor, *doi;
+        bool hr, hi;
+        if ((s = imp::to_device_staged(ctx, p_r, N, &dpr, nullptr)) ||
+            (s = imp::to_device_staged(ctx, p_i, N, &dpi, nullptr)) ||
+            (s = imp::out_device_staged(ctx, q_out_r, N, &dor, &hr)) ||
+            (s = imp::out_device_staged(ctx, q_out_i, N, &doi, &hi)))
+            return s;
+        IMP_CUDA(ts->apply(dpr, dpi, dor, doi), "toeplitz apply");
+        if (hr && (s = copy_out(ctx, q_out_r, dor, N))) return s;
+        if (hi && (s = copy_out(ctx, q_out_i, doi, N))) return s;
+        s = imp::finish(ctx);
+        ctx->launches = ts->launches();
         return s;
-    IMP_CUDA(ts->apply(dpr, dpi, dor, doi), "toeplitz apply");
-    if (hr && (s = copy_out(ctx, q_out_r, dor, N))) return s;
-    if (hi && (s = copy_out(ctx, q_out_i, doi, N))) return s;
-    s = imp::finish(ctx);
-    ctx->launches = ts->launches();
-    return s;
+    });
 }
 
 }  // extern "C"

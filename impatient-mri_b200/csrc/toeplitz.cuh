@@ -43,6 +43,7 @@ struct ToepConfig {
     bool use_graphs = true;
     const imp_sparse *reg = nullptr;  // -reg roughness matrix (host COO), null = off
     bool q_only = false;  // compute_q only: no coils, phases, engine or CG buffers
+    bool cg = false;      // load_q and the CG (or apply) follow
 };
 
 class ToepSolver {
@@ -80,6 +81,8 @@ public:
     size_t q_elems() const { return G2_; }
     size_t voxels() const { return N_; }
     void release();
+    // Whether the call that ran out of memory can be made with less.
+    bool shrink();
 
 private:
     cudaError_t apply_aha(const float2 *p, float2 *q);  // q = A^H A p (no TV term)
@@ -87,11 +90,16 @@ private:
     cudaError_t penalty_dot(float2 *q, const float2 *p);
     const int *done_flag() const;
     cudaError_t set_reg();
+    cudaError_t prepare_cg();
+    cudaError_t build_cg();
+    void release_cg();
     cudaError_t cg_iteration();
     cudaError_t ensure_grid_plan(const GridSpec &g, GridFft *plan, int batch);
 
     ToepConfig cfg_;
     bool ready_ = false;       // the last set-up was completed
+    bool cg_ready_ = false;    // build_cg was
+    int lean_ = 0;             // see shrink()
     SparseReg reg_;            // -reg: C and C^T on the device
     cudaStream_t st_ = nullptr;
     unsigned *err_ = nullptr;

@@ -47,8 +47,8 @@ def brute_force(pkg, C, M, slices, seed=0, n=16):
     return call
 
 
-def toeplitz(pkg, dims, C, L, seed=0):
-    """call(ctx) -> image: 2 CG iterations from a given Q."""
+def toeplitz(pkg, dims, C, L, what="recon", seed=0):
+    """call(ctx) -> image: 2 CG iterations from a given Q, one application of it, or F^H d."""
     r = np.random.default_rng(seed)
     dev = lambda a: torch.as_tensor(np.ascontiguousarray(a, np.float32)).cuda()
     nx, ny, nz = dims
@@ -59,11 +59,18 @@ def toeplitz(pkg, dims, C, L, seed=0):
     b = [dev(r.standard_normal(N)) for _ in range(2)]
     s = [dev(r.standard_normal(C * N)) for _ in range(2)]
     o = pkg.toeplitz_options(cg_num=2, ntime_segs=L)
+    x = [torch.zeros(N, device="cuda") for _ in range(2)]
+    k = [dev(r.uniform(-v / 2, v / 2 - 1, 64)) for v in dims]
+    d = [dev(r.standard_normal(C * 64)) for _ in range(2)]
 
     def call(ctx):
-        x = [torch.zeros(N, device="cuda") for _ in range(2)]
-        pkg.toeplitz_recon(ctx, o, *x, *b, *q, t, 64, fm, *s, C, *dims)
-        return (x[0] + 1j * x[1]).cpu().numpy()
+        if what == "fhd":
+            pkg.toeplitz_fhd(ctx, o, *x, *d, *k, t, fm, *s, 64, C, *dims)
+        elif what == "apply":
+            pkg.toeplitz_apply(ctx, o, *x, *b, *q, t, 64, fm, *s, C, *dims)
+        else:
+            pkg.toeplitz_recon(ctx, o, *x, *b, *q, t, 64, fm, *s, C, *dims)
+        return x[0].cpu().numpy() + 1j * x[1].cpu().numpy()
     return call
 
 
@@ -73,7 +80,7 @@ def test_failed_setup_is_done_again(pkg, what, C):
     """Two calls without room, then one with it, on one context."""
     call = {"one": lambda: brute_force(pkg, C, 1 << 18, 0),
             "batch": lambda: brute_force(pkg, C, 1 << 17, 2),
-            "toeplitz": lambda: toeplitz(pkg, (256, 256, 1), C, 3)}[what]()
+            "toeplitz": lambda: toeplitz(pkg, (512, 512, 1), C, 3)}[what]()
     with pkg.Context(0) as fresh:
         want = call(fresh)
     with pkg.Context(0) as one:
@@ -105,3 +112,40 @@ def test_optional_image_gives_way(pkg, monkeypatch, slices):
         got = call(ctx)
     # one CG update of FP16- and TF32-split sums, both 22 bits
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < 1e-5
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+# what is left: enough for the spectra of one transform at a time (power-of-two side: its Q
+# and one Qf_l of scratch), or for the zero-padded chain only (520 runs on 576 otherwise)
+@pytest.mark.parametrize("n,C,segs,extra", [(512, 16, 42, 8 * 512 * 1024), (520, 1, 42, 0)])
+def test_toeplitz_runs_leaner(pkg, n, C, segs, extra):
+    """A^H A in the memory of one transform at a time, or of the zero-padded chain."""
+    L, N = 40, n * n
+    call, grids = (toeplitz(pkg, (n, n, 1), C, L, what) for what in ("apply", "fhd"))
+    with pkg.Context(0) as ctx:
+        want = call(ctx)
+    need = 8 * 4 * N * segs + extra + 8 * N * (C + L + 1 + 6) + 4 * N
+    for first in ("apply", "fhd"):
+        with pkg.Context(0) as ctx, leave(need + (40 << 20)):
+            if first == "fhd":  # its grids give way too
+                grids(ctx)
+            assert rel(call(ctx), want) < 1e-5
+
+
+def test_fhd_needs_no_engine(pkg):
+    """F^H d in the memory of its inputs and a single gridding grid (a batch takes 64 MB), also
+    on a context that holds the engine."""
+    n, C, L = 512, 4, 40
+    call, other = (toeplitz(pkg, (n, n, 1), C, L, what) for what in ("fhd", "apply"))
+    with pkg.Context(0) as ctx:
+        want, image = call(ctx), other(ctx)
+    with pkg.Context(0) as ctx, leave(8 * n * n * (C + L + 2) + 8 * 768 * 768 + (16 << 20)):
+        assert rel(call(ctx), want) < 1e-5
+    with pkg.Context(0) as ctx:
+        other(ctx)
+        with leave(8 << 20):
+            assert rel(call(ctx), want) < 1e-5
+        assert rel(other(ctx), image) < 1e-5
