@@ -146,10 +146,10 @@ imp_status op_work(imp_context *ctx, int M, int N, int C, bool use_z, bool adj, 
         void *base = nullptr;
         const imp_status s = scratch(ctx, b_k + b_v + b_s + b_d + b_p + align256(image), &base);
         if (s == IMP_ERR_NOMEM && image) {  // the kernel that needs no image
-            cudaGetLastError();
             image = 0;
             continue;
         }
+        if (s == IMP_ERR_NOMEM && imp::give_back(ctx)) continue;
         if (s != IMP_OK) return s;
         char *at = (char *)base;
         p.kgeo = (double4 *)at;
@@ -303,8 +303,20 @@ imp_status out_device(imp_context *ctx, float *p, size_t n, DevKeep &keep, float
     return IMP_OK;
 }
 
+bool give_back(imp_context *ctx) {
+    if (ctx->scratch) {
+        cudaFree(ctx->scratch);
+        ctx->scratch = nullptr;
+        ctx->scratch_bytes = 0;
+        return true;
+    }
+    return (ctx->bf && ctx->bf->drop_image()) || (ctx->bb && ctx->bb->drop_image()) ||
+           (ctx->tp && ctx->tp->shrink()) || (ctx->tp_q && ctx->tp_q->shrink());
+}
+
 }  // namespace imp
 
+using imp::in_less_memory;
 using imp::stage_reset;
 using imp::to_device;
 using imp::to_device_staged;
@@ -482,61 +494,63 @@ imp_status imp_bruteforce_recon(imp_context *ctx, const imp_bf_options *opt, flo
     if (opt->enable_tv && opt->tv_num <= 0) return fail(IMP_ERR_INVALID_ARG, "tv_num must be > 0");
     imp::BfConfig cfg;
     if ((s = bf_config(opt, num_k, num_i, num_coil, &cfg)) != IMP_OK) return s;
-    if ((s = begin(ctx)) != IMP_OK) return s;
-    const size_t M = num_k, N = num_i, C = num_coil, S = num_slices;
-    const float *d_kx, *d_ky, *d_kz = nullptr, *d_ix, *d_iy, *d_iz = nullptr, *d_t, *d_fm = nullptr;
-    const float *d_sr = nullptr, *d_si = nullptr, *d_kr, *d_ki, *d_xr0, *d_xi0;
-    bool x_host = false, dummy;
-    stage_reset(ctx);
-    if ((s = to_device_staged(ctx, kx, M, &d_kx, &dummy)) ||
-        (s = to_device_staged(ctx, ky, M, &d_ky, &dummy)) ||
-        (s = to_device_staged(ctx, kz, M, &d_kz, &dummy)) ||
-        (s = to_device_staged(ctx, t, M, &d_t, &dummy)) ||
-        (s = to_device_staged(ctx, ix, N, &d_ix, &dummy)) ||
-        (s = to_device_staged(ctx, iy, N, &d_iy, &dummy)) ||
-        (s = to_device_staged(ctx, iz, N, &d_iz, &dummy)) ||
-        (s = to_device_staged(ctx, fm, S * N, &d_fm, &dummy)) ||
-        (s = to_device_staged(ctx, sensi_r, C * N, &d_sr, &dummy)) ||
-        (s = to_device_staged(ctx, sensi_i, C * N, &d_si, &dummy)) ||
-        (s = to_device_staged(ctx, kdata_r, S * C * M, &d_kr, &dummy)) ||
-        (s = to_device_staged(ctx, kdata_i, S * C * M, &d_ki, &dummy)) ||
-        (s = to_device_staged(ctx, idata_r, S * N, &d_xr0, &x_host)) ||
-        (s = to_device_staged(ctx, idata_i, S * N, &d_xi0, &dummy)))
+    return in_less_memory(ctx, [&]() -> imp_status {
+        if ((s = begin(ctx)) != IMP_OK) return s;
+        const size_t M = num_k, N = num_i, C = num_coil, S = num_slices;
+        const float *d_kx, *d_ky, *d_kz = nullptr, *d_ix, *d_iy, *d_iz = nullptr, *d_t;
+        const float *d_fm = nullptr, *d_sr = nullptr, *d_si = nullptr, *d_kr, *d_ki, *d_xr0, *d_xi0;
+        bool x_host = false, dummy;
+        stage_reset(ctx);
+        if ((s = to_device_staged(ctx, kx, M, &d_kx, &dummy)) ||
+            (s = to_device_staged(ctx, ky, M, &d_ky, &dummy)) ||
+            (s = to_device_staged(ctx, kz, M, &d_kz, &dummy)) ||
+            (s = to_device_staged(ctx, t, M, &d_t, &dummy)) ||
+            (s = to_device_staged(ctx, ix, N, &d_ix, &dummy)) ||
+            (s = to_device_staged(ctx, iy, N, &d_iy, &dummy)) ||
+            (s = to_device_staged(ctx, iz, N, &d_iz, &dummy)) ||
+            (s = to_device_staged(ctx, fm, S * N, &d_fm, &dummy)) ||
+            (s = to_device_staged(ctx, sensi_r, C * N, &d_sr, &dummy)) ||
+            (s = to_device_staged(ctx, sensi_i, C * N, &d_si, &dummy)) ||
+            (s = to_device_staged(ctx, kdata_r, S * C * M, &d_kr, &dummy)) ||
+            (s = to_device_staged(ctx, kdata_i, S * C * M, &d_ki, &dummy)) ||
+            (s = to_device_staged(ctx, idata_r, S * N, &d_xr0, &x_host)) ||
+            (s = to_device_staged(ctx, idata_i, S * N, &d_xi0, &dummy)))
+            return s;
+        float *d_xr = const_cast<float *>(d_xr0), *d_xi = const_cast<float *>(d_xi0);
+        if (num_coil == 1) {
+            d_sr = nullptr;  // one coil: unit sensitivity (kernels/structures.cpp:710-716)
+            d_si = nullptr;
+        }
+        // the context keeps one solver: buffers, tuned shapes and CUDA graphs are
+        // reused by later calls of the same problem size
+        if (!ctx->bf) ctx->bf.reset(new imp::BfSolver());
+        imp::BfSolver &solver = *ctx->bf;
+        IMP_CUDA(solver.setup(cfg, d_kx, d_ky, d_kz, d_t, d_ix, d_iy, d_iz, d_sr, d_si,
+                              ctx->dev_err, ctx->stream),
+                 "brute-force setup");
+        solver.set_profiling(ctx->prof_on);
+        long launches = 4;
+        for (int sl = 0; sl < num_slices; ++sl) {
+            IMP_CUDA(solver.solve(d_fm ? d_fm + (size_t)sl * N : nullptr, d_kr + (size_t)sl * C * M,
+                                  d_ki + (size_t)sl * C * M, d_xr + (size_t)sl * N,
+                                  d_xi + (size_t)sl * N),
+                     "brute-force solve");
+            launches += solver.launches();
+        }
+        if (x_host) {
+            IMP_CUDA(cudaMemcpyAsync(idata_r, d_xr, S * N * sizeof(float), cudaMemcpyDeviceToHost,
+                                     ctx->stream),
+                     "output D2H");
+            IMP_CUDA(cudaMemcpyAsync(idata_i, d_xi, S * N * sizeof(float), cudaMemcpyDeviceToHost,
+                                     ctx->stream),
+                     "output D2H");
+        }
+        s = finish(ctx);
+        ctx->launches = launches;
+        if (s == IMP_OK && ctx->prof_on)
+            IMP_CUDA(solver.profile_collect(ctx->prof_ms, ctx->prof_count), "profile collect");
         return s;
-    float *d_xr = const_cast<float *>(d_xr0), *d_xi = const_cast<float *>(d_xi0);
-    if (num_coil == 1) {
-        d_sr = nullptr;  // one coil: unit sensitivity (kernels/structures.cpp:710-716)
-        d_si = nullptr;
-    }
-    // the context keeps one solver: buffers, tuned shapes and CUDA graphs are
-    // reused by later calls of the same problem size
-    if (!ctx->bf) ctx->bf.reset(new imp::BfSolver());
-    imp::BfSolver &solver = *ctx->bf;
-    IMP_CUDA(solver.setup(cfg, d_kx, d_ky, d_kz, d_t, d_ix, d_iy, d_iz, d_sr, d_si, ctx->dev_err,
-                          ctx->stream),
-             "brute-force setup");
-    solver.set_profiling(ctx->prof_on);
-    long launches = 4;
-    for (int sl = 0; sl < num_slices; ++sl) {
-        IMP_CUDA(solver.solve(d_fm ? d_fm + (size_t)sl * N : nullptr, d_kr + (size_t)sl * C * M,
-                              d_ki + (size_t)sl * C * M, d_xr + (size_t)sl * N,
-                              d_xi + (size_t)sl * N),
-                 "brute-force solve");
-        launches += solver.launches();
-    }
-    if (x_host) {
-        IMP_CUDA(cudaMemcpyAsync(idata_r, d_xr, S * N * sizeof(float), cudaMemcpyDeviceToHost,
-                                 ctx->stream),
-                 "output D2H");
-        IMP_CUDA(cudaMemcpyAsync(idata_i, d_xi, S * N * sizeof(float), cudaMemcpyDeviceToHost,
-                                 ctx->stream),
-                 "output D2H");
-    }
-    s = finish(ctx);
-    ctx->launches = launches;
-    if (s == IMP_OK && ctx->prof_on)
-        IMP_CUDA(solver.profile_collect(ctx->prof_ms, ctx->prof_count), "profile collect");
-    return s;
+    });
 }
 
 imp_status imp_bruteforce_batch(imp_context *ctx, const imp_bf_options *opt, float *idata_r,
@@ -561,56 +575,58 @@ imp_status imp_bruteforce_batch(imp_context *ctx, const imp_bf_options *opt, flo
         return fail(IMP_ERR_INVALID_ARG, "sensi needed for num_coil > 1");
     if (opt->cg_num <= 0) return fail(IMP_ERR_INVALID_ARG, "cg_num must be > 0");
     if (opt->enable_tv && opt->tv_num <= 0) return fail(IMP_ERR_INVALID_ARG, "tv_num must be > 0");
-    if ((s = begin(ctx)) != IMP_OK) return s;
-    const size_t N = num_i, C = num_coil, S = num_slices;
-    const float *d_kx, *d_ky, *d_kz = nullptr, *d_ix, *d_iy, *d_iz = nullptr, *d_t, *d_fm = nullptr;
-    const float *d_sr = nullptr, *d_si = nullptr, *d_kr, *d_ki, *d_xr0, *d_xi0;
-    bool x_host = false, dummy;
-    stage_reset(ctx);
-    if ((s = to_device_staged(ctx, kx, Mt, &d_kx, &dummy)) ||
-        (s = to_device_staged(ctx, ky, Mt, &d_ky, &dummy)) ||
-        (s = to_device_staged(ctx, kz, Mt, &d_kz, &dummy)) ||
-        (s = to_device_staged(ctx, t, Mt, &d_t, &dummy)) ||
-        (s = to_device_staged(ctx, ix, N, &d_ix, &dummy)) ||
-        (s = to_device_staged(ctx, iy, N, &d_iy, &dummy)) ||
-        (s = to_device_staged(ctx, iz, N, &d_iz, &dummy)) ||
-        (s = to_device_staged(ctx, fm, S * N, &d_fm, &dummy)) ||
-        (s = to_device_staged(ctx, sensi_r, C * N, &d_sr, &dummy)) ||
-        (s = to_device_staged(ctx, sensi_i, C * N, &d_si, &dummy)) ||
-        (s = to_device_staged(ctx, kdata_r, C * Mt, &d_kr, &dummy)) ||
-        (s = to_device_staged(ctx, kdata_i, C * Mt, &d_ki, &dummy)) ||
-        (s = to_device_staged(ctx, idata_r, S * N, &d_xr0, &x_host)) ||
-        (s = to_device_staged(ctx, idata_i, S * N, &d_xi0, &dummy)))
+    return in_less_memory(ctx, [&]() -> imp_status {
+        if ((s = begin(ctx)) != IMP_OK) return s;
+        const size_t N = num_i, C = num_coil, S = num_slices;
+        const float *d_kx, *d_ky, *d_kz = nullptr, *d_ix, *d_iy, *d_iz = nullptr, *d_t;
+        const float *d_fm = nullptr, *d_sr = nullptr, *d_si = nullptr, *d_kr, *d_ki, *d_xr0, *d_xi0;
+        bool x_host = false, dummy;
+        stage_reset(ctx);
+        if ((s = to_device_staged(ctx, kx, Mt, &d_kx, &dummy)) ||
+            (s = to_device_staged(ctx, ky, Mt, &d_ky, &dummy)) ||
+            (s = to_device_staged(ctx, kz, Mt, &d_kz, &dummy)) ||
+            (s = to_device_staged(ctx, t, Mt, &d_t, &dummy)) ||
+            (s = to_device_staged(ctx, ix, N, &d_ix, &dummy)) ||
+            (s = to_device_staged(ctx, iy, N, &d_iy, &dummy)) ||
+            (s = to_device_staged(ctx, iz, N, &d_iz, &dummy)) ||
+            (s = to_device_staged(ctx, fm, S * N, &d_fm, &dummy)) ||
+            (s = to_device_staged(ctx, sensi_r, C * N, &d_sr, &dummy)) ||
+            (s = to_device_staged(ctx, sensi_i, C * N, &d_si, &dummy)) ||
+            (s = to_device_staged(ctx, kdata_r, C * Mt, &d_kr, &dummy)) ||
+            (s = to_device_staged(ctx, kdata_i, C * Mt, &d_ki, &dummy)) ||
+            (s = to_device_staged(ctx, idata_r, S * N, &d_xr0, &x_host)) ||
+            (s = to_device_staged(ctx, idata_i, S * N, &d_xi0, &dummy)))
+            return s;
+        float *d_xr = const_cast<float *>(d_xr0), *d_xi = const_cast<float *>(d_xi0);
+        if (num_coil == 1) {
+            d_sr = nullptr;  // one coil: unit sensitivity (kernels/structures.cpp:710-716)
+            d_si = nullptr;
+        }
+        // all slices in lockstep: every CG step is one launch over all slices
+        imp::BfConfig cfg;
+        if ((s = bf_config(opt, k_off[1] - k_off[0], num_i, num_coil, &cfg)) != IMP_OK) return s;
+        if (cfg.reg)
+            return fail(IMP_ERR_UNSUPPORTED, "-reg is not available in the batched multi-slice "
+                                             "solver; reconstruct the slices with "
+                                             "imp_bruteforce_recon");
+        if (!ctx->bb) ctx->bb.reset(new imp::BfBatch());
+        IMP_CUDA(ctx->bb->setup(cfg, num_slices, k_off, d_kx, d_ky, d_kz, d_t, d_ix, d_iy, d_iz,
+                                d_fm, d_sr, d_si, ctx->dev_err, ctx->stream),
+                 "batched brute-force setup");
+        IMP_CUDA(ctx->bb->solve(d_kr, d_ki, d_xr, d_xi), "batched brute-force solve");
+        const long launches = ctx->bb->launches();
+        if (x_host) {
+            IMP_CUDA(cudaMemcpyAsync(idata_r, d_xr, S * N * sizeof(float), cudaMemcpyDeviceToHost,
+                                     ctx->stream),
+                     "output D2H");
+            IMP_CUDA(cudaMemcpyAsync(idata_i, d_xi, S * N * sizeof(float), cudaMemcpyDeviceToHost,
+                                     ctx->stream),
+                     "output D2H");
+        }
+        s = finish(ctx);
+        ctx->launches = launches;
         return s;
-    float *d_xr = const_cast<float *>(d_xr0), *d_xi = const_cast<float *>(d_xi0);
-    if (num_coil == 1) {
-        d_sr = nullptr;  // one coil: unit sensitivity (kernels/structures.cpp:710-716)
-        d_si = nullptr;
-    }
-    // all slices in lockstep: every CG step is one launch over all slices
-    imp::BfConfig cfg;
-    if ((s = bf_config(opt, k_off[1] - k_off[0], num_i, num_coil, &cfg)) != IMP_OK) return s;
-    if (cfg.reg)
-        return fail(IMP_ERR_UNSUPPORTED, "-reg is not available in the batched multi-slice "
-                                         "solver; reconstruct the slices with "
-                                         "imp_bruteforce_recon");
-    if (!ctx->bb) ctx->bb.reset(new imp::BfBatch());
-    IMP_CUDA(ctx->bb->setup(cfg, num_slices, k_off, d_kx, d_ky, d_kz, d_t, d_ix, d_iy, d_iz, d_fm,
-                            d_sr, d_si, ctx->dev_err, ctx->stream),
-             "batched brute-force setup");
-    IMP_CUDA(ctx->bb->solve(d_kr, d_ki, d_xr, d_xi), "batched brute-force solve");
-    const long launches = ctx->bb->launches();
-    if (x_host) {
-        IMP_CUDA(cudaMemcpyAsync(idata_r, d_xr, S * N * sizeof(float), cudaMemcpyDeviceToHost,
-                                 ctx->stream),
-                 "output D2H");
-        IMP_CUDA(cudaMemcpyAsync(idata_i, d_xi, S * N * sizeof(float), cudaMemcpyDeviceToHost,
-                                 ctx->stream),
-                 "output D2H");
-    }
-    s = finish(ctx);
-    ctx->launches = launches;
-    return s;
+    });
 }
 
 imp_status imp_check_wait_expiry(imp_context *ctx, int polls) {

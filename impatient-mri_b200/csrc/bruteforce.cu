@@ -296,11 +296,12 @@ cudaError_t BfSolver::setup(const BfConfig &cfg, const float *kx, const float *k
                             const float *kz, const float *t, const float *ix, const float *iy,
                             const float *iz, const float *sensi_r, const float *sensi_i,
                             unsigned *dev_err, cudaStream_t st) {
-    const bool same_shape = ready_ && st == st_ && dev_err == err_ && cfg.M == cfg_.M &&
-                            cfg.N == cfg_.N && cfg.C == cfg_.C && cfg.use_z == cfg_.use_z &&
-                            cfg.n0 == cfg_.n0 && cfg.n1 == cfg_.n1 && cfg.n2 == cfg_.n2 &&
-                            cfg.autotune == cfg_.autotune;
+    const bool like = st == st_ && dev_err == err_ && cfg.M == cfg_.M && cfg.N == cfg_.N &&
+                      cfg.C == cfg_.C && cfg.use_z == cfg_.use_z && cfg.n0 == cfg_.n0 &&
+                      cfg.n1 == cfg_.n1 && cfg.n2 == cfg_.n2 && cfg.autotune == cfg_.autotune;
+    const bool same_shape = ready_ && like;
     ready_ = false;  // until this set-up is complete
+    if (!like) image_ = true;
     if (same_shape) {
         // keep buffers, tuned launch shapes and (if the captured scalars match) the graphs
         bool stale = cfg.fd != cfg_.fd || cfg.lambda != cfg_.lambda;
@@ -316,29 +317,13 @@ cudaError_t BfSolver::setup(const BfConfig &cfg, const float *kx, const float *k
         ready_ = true;
         return cudaSuccess;
     }
+    release();
     cfg_ = cfg;
     st_ = st;
     err_ = dev_err;
-    // The FP16 kernel's image is optional: where it leaves no room for the rest, the
-    // set-up is done without it (the TF32 kernel).
-    cudaError_t e = build(kx, ky, kz, t, ix, iy, iz, sensi_r, sensi_i, true);
-    if (e == cudaErrorMemoryAllocation && plan_.img_bytes) {
-        cudaGetLastError();
-        e = build(kx, ky, kz, t, ix, iy, iz, sensi_r, sensi_i, false);
-    }
-    ready_ = e == cudaSuccess;
-    return e;
-}
-
-// Plan, buffers and launch shapes of cfg_.
-cudaError_t BfSolver::build(const float *kx, const float *ky, const float *kz, const float *t,
-                            const float *ix, const float *iy, const float *iz,
-                            const float *sensi_r, const float *sensi_i, bool image) {
-    release();
-    const BfConfig &cfg = cfg_;
     // field map is set per slice in solve()
     IMP_TRY(nu_plan_create(plan_, kx, ky, kz, t, ix, iy, iz, nullptr, sensi_r, sensi_i, cfg.M,
-                           cfg.N, cfg.C, cfg.use_z, image, err_, st_));
+                           cfg.N, cfg.C, cfg.use_z, image_, dev_err, st));
     const size_t nk = (size_t)plan_.G * plan_.Mpad * plan_.CG;
     const size_t nxs = (size_t)plan_.G * plan_.Npad * plan_.CG;
     IMP_TRY(dalloc(&y_, nk));
@@ -369,8 +354,16 @@ cudaError_t BfSolver::build(const float *kx, const float *ky, const float *kz, c
     IMP_TRY(cudaMemsetAsync(dots_, 0, sizeof(double) * 5 * kDotBlocks, st_));
     bool moved = false;
     IMP_TRY(set_reg(&moved));
-    if (plan_.img_bytes && !nu_room_beside_image()) return cudaErrorMemoryAllocation;
-    return cudaGetLastError();
+    IMP_TRY(cudaGetLastError());
+    ready_ = true;
+    return cudaSuccess;
+}
+
+bool BfSolver::drop_image() {
+    if (!plan_.img_bytes) return false;
+    release();
+    image_ = false;
+    return true;
 }
 
 // Uploads (or drops) the -reg matrix of cfg_; *graphs_stale when the penalty

@@ -42,6 +42,9 @@ public:
     long launches() const { return launches_; }
     NuPlan &plan() { return plan_; }
     void release();
+    // Gives back the FP16 kernel's image, with the rest: false when there is none.  The next
+    // set-ups of these sizes do without it (on the TF32 kernel).
+    bool drop_image();
 
     // Kernel timing: when on, graphs are not used and every NUDFT launch is
     // bracketed by CUDA events on the launching stream.
@@ -62,12 +65,10 @@ private:
     size_t prof_used_ = 0;
 
     cudaError_t set_reg(bool *graphs_stale);
-    cudaError_t build(const float *kx, const float *ky, const float *kz, const float *t,
-                      const float *ix, const float *iy, const float *iz, const float *sensi_r,
-                      const float *sensi_i, bool image);
 
     BfConfig cfg_;
     bool ready_ = false;      // the last set-up was completed
+    bool image_ = true;       // plans take the FP16 kernel's image (see drop_image)
     NuPlan plan_;
     SparseReg reg_;           // -reg: C and C^T on the device
     cudaStream_t st_ = nullptr;
@@ -110,21 +111,20 @@ public:
     long launches() const { return launches_; }
     int slices() const { return S_; }
     void release();
+    bool drop_image();  // as BfSolver's
 
 private:
     cudaError_t run_init();
     cudaError_t run_iteration();
     cudaError_t set_table(bool adj, int split);
     cudaError_t tune_shapes(bool adj);
-    cudaError_t build(int S, const int *k_off, const float *kx, const float *ky, const float *kz,
-                      const float *t, const float *ix, const float *iy, const float *iz,
-                      const float *fm, const float *sensi_r, const float *sensi_i, bool image);
 
     BfConfig cfg_;
     cudaError_t place_inputs(const float *kx, const float *ky, const float *kz, const float *t,
                              const float *ix, const float *iy, const float *iz, const float *fm,
                              const float *sensi_r, const float *sensi_i);
     bool ready_ = false;   // set up in full: a like call packs its inputs only
+    bool image_ = true;    // with the FP16 kernel's image (see drop_image)
     int switches_ = 0;     // kernel-choice switches of that set-up
     unsigned char *img_ = nullptr;  // B operand image of the FP16 tensor-core kernel
     NuPlan plan_;          // C, CG, G, Npad, use_z and the shared sensitivities

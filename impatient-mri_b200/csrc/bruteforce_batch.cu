@@ -348,36 +348,22 @@ cudaError_t BfBatch::setup(const BfConfig &cfg, int S, const int *k_off, const f
     // otherwise); only the per-call inputs are packed again.
     const int switches = (nu_tuning_enabled() ? 1 : 0) | (nu_tc_enabled() ? 2 : 0) |
                          (nu_tc_forced() ? 4 : 0);
-    if (ready_ && S == S_ && st == st_ && dev_err == err_ && switches == switches_ &&
-        cfg.N == cfg_.N && cfg.C == cfg_.C && cfg.use_z == cfg_.use_z && cfg.fd == cfg_.fd &&
-        cfg.lambda == cfg_.lambda && cfg.n0 == cfg_.n0 && cfg.n1 == cfg_.n1 &&
-        cfg.n2 == cfg_.n2 && std::equal(k_off_.begin(), k_off_.end(), k_off)) {
+    const bool like = (int)k_off_.size() == S + 1 && st == st_ && dev_err == err_ &&
+                      switches == switches_ && cfg.N == cfg_.N && cfg.C == cfg_.C &&
+                      cfg.use_z == cfg_.use_z && cfg.fd == cfg_.fd && cfg.lambda == cfg_.lambda &&
+                      cfg.n0 == cfg_.n0 && cfg.n1 == cfg_.n1 && cfg.n2 == cfg_.n2 &&
+                      std::equal(k_off_.begin(), k_off_.end(), k_off);
+    if (!like) image_ = true;
+    if (ready_ && like) {
         cfg_ = cfg;
         BB_TRY(place_inputs(kx, ky, kz, t, ix, iy, iz, fm, sensi_r, sensi_i));
         return cudaStreamSynchronize(st);
     }
+    release();
     switches_ = switches;
     cfg_ = cfg;
     st_ = st;
     err_ = dev_err;
-    // as BfSolver::setup: the image only where it leaves room for the rest
-    cudaError_t e = build(S, k_off, kx, ky, kz, t, ix, iy, iz, fm, sensi_r, sensi_i, true);
-    if (e == cudaErrorMemoryAllocation && img_) {
-        cudaGetLastError();
-        e = build(S, k_off, kx, ky, kz, t, ix, iy, iz, fm, sensi_r, sensi_i, false);
-    }
-    ready_ = e == cudaSuccess;
-    return e;
-}
-
-// Geometry, tables, buffers and launch shapes of cfg_ for S slices.
-cudaError_t BfBatch::build(int S, const int *k_off, const float *kx, const float *ky,
-                           const float *kz, const float *t, const float *ix, const float *iy,
-                           const float *iz, const float *fm, const float *sensi_r,
-                           const float *sensi_i, bool image) {
-    release();
-    const BfConfig &cfg = cfg_;
-    const cudaStream_t st = st_;
     S_ = S;
     k_off_.assign(k_off, k_off + S + 1);
     m_.resize(S);
@@ -406,7 +392,7 @@ cudaError_t BfBatch::build(int S, const int *k_off, const float *kx, const float
     plan_.vgeo = vgeo_;
     plan_.sens = sens_;
     // B operand image of the FP16 tensor-core kernel (without the memory: the TF32 one)
-    if (image && nu_wants_image(CG)) {
+    if (image_ && nu_wants_image(CG)) {
         const size_t need = nu_image_bytes(
             CG, (size_t)G * std::max<size_t>((size_t)mpad_total_, (size_t)S * Npad));
         if (cudaMalloc(&img_, need) == cudaSuccess) {
@@ -451,8 +437,16 @@ cudaError_t BfBatch::build(int S, const int *k_off, const float *kx, const float
     kb_ = std::max(2, std::min(kDotBlocks, (kDotBlocks + S - 1) / S));
     BB_TRY(dalloc(&dots_, (size_t)S * 5 * kb_));
     BB_TRY(cudaMemsetAsync(dots_, 0, sizeof(double) * S * 5 * kb_, st));
-    if (img_ && !nu_room_beside_image()) return cudaErrorMemoryAllocation;
-    return cudaStreamSynchronize(st);
+    BB_TRY(cudaStreamSynchronize(st));
+    ready_ = true;
+    return cudaSuccess;
+}
+
+bool BfBatch::drop_image() {
+    if (!img_) return false;
+    release();
+    image_ = false;
+    return true;
 }
 
 // Geometry of every slice, placed at its offsets (the shared sensitivities are

@@ -61,6 +61,17 @@ void stage_reset(imp_context *ctx);
 imp_status to_device_staged(imp_context *ctx, const float *p, size_t n, const float **out,
                             bool *was_host);
 imp_status out_device_staged(imp_context *ctx, float *p, size_t n, float **out, bool *was_host);
+// Gives back a part of the context's memory that a call can be made without: the operators'
+// scratch, the FP16 kernel's images, then the Toeplitz solvers' larger chunks.  False: none left.
+bool give_back(imp_context *ctx);
+// Makes a call, and while it runs out of device memory and there is something to give back,
+// makes it again.  Nothing of a call's in- and outputs is written before its last allocation.
+template <class F>
+imp_status in_less_memory(imp_context *ctx, F call) {
+    imp_status s = call();
+    while (s == IMP_ERR_NOMEM && give_back(ctx)) s = call();
+    return s;
+}
 
 }  // namespace imp
 

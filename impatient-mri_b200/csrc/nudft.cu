@@ -603,11 +603,6 @@ void nu_plan_reserve_image(NuPlan &p) {
     }
 }
 
-bool nu_room_beside_image() {
-    size_t free_b = 0, total = 0;
-    return cudaMemGetInfo(&free_b, &total) == cudaSuccess && free_b >= ((size_t)64 << 20);
-}
-
 cudaError_t nu_plan_repack(NuPlan &p, const float *kx, const float *ky, const float *kz,
                            const float *t, const float *ix, const float *iy, const float *iz,
                            const float *sensi_r, const float *sensi_i, unsigned *dev_err,

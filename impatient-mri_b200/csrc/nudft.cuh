@@ -73,9 +73,6 @@ void nu_plan_destroy(NuPlan &p);
 // Gives the plan the FP16 tensor-core kernel's image for both directions (of
 // the plan's own sizes).  Without the memory the plan goes on without it.
 void nu_plan_reserve_image(NuPlan &p);
-// Whether a complete set-up that holds an image leaves room for what comes with the
-// first launches (code, graphs).
-bool nu_room_beside_image();
 
 // Heuristic launch shape (replaced by the autotuner when enabled).
 NuLaunch nu_default_launch(const NuPlan &p, bool adj);

@@ -1204,6 +1204,7 @@ cudaError_t ToepSolver::apply(const float *p_r, const float *p_i, float *q_r, fl
 
 using imp::DevKeep;
 using imp::fail;
+using imp::in_less_memory;
 
 namespace {
 
@@ -1263,17 +1264,6 @@ imp::ToepSolver &solver_of(imp_context *ctx) {
 imp::ToepSolver &solver_q_of(imp_context *ctx) {
     if (!ctx->tp_q) ctx->tp_q.reset(new imp::ToepSolver());
     return *ctx->tp_q;
-}
-
-// Makes a call, and while it runs out of device memory, once more with less work memory
-// (nothing of a call's in- and outputs is written before its last allocation).
-template <class F>
-imp_status in_less_memory(imp_context *ctx, F call) {
-    imp_status s = call();
-    while (s == IMP_ERR_NOMEM &&
-           ((ctx->tp && ctx->tp->shrink()) || (ctx->tp_q && ctx->tp_q->shrink())))
-        s = call();
-    return s;
 }
 
 imp_status copy_out(imp_context *ctx, float *dst, const float *src, size_t n) {

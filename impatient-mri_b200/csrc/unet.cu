@@ -1765,18 +1765,20 @@ imp_status imp_unet_create(imp_context *ctx, int batch, int height, int width,
     *out = nullptr;
     if (batch < 1 || height < 8 || width < 8 || height % 8 || width % 8)
         return fail(IMP_ERR_INVALID_ARG, "batch >= 1 and height, width multiples of 8 required");
-    imp_status s = imp::begin(ctx);
-    if (s != IMP_OK) return s;
-    imp_unet *u = new imp_unet();
-    u->ctx = ctx;
-    cudaError_t e = u->net.setup(batch, height, width, seed, ctx->stream, ctx->dev_err);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) {
-        delete u;
-        return imp::from_cuda(e, "unet setup");
-    }
-    *out = u;
-    return IMP_OK;
+    return imp::in_less_memory(ctx, [&]() -> imp_status {
+        imp_status s = imp::begin(ctx);
+        if (s != IMP_OK) return s;
+        imp_unet *u = new imp_unet();
+        u->ctx = ctx;
+        cudaError_t e = u->net.setup(batch, height, width, seed, ctx->stream, ctx->dev_err);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) {
+            delete u;
+            return imp::from_cuda(e, "unet setup");
+        }
+        *out = u;
+        return IMP_OK;
+    });
 }
 
 // Frees the network's device memory (cudaFree synchronizes the device); does

@@ -149,3 +149,24 @@ def test_fhd_needs_no_engine(pkg):
         with leave(8 << 20):
             assert rel(call(ctx), want) < 1e-5
         assert rel(other(ctx), image) < 1e-5
+
+
+def test_kept_memory_is_given_back(pkg, monkeypatch):
+    """What earlier calls keep (operator scratch, images, engines) does not refuse a larger one."""
+    monkeypatch.setenv("IMP_AUTOTUNE", "0")
+    z = lambda n: torch.zeros(n, device="cuda")
+    M, N, C = 1 << 19, 64, 12
+    args = [z(n) for n in (N, N, C * M, C * M, M, M, M, N, N, N)] + [None, z(M)]
+    sens = [z(C * N), z(C * N)]
+    op = lambda ctx: pkg.parallelIftGpu(ctx, *args, M, N, *sens, C, 0)
+    before = [op, toeplitz(pkg, (512, 512, 1), 4, 20, "apply"), brute_force(pkg, C, 1 << 18, 0),
+              brute_force(pkg, C, 1 << 17, 2)]
+    for larger in (toeplitz(pkg, (512, 512, 1), 4, 40, "apply"), brute_force(pkg, C, 3 << 17, 0),
+                   brute_force(pkg, C, 3 << 16, 2)):
+        with pkg.Context(0) as fresh:
+            want = larger(fresh)
+        with pkg.Context(0) as ctx:
+            for f in before:
+                f(ctx)
+            with leave(24 << 20):
+                assert rel(larger(ctx), want) < 1e-5
