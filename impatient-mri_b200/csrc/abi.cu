@@ -178,7 +178,7 @@ imp_status run_forward(imp_context *ctx, float *yr, float *yi, const float *xr, 
              "pack");
     IMP_CUDA(imp::nu_forward_partials(w.p, w.l, w.packed, w.part, ctx->dev_err, ctx->stream), "F");
     IMP_CUDA(imp::nu_forward_finish_soa(w.p, w.l, w.part, yr, yi, ctx->stream), "F finish");
-    ctx->launches = 3;
+    ctx->launches = 2 + w.l.launches();  // pack, NUDFT, finish
     return finish(ctx);
 }
 
@@ -198,7 +198,7 @@ imp_status run_adjoint(imp_context *ctx, float *xr, float *xi, const float *dr, 
              "pack");
     IMP_CUDA(imp::nu_adjoint_partials(w.p, w.l, w.packed, w.part, ctx->dev_err, ctx->stream), "F^H");
     IMP_CUDA(imp::nu_adjoint_finish_soa(w.p, w.l, w.part, xr, xi, ctx->stream), "F^H finish");
-    ctx->launches = 3;
+    ctx->launches = 2 + w.l.launches();  // pack, NUDFT, finish
     return finish(ctx);
 }
 

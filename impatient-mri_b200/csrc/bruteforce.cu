@@ -396,7 +396,7 @@ cudaError_t BfSolver::run_init() {
     IMP_TRY(cudaGetLastError());
     IMP_TRY(cudaMemsetAsync(d_, 0, sizeof(float2) * plan_.Npad, st_));
     IMP_TRY(cudaMemsetAsync(dots_ + DOT_OLD * kDotBlocks, 0, sizeof(double), st_));
-    per_init_launches_ = 3;
+    per_init_launches_ = 2 + plan_.fwd.launches();
     return cudaSuccess;
 }
 
@@ -408,7 +408,7 @@ cudaError_t BfSolver::run_iteration() {
     IMP_TRY(prof_mark(1));
     // -reg takes precedence over -fd (bruteForce/bruteForceCpu.cpp:306-325)
     const int pen = reg_.on() ? PEN_REG : cfg_.fd ? PEN_FD : PEN_NONE;
-    int n = 5;
+    int n = 3 + plan_.fwd.launches() + plan_.adj.launches();
     if (pen == PEN_REG) {  // y = W C x
         IMP_TRY(reg_.apply_cw(x_, w_, nullptr, st_));
         ++n;

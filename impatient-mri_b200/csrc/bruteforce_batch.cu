@@ -601,7 +601,7 @@ cudaError_t BfBatch::run_init() {
     BB_TRY(cudaGetLastError());
     BB_TRY(cudaMemsetAsync(d_, 0, sizeof(float2) * S_ * Npad, st_));
     BB_TRY(cudaMemsetAsync(dots_, 0, sizeof(double) * S_ * 5 * kb_, st_));
-    per_init_launches_ = 3;
+    per_init_launches_ = 2 + fwd_.launches();
     return cudaSuccess;
 }
 
@@ -621,7 +621,7 @@ cudaError_t BfBatch::run_iteration() {
                              err_, st_));
     k_bb_q<<<grid, kVB, 0, st_>>>(q_, pf_, fwd_.split, tv, plan_.C, CG, G, dots_, kb_);
     BB_TRY(cudaGetLastError());
-    int n = 5;
+    int n = 3 + fwd_.launches() + adj_.launches();
     if (cfg_.fd) {
         k_bb_tvdot<<<grid, kVB, 0, st_>>>(d_, w_, plan_.N, Npad, gd, cfg_.lambda, dots_, kb_);
         BB_TRY(cudaGetLastError());

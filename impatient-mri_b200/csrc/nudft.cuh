@@ -28,6 +28,7 @@ struct NuLaunch {
     int occ = 4;    // blocks per SM the register budget is sized for (4 or 6)
     int tc = 0;     // tensor-core kernel (pt and occ unused): 1 TF32 (nudft_tc.cu), 2 FP16
                     // head / tail (nudft_h.cu, needs the plan's image)
+    int launches() const { return tc == 2 ? 2 : 1; }  // kernels of one apply (image, NUDFT)
 };
 
 struct NuPlan {

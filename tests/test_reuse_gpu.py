@@ -66,3 +66,25 @@ def test_new_context_takes_no_work_memory(pkg):
     before = torch.cuda.mem_get_info()[0]
     with pkg.Context(0):
         assert before - torch.cuda.mem_get_info()[0] < 4 << 20
+
+
+def test_launch_counts(pkg, synth):
+    """Above 8 coils every apply of the operator is two launches (operand image and NUDFT): three
+    launches of an operator call become four; a reconstruction of n updates has one more for the
+    start and two per update."""
+    from gpu_util import gpu_ft, gpu_ift, gpu_recon
+    counts = {}
+    for C in (8, 12):
+        c = case_nd(synth, 16, 16, 1, C, 300, seed=C)
+        rng = np.random.default_rng(C)
+        c["kdata"] = (rng.standard_normal((C, 300)) + 1j * rng.standard_normal((C, 300))).astype(
+            np.complex64)
+        with pkg.Context(0) as ctx:
+            counts[C] = []
+            for f in (lambda: gpu_ft(pkg, ctx, c, np.ones(256)),
+                      lambda: gpu_ift(pkg, ctx, c, c["kdata"]),
+                      lambda: gpu_recon(pkg, ctx, c, cg_num=6, lam=None, tv=False)):
+                f()
+                counts[C].append(ctx.launch_count())
+    assert counts[8][:2] == [3, 3] and counts[12][:2] == [4, 4]
+    assert counts[12][2] - counts[8][2] == 1 + 2 * 5
