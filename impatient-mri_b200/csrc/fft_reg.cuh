@@ -202,5 +202,48 @@ __device__ __forceinline__ void dft(float2 (&v)[R]) {
     }
 }
 
+// Mean gain error of the constants above, relative and averaged over all (input,
+// output) pairs: rounded to FP32 a constant is not of modulus one, and the powers of
+// two share few of them (sqrt(1/2), cos(pi / 8)), which err to the same side: a
+// 32-point transform loses 3e-8 of its amplitude, F^H F of 512x512 with its twelve
+// passes 3e-7, as much as all its rounding errors.  The twiddle tables between the two
+// passes of a line make up for it (their own roundings are as many as the line's
+// points, and even out).
+constexpr double gain_of(double c, double s, double re, double im) { return c * re + s * im - 1.0; }
+constexpr double kStep = -2.0 * 3.14159265358979323846264338327950288;
+
+constexpr double mulw_gain(int num, int den) {  // of mulw<num, den>
+    const int m = num % den;
+    if (4 * m % den == 0) return 0.0;
+    const double c = ccos(kStep * m / den), s = csin(kStep * m / den);
+    return gain_of(c, s, (float)c, (float)s);
+}
+constexpr double butterfly_gain(int k, int den) {  // of butterfly<k, den>'s factor
+    if (k == 0 || 4 * k == den) return 0.0;
+    const double c = ccos(kStep * k / den), s = csin(kStep * k / den);
+    const bool big_c = c * c >= s * s;
+    const double m = (float)(big_c ? c : s), t = (float)(big_c ? s / c : c / s);
+    return big_c ? gain_of(c, s, m, m * t) : gain_of(c, s, m * t, m);
+}
+constexpr double dft_gain(int r) {
+    double g = 0.0;
+    if ((r & (r - 1)) == 0) {  // the lower half of every stage's inputs is multiplied
+        for (int half = 2; half < r; half *= 2)
+            for (int k = 0; k < half; ++k) g += butterfly_gain(k, 2 * half) / (2 * half);
+    } else if (odd_factor(r) == r) {
+        for (int j = 1; j < r; ++j)
+            for (int k = 1; k < r; ++k) {
+                const double c = ccos(kStep * (j * k % r) / r), s = csin(kStep * (j * k % r) / r);
+                g += gain_of(c, s, (float)c, (float)s) / (r * r);
+            }
+    } else {
+        const int a = odd_factor(r), b = r / a;
+        g = dft_gain(a) + dft_gain(b);
+        for (int j = 0; j < b; ++j)
+            for (int k = 0; k < a; ++k) g += mulw_gain(j * k, r) / r;
+    }
+    return g;
+}
+
 }  // namespace fftr
 }  // namespace imp

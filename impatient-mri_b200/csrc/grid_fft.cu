@@ -380,10 +380,12 @@ cudaError_t grid_fft_create(GridFft *f, int n0, int n1, int n2, int batch) {
         f->rs[a] = row_stride(len, cw);
         f->smem[a] = sizeof(float2) * 2 * (size_t)cw * f->rs[a];
         std::vector<float2> h(len);
+        const bool two = fft2_lines(len) > 0;
+        const double gain = two ? fft2_gain(len) : 1.0;
         for (int j = 0; j < len; ++j) {
-            const int e = fft2_lines(len) ? fft2_twiddle_exp(len, j) : j;
+            const int e = two ? fft2_twiddle_exp(len, j) : j;
             const double ang = -2.0 * kPiD * (double)e / (double)len;
-            h[j] = make_float2((float)std::cos(ang), (float)std::sin(ang));
+            h[j] = make_float2((float)(std::cos(ang) / gain), (float)(std::sin(ang) / gain));
         }
         cudaError_t e = cudaMalloc(&f->tw[a], sizeof(float2) * len);
         if (e == cudaSuccess)

@@ -137,6 +137,11 @@ int fft2_twiddle_exp(int n, int i) {
     return (i % r1) * (i / r1);
 }
 
+double fft2_gain(int n) {
+    const int r2 = entry_of(n)->r2;
+    return 1.0 + fftr::dft_gain(n / r2) + fftr::dft_gain(r2);
+}
+
 cudaError_t fft2_setup() {
     for (const Entry &e : kEntries) {
         if (e.smem(lines_of(e.n)) <= 48 * 1024) continue;

@@ -41,6 +41,8 @@ __device__ __forceinline__ long long line_offset(const AxisArgs &p, long long ic
 int fft2_lines(int n);
 // Exponent of entry i < n of its twiddle table exp(-2 pi i e / n) (fft2_lines(n) > 0).
 int fft2_twiddle_exp(int n, int i);
+// Mean gain of its register transforms, which the table's entries are divided by.
+double fft2_gain(int n);
 // Launches it with p.cw lines per block (a power of two, at most fft2_lines).
 cudaError_t fft2_launch(float2 *data, const AxisArgs &p, const float2 *tw, bool inverse,
                         cudaStream_t st);

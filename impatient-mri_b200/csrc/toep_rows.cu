@@ -501,15 +501,20 @@ cudaError_t smem_opt(const Entry &e) {
 cudaError_t twiddles(const Entry &e, float2 **tw) {
     const int n = e.n;
     std::vector<float2> h(4 * (size_t)n);
-    for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < 2; ++a) {
+        // the register transforms' mean gain, parity 1 with the half twist's
+        double gain = 1.0 + fftr::dft_gain(e.r1) + fftr::dft_gain(e.r2);
+        for (int q = 0; a && q < e.r2; ++q) gain += fftr::mulw_gain(q, 2 * e.r2) / e.r2;
         for (int k2 = 0; k2 < e.r2; ++k2)
             for (int j1 = 0; j1 < e.r1; ++j1) {
                 const double ang =
                     -3.14159265358979323846264338327950288 * ((double)j1 * (2 * k2 + a)) / n;
-                const float2 w = make_float2((float)std::cos(ang), (float)std::sin(ang));
+                const float2 w =
+                    make_float2((float)(std::cos(ang) / gain), (float)(std::sin(ang) / gain));
                 h[(size_t)(a * e.r2 + k2) * e.r1 + j1] = w;
                 h[2 * (size_t)n + (size_t)(j1 * 2 + a) * e.r2 + k2] = w;
             }
+    }
     cudaError_t r = cudaMalloc(tw, sizeof(float2) * h.size());
     if (r != cudaSuccess) return r;
     return cudaMemcpy(*tw, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice);

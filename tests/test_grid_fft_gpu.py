@@ -88,6 +88,22 @@ def test_grid_fft_rejects_unsupported(pkg, ctx):
         pkg.grid_fft(ctx, y, y.copy(), 1, 1, 8192)
 
 
+@pytest.mark.parametrize("shape", [(1, 512, 512), (1, 1024, 1024), (64, 256, 256),
+                                   (1, 480, 672)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_grid_fft_amplitude(pkg, ctx, shape, inverse):
+    """Rounding errors even out; what all outputs lose or gain together (the register transforms'
+    FP32 constants are shared by few values) stays below half an FP32 ulp."""
+    rng = np.random.default_rng(11)
+    x = (rng.standard_normal((1, *shape)) + 1j * rng.standard_normal((1, *shape))).astype(
+        np.complex64)
+    got = run(pkg, ctx, x, shape, 1, inverse, device=True)
+    ref = want(x.astype(np.complex128), inverse)
+    gain = np.vdot(ref, got - ref).real / np.vdot(ref, ref).real
+    print(f"{shape} {'inverse' if inverse else 'forward'}: {gain:.1e}")
+    assert abs(gain) < 2.0 ** -24
+
+
 # lengths n = R1 R2 of the two-pass register kernel (grid_fft2.cu): smallest, odd
 # radices, both ends of the shared-memory tile, and their neighbours that the
 # Stockham kernel takes (22 = 2 x 11, 34 = 2 x 17)

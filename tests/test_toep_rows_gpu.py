@@ -55,6 +55,21 @@ def test_coils_and_segments_match_oracle(pkg, ctx, C, L):
     assert rel(got, oracle_apply(c, Q, p, c["fdp"])) < TOL_OP
 
 
+@pytest.mark.parametrize("dims", [(512, 512, 1), (256, 256, 1), (1024, 2, 1), (2, 1024, 1),
+                                  (128, 64, 32), (240, 480, 1)])
+def test_amplitude_matches_oracle(pkg, ctx, dims):
+    """The share of the result that all outputs lose or gain together is below one FP32 ulp over
+    the twelve or eighteen register transforms of an application."""
+    c, Q, p = make(dims, 2, 0, 9)
+    want = oracle_apply(c, Q, p, None)
+    o = opts_of(pkg, c)
+    o.enable_fd = 0
+    err = gpu_apply(pkg, ctx, o, c, Q, p) - want
+    gain = np.vdot(want, err).real / np.vdot(want, want).real
+    print(f"{dims}: gain {gain:.1e}, error {rel(err + want, want):.2e}")
+    assert abs(gain) < 2.0 ** -23
+
+
 def test_sizes_past_the_table(pkg, ctx):
     """A side longer than the table runs the zero-padded chain; a doubled side with a prime
     factor above 255 is refused as before."""
