@@ -347,7 +347,7 @@ cudaError_t BfBatch::setup(const BfConfig &cfg, int S, const int *k_off, const f
     // shapes and captured graphs stay (some twenty allocations and a capture
     // otherwise); only the per-call inputs are packed again.
     const int switches = (nu_tuning_enabled() ? 1 : 0) | (nu_tc_enabled() ? 2 : 0) |
-                         (nu_tc_forced() ? 4 : 0);
+                         (nu_tc_forced() ? 4 : 0) | (nu_wants_image(16) ? 8 : 0);
     const bool like = (int)k_off_.size() == S + 1 && st == st_ && dev_err == err_ &&
                       switches == switches_ && cfg.N == cfg_.N && cfg.C == cfg_.C &&
                       cfg.use_z == cfg_.use_z && cfg.fd == cfg_.fd && cfg.lambda == cfg_.lambda &&

@@ -497,13 +497,21 @@ bool nu_tc_enabled() {
 
 bool nu_tc_forced() {
     const char *e = std::getenv("IMP_NUDFT_TC");
-    return e && e[0] == '1';
+    return e && (e[0] == '1' || e[0] == 't');
+}
+
+// IMP_NUDFT_TC=tf32: the plans' state without the memory for an image.
+static bool tf32_only() {
+    const char *e = std::getenv("IMP_NUDFT_TC");
+    return e && e[0] == 't';
 }
 
 // Up to 8 coils the CUDA-core kernel's FP32 products are the more accurate ones
 // (a CG of 8 iterations on 91x91 voxels, 5 coils: 3e-6 from 64 bits against 1.2e-5),
 // so a faster split does not replace them there.
-bool nu_wants_image(int CG) { return nu_tc_enabled() && (CG > 8 || nu_tc_forced()); }
+bool nu_wants_image(int CG) {
+    return nu_tc_enabled() && !tf32_only() && (CG > 8 || nu_tc_forced());
+}
 
 bool nu_shape_supported(int CG, int pt) {
     return (CG == 1 && (pt == 4 || pt == 8)) || (CG == 2 && pt == 4) ||

@@ -135,12 +135,14 @@ bool nu_shape_supported(int CG, int pt);
 // True when `split` partitions n_theirs into whole shared-memory tiles.
 bool nu_split_ok(int n_theirs, int split);
 
-// Tensor-core kernel (nudft_tc.cu): same partial-sum layouts as
-// nu_forward_partials / nu_adjoint_partials / nu_partials_batch; coil groups
-// of 1, 2, 4, 8, 16 or 32.  It is an autotuner candidate unless
-// IMP_NUDFT_TC=0 (nu_tc_enabled), the default launch shape when
-// IMP_NUDFT_TC=1 (nu_tc_forced), and the only kernel for coil groups of 16
-// and 32 (plans of more than 8 coils, unless IMP_NUDFT_TC=0).
+// Tensor-core kernels: same partial-sum layouts as nu_forward_partials /
+// nu_adjoint_partials / nu_partials_batch; coil groups of 1, 2, 4, 8, 16 or 32
+// (16 and 32: plans of more than 8 coils, on these kernels only, unless
+// IMP_NUDFT_TC=0, nu_tc_enabled).  Plans that hold an image (nu_wants_image: more
+// than 8 coils, or IMP_NUDFT_TC=1) run the FP16 kernel (nudft_h.cu); the others the
+// TF32 one (nudft_tc.cu): up to 8 coils as an autotuner candidate, above where the
+// memory for the image is missing, and everywhere with IMP_NUDFT_TC=tf32.  With
+// =1 and =tf32 (nu_tc_forced) they are the default launch of every coil group.
 bool nu_tc_supported(int CG);
 bool nu_tc_enabled();
 bool nu_tc_forced();

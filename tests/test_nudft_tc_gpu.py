@@ -1,8 +1,10 @@
-"""The tensor-core NUDFT kernel (TF32 tcgen05 MMA, A operand written into
-tensor memory; nudft_tc.cu) against the CUDA-core kernel (IMP_NUDFT_TC=0) and
-the FP64 oracle, through the operator C-ABI (parallelFtGpu / parallelIftGpu,
-kernels/parImagingGpu.cu:92-152 in the reference).  Tolerance: 1e-5 relative
-L2 per apply, the operator bar of the CUDA-core kernel."""
+"""The two tensor-core NUDFT kernels -- FP16 head / tail operands (nudft_h.cu,
+IMP_NUDFT_TC=1) and TF32 (nudft_tc.cu, IMP_NUDFT_TC=tf32; otherwise taken where
+the memory for the FP16 kernel's image is missing) -- against the CUDA-core
+kernel (IMP_NUDFT_TC=0) and the FP64 oracle, through the operator C-ABI
+(parallelFtGpu / parallelIftGpu, kernels/parImagingGpu.cu:92-152 in the
+reference).  Tolerance: 1e-5 relative L2 per apply, the operator bar of the
+CUDA-core kernel."""
 import os
 
 import numpy as np
@@ -38,15 +40,24 @@ def built(tmp_path_factory):
             os.environ[k] = v
 
 
+KERNEL = "1"
+
+
+@pytest.fixture(autouse=True, params=["1", "tf32"])
+def kernel(request):
+    global KERNEL
+    KERNEL = request.param
+
+
 def both(fn):
     """fn() with the tensor-core kernel, then with the CUDA-core kernel."""
-    os.environ["IMP_NUDFT_TC"] = "1"
+    os.environ["IMP_NUDFT_TC"] = KERNEL
     a = fn()
     os.environ["IMP_NUDFT_TC"] = "0"
     try:
         b = fn()
     finally:
-        os.environ["IMP_NUDFT_TC"] = "1"
+        os.environ["IMP_NUDFT_TC"] = KERNEL
     return a, b
 
 
@@ -107,7 +118,8 @@ def test_ragged_sizes(pkg, ctx, M, N):
 
 def test_large_dynamic_range(pkg, ctx, synth):
     """k-space values over twelve decades: the TF32 head/tail split of the
-    data keeps the relative error of every product near 2^-21."""
+    data keeps the relative error of every product near 2^-21, the FP16 one's
+    power-of-two scales that of a tile's largest."""
     from gpu_util import gpu_ift
     c = case_nd(synth, 32, 32, 1, 4, 2000, seed=61)
     rng = np.random.default_rng(61)
@@ -133,4 +145,41 @@ def test_full_size_3d_against_cuda_cores(pkg, ctx, synth):
                t=case["t"][sel])
     assert oracle.rel_l2(a[:, sel], oracle.ft(x, sub, use_z=1)) < TOL_OP
     a, b = both(lambda: gpu_ift(pkg, ctx, case, y, use_z=1))
+    assert oracle.rel_l2(a, b) < TOL_OP and not np.array_equal(a, b)
+
+
+def test_kernels_differ(pkg, ctx, synth):
+    """The switch does select: the two kernels' roundings are not the same."""
+    from gpu_util import gpu_ft
+    c = case_nd(synth, 24, 24, 1, 12, 500, seed=5)
+    got = []
+    for k in ("1", "tf32"):
+        os.environ["IMP_NUDFT_TC"] = k
+        got.append((gpu_ft(pkg, ctx, c, np.ones(576)), ctx.launch_count()))
+    assert not np.array_equal(got[0][0], got[1][0])
+    assert got[0][1] == got[1][1] + 1  # the operand image
+
+
+@pytest.mark.parametrize("C,use_z", [(4, 0), (12, 0), (20, 1)])
+def test_batched(pkg, synth, C, use_z):
+    """Slices of unlike lengths in one launch (one CG update)."""
+    rng = np.random.default_rng(C)
+    f32 = lambda a: np.ascontiguousarray(a, np.float32)
+    n, counts = 16, (1500, 300, 2100)
+    off = np.cumsum((0,) + counts)
+    N, M, S = n * n, int(off[-1]), len(counts)
+    ix, iy, _ = synth.grid_positions(n, n, 1)
+    iz = f32(rng.uniform(-0.5, 0.5, N))
+    k = [f32(rng.uniform(-n / 2, n / 2, M)) for _ in range(3)]
+    args = [f32(rng.standard_normal(C * M)) for _ in range(2)] + k + [f32(rng.uniform(0, 0.01, M)),
+                                                                     off, ix, iy, iz]
+    tail = [f32(rng.uniform(-300, 300, S * N))] + [f32(rng.standard_normal(C * N)) for _ in range(2)]
+
+    def run():
+        xr, xi = np.zeros(S * N, np.float32), np.zeros(S * N, np.float32)
+        with pkg.Context(0) as one:
+            pkg.bruteForceBatch(one, pkg.bf_options(cg_num=2, use_z=use_z, dims=(n, n, 1)), xr, xi,
+                                *args, *tail, N, C)
+        return xr + 1j * xi
+    a, b = both(run)
     assert oracle.rel_l2(a, b) < TOL_OP and not np.array_equal(a, b)
