@@ -428,11 +428,11 @@ def test_batch_many_slices_against_oracle(pkg, ctx, synth):
     assert launches[0] == launches[1]
 
 
-def test_batch_tuned_shapes_are_cached(pkg, ctx, synth, monkeypatch, tmp_path):
+def test_batch_tuned_shapes_are_cached(pkg, synth, monkeypatch, tmp_path):
     """The batched solver tunes its launch shape per batched problem (both
     directions, timed over the whole batch) and caches it as "b1" lines; a
-    second solve of the same problem reads the cache and gives the same image
-    bit for bit; every slice stays within 1e-4 of the FP64 oracle."""
+    second solve of the same problem, on a context of its own, reads the cache
+    and gives the same image bit for bit; every slice stays within 1e-4 of the FP64 oracle."""
     cache = tmp_path / "tune.txt"
     monkeypatch.setenv("IMP_TUNE_CACHE", str(cache))
     monkeypatch.delenv("IMP_AUTOTUNE", raising=False)
@@ -458,9 +458,10 @@ def test_batch_tuned_shapes_are_cached(pkg, ctx, synth, monkeypatch, tmp_path):
     for _ in range(2):
         xr = np.zeros(S * N, np.float32)
         xi = np.zeros(S * N, np.float32)
-        pkg.bruteForceBatch(ctx, pkg.bf_options(cg_num=6), xr, xi, f32(kd.real), f32(kd.imag),
-                            cat("kx"), cat("ky"), cat("kz"), cat("t"), k_off, ix, iy, iz,
-                            cat("fm"), f32(sens.real), f32(sens.imag), N, C)
+        with pkg.Context(0) as own:
+            pkg.bruteForceBatch(own, pkg.bf_options(cg_num=6), xr, xi, f32(kd.real), f32(kd.imag),
+                                cat("kx"), cat("ky"), cat("kz"), cat("t"), k_off, ix, iy, iz,
+                                cat("fm"), f32(sens.real), f32(sens.imag), N, C)
         images.append(xr + 1j * xi.astype(np.float64))
     lines = [ln.split() for ln in cache.read_text().splitlines() if ln.startswith("b1 ")]
     assert sorted(int(ln[1]) for ln in lines) == [0, 1]  # one line per direction, written once
