@@ -30,6 +30,7 @@
 #include "tv.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstddef>
@@ -115,8 +116,8 @@ __device__ __forceinline__ float kb_transform(float u, float beta) {
 // covers (ready for the inverse FFT), for a batch of grids at once: segments
 // [l0, l0 + nl) x coils [0, nc) of dr / di, grid (l - l0) nc + c at
 // `cells` elements each.  Without data (Q: the samples' real window values) a
-// grid holds two segments, 2 m in the real and 2 m + 1 in the imaginary part
-// (l0 even, nc 1, L1 segments in all).  A sample's footprint, indices and KB weights are
+// grid holds two segments, 2 m in the real and 2 m + 1 in the imaginary part,
+// the latter scaled by segw's pair_scale (l0 even, nc 1, L1 segments in all).  A sample's footprint, indices and KB weights are
 // formed once for the (at most two) segments whose Hanning window covers it
 // and for all coils, whose values the lanes load in parallel; one launch per
 // (segment, coil) had recomputed them each time and was too short to fill the
@@ -129,6 +130,51 @@ __device__ __forceinline__ float kb_transform(float u, float beta) {
 constexpr int kGridWarps = 8;
 constexpr int kGridCoils = 32;  // coils per launch at most
 
+// Sum of the samples' window values per segment: how strong each segment's Q is.
+// Neighbouring samples are nearly always of the same segments: one addition per warp
+// then (a shared-memory addition per lane loops: Q of 128x128x32 3.29 ms against 3.17;
+// this kernel takes 18 us of it, for 524288 samples).
+constexpr int kSegShared = 1024;
+__global__ void k_seg_weights(float *w, const float *t, int M, float tau, float t0, int L1) {
+    __shared__ float sh[kSegShared];
+    const bool own = L1 <= kSegShared;
+    float *sum = own ? sh : w;
+    if (own)
+        for (int l = threadIdx.x; l < L1; l += blockDim.x) sh[l] = 0.f;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int s0 = blockIdx.x * blockDim.x + threadIdx.x - lane; s0 < M;
+         s0 += gridDim.x * blockDim.x) {
+        const float ts = __ldg(&t[min(s0 + lane, M - 1)]), xs = (ts - t0) / tau;
+        const bool in = s0 + lane < M && tau > 0.f && xs > -2.f && xs < (float)L1 + 1.f;
+        const int la = in ? (int)floorf(xs) - 1 : INT_MIN;  // windows la .. la + 3
+        int same;
+        __match_all_sync(~0u, la, &same);
+        if (same && la == INT_MIN) continue;
+        for (int d = 0; d < 4; ++d) {
+            const int l = la + d;
+            float h = in && l >= 0 && l < L1 ? hanning(ts, tau, l, t0) : 0.f;
+            if (same)
+                for (int o = 16; o; o >>= 1) h += __shfl_xor_sync(~0u, h, o);
+            if (h != 0.f && (!same || lane == 0)) atomicAdd(&sum[l], h);
+        }
+    }
+    __syncthreads();
+    if (own)
+        for (int l = threadIdx.x; l < L1; l += blockDim.x)
+            if (sh[l] != 0.f) atomicAdd(&w[l], sh[l]);
+}
+
+// Power of two (or with sign -1 its inverse) that brings the second of two segments that
+// share a grid to the strength of the first, of weights w.x and w.y.  Each segment's Q then
+// has the accuracy of a grid of its own; without it one of 1e-4 of its partner's weight
+// came out 7.9e-5 from 64 bits instead of 1.1e-5, and one without samples not zero.
+__device__ __forceinline__ float pair_scale(float2 w, int sign) {
+    if (!(w.x > 0.f && w.y > 0.f)) return 1.f;
+    const int k = (__float_as_int(w.x) >> 23) - (__float_as_int(w.y) >> 23);
+    return __int_as_float((127 + sign * min(max(k, -60), 60)) << 23);
+}
+
 // ONE: a single value per sample and step (nc 1), kept in registers (the coil
 // loop's shared-memory read per cell costs: Q of 128x128x32 3.41 -> 3.09 ms).
 // D3: a 3-D grid; the axes' roles are compile-time, their arrays in registers.
@@ -138,7 +184,7 @@ template <bool ONE, bool D3>
 __global__ void __launch_bounds__(kGridWarps * 32, kGridBlocks)
     k_grid_w(float2 *grid, size_t cells, const float *kx, const float *ky, const float *kz,
              const float *t, const float *dr, const float *di, int M, GridSpec g, float tau,
-             float t0, int l0, int nl, int nc, int L1) {
+             float t0, int l0, int nl, int nc, int L1, const float2 *segw) {
     __shared__ float wsh[kGridWarps][3][kMaxTaps];
     __shared__ float2 vsh[ONE ? 1 : kGridWarps][kGridCoils];
     if (!(tau > 0.f)) return;  // every window is empty
@@ -161,8 +207,9 @@ __global__ void __launch_bounds__(kGridWarps * 32, kGridBlocks)
         int lo[3], cnt[3];
         for (int l = la; l < lb; ++l) {
             const float h = hanning(ts, tau, dr ? l : 2 * l, t0);
-            const float h1 = !dr && 2 * l + 1 < L1 ? hanning(ts, tau, 2 * l + 1, t0) : 0.f;
+            float h1 = !dr && 2 * l + 1 < L1 ? hanning(ts, tau, 2 * l + 1, t0) : 0.f;
             if (h == 0.f && h1 == 0.f) continue;
+            if (!dr && h1 != 0.f) h1 *= pair_scale(__ldg(&segw[l]), 1);
             float2 v1 = make_float2(h, h1);
             if constexpr (ONE) {
                 if (dr) {
@@ -317,9 +364,10 @@ __device__ __forceinline__ GridAt grid_at(const GridSpec &g, int x, int y, int z
 // reference layout.  The gridded windows are real, so each segment's transform
 // F is Hermitian and G = F_0 + i F_1 separates into F_0 = (G(r) + conj G(-r)) / 2
 // and F_1 = (G(r) - conj G(-r)) / 2i: half the transforms and scatters.  A
-// voxel's indices and deapodisation (sinh per axis) serve all segments.
+// voxel's indices and deapodisation (sinh per axis) serve all segments.  segw: the
+// weights of these segments, two per grid; one without samples gives zeros.
 __global__ void k_q_post(const float2 *A, size_t cells, GridSpec g, NV n2, float *qr, float *qi,
-                         size_t G2, int nl) {
+                         size_t G2, int nl, const float2 *segw) {
     // n2: the 2N grid in voxel axis order
     const int nv[3] = {n2.v[0], n2.v[1], n2.v[2]};
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < G2;
@@ -330,12 +378,14 @@ __global__ void k_q_post(const float2 *A, size_t cells, GridSpec g, NV n2, float
         const float s = 0.5f * at.s;
         for (int l = 0; l < nl; l += 2) {
             const float2 *Al = A + (size_t)(l >> 1) * cells;
-            const float2 v = Al[at.idx], m = Al[at.neg];
-            qr[(size_t)l * G2 + q] = (v.x + m.x) * s;
-            qi[(size_t)l * G2 + q] = (v.y - m.y) * s;
+            const float2 v = Al[at.idx], m = Al[at.neg], w = __ldg(&segw[l >> 1]);
+            const float s0 = w.x > 0.f ? s : 0.f;
+            qr[(size_t)l * G2 + q] = (v.x + m.x) * s0;
+            qi[(size_t)l * G2 + q] = (v.y - m.y) * s0;
             if (l + 1 < nl) {
-                qr[(size_t)(l + 1) * G2 + q] = (v.y + m.y) * s;
-                qi[(size_t)(l + 1) * G2 + q] = (m.x - v.x) * s;
+                const float s1 = w.y > 0.f ? s * pair_scale(w, -1) : 0.f;
+                qr[(size_t)(l + 1) * G2 + q] = (v.y + m.y) * s1;
+                qi[(size_t)(l + 1) * G2 + q] = (m.x - v.x) * s1;
             }
         }
     }
@@ -701,8 +751,9 @@ void ToepSolver::release() {
     free_plan(&gfq_);
     free_plan(&gff_);
     for (void *b : {(void *)sens_, (void *)eph_, (void *)fm_, (void *)fhd_, (void *)t_,
-                    (void *)grid_})
+                    (void *)grid_, (void *)segw_})
         if (b) cudaFree(b);
+    segw_ = nullptr;
     sens_ = eph_ = fhd_ = grid_ = nullptr;
     fm_ = t_ = nullptr;
     grid_cells_ = 0;
@@ -805,6 +856,7 @@ cudaError_t ToepSolver::setup(const ToepConfig &cfg, const float *t, const float
     T_TRY(cudaMemcpyAsync(t_, t, sizeof(float) * cfg.M, cudaMemcpyDeviceToDevice, st));
     launches_ = 0;
     if (cfg.q_only) {
+        T_TRY(cudaMalloc(&segw_, sizeof(float2) * (L_ / 2 + 1)));
         ready_ = true;
         return cudaSuccess;
     }
@@ -916,17 +968,23 @@ cudaError_t ToepSolver::compute_q(const float *kx, const float *ky, const float 
     T_TRY(ensure_grid_plan(g, &gfq_, nb));
     const NV n2d{{n2[0], n2[1], n2[2]}};
     const Crop crop = crop_of(g, true);
+    T_TRY(cudaMemsetAsync(segw_, 0, sizeof(float2) * (L_ / 2 + 1), st_));
+    k_seg_weights<<<std::min((cfg_.M + kVB - 1) / kVB, 148 * 6), kVB, 0, st_>>>(
+        reinterpret_cast<float *>(segw_), t_, cfg_.M, tau_, t0_, L_ + 1);
+    T_TRY(cudaGetLastError());
+    ++launches_;
     for (int l = 0; l <= L_; l += 2 * nb) {
         const int nl = std::min(2 * nb, L_ + 1 - l), ng = (nl + 1) / 2;
         T_TRY(cudaMemsetAsync(grid_, 0, sizeof(float2) * g.cells() * ng, st_));
         auto scatter = g.is3d ? k_grid_w<true, true> : k_grid_w<true, false>;
         scatter<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(
             grid_, g.cells(), kx, ky, kz, t_, nullptr, nullptr, cfg_.M, g, tau_, t0_, l, nl, 1,
-            L_ + 1);
+            L_ + 1, segw_);
         T_TRY(cudaGetLastError());
         T_TRY(grid_fft_exec_cropped(gfq_, grid_, true, crop.lo, crop.hi, st_, ng));
         k_q_post<<<gridn(G2_), kVB, 0, st_>>>(grid_, g.cells(), g, n2d, q_out_r + (size_t)l * G2_,
-                                             q_out_i + (size_t)l * G2_, G2_, nl);
+                                             q_out_i + (size_t)l * G2_, G2_, nl,
+                                             segw_ + l / 2);
         T_TRY(cudaGetLastError());
         launches_ += 2 + gfq_.passes();
     }
@@ -978,7 +1036,7 @@ cudaError_t ToepSolver::compute_fhd(const float *kx, const float *ky, const floa
                                    : (g.is3d ? k_grid_w<false, true> : k_grid_w<false, false>);
             scatter<<<grid_blocks(), kGridWarps * 32, 0, st_>>>(
                 grid_, g.cells(), kx, ky, kz, t_, kd_r + (size_t)c * cfg_.M,
-                kd_i + (size_t)c * cfg_.M, cfg_.M, g, tau_, t0_, l, nl, nc, L_ + 1);
+                kd_i + (size_t)c * cfg_.M, cfg_.M, g, tau_, t0_, l, nl, nc, L_ + 1, nullptr);
             T_TRY(cudaGetLastError());
             T_TRY(grid_fft_exec_cropped(gff_, grid_, true, crop.lo, crop.hi, st_, nc * nl));
             k_fh_post<<<gridn(N_), kVB, 0, st_>>>(grid_, g.cells(), g, nvd, N_,

@@ -124,6 +124,7 @@ private:
     GridFft gfq_, gff_;        // gridding grids of Q and F^H d
     float2 *grid_ = nullptr;   // gridding scratch
     size_t grid_cells_ = 0;
+    float2 *segw_ = nullptr;   // [L/2+1] window sums of the segments of each pair (Q)
     cudaGraphExec_t g_iter_ = nullptr;
     long launches_ = 0;
     // pruned mixed-radix engine (sides up to its longest length); the

@@ -512,3 +512,32 @@ def test_odd_grids_match_oracle(pkg, ctx, nz, os_fh):
     want = np.asarray(T.compute_q(c["kx"], c["ky"], c["kz"], c["t"], dims, L, 1.125))
     for l in range(L + 1):
         assert rel(got[l], want.reshape(L + 1, -1)[l]) < 2 * TOL_OP
+
+
+@pytest.mark.parametrize("dims", [(32, 32, 1), (8, 10, 6)])
+@pytest.mark.parametrize("weak", ["first", "second", "none"])
+def test_q_segments_of_unlike_weight(pkg, ctx, dims, weak):
+    """Two segments share a grid: one whose samples weigh 1e-4 of its partner's keeps its own
+    accuracy, one without samples is zero."""
+    nx, ny, nz = dims
+    M, L, few = 20000, 3, 2
+    rng = np.random.default_rng(M + nz)
+    if weak == "none":  # samples at the first and last segments' centres only
+        t = np.concatenate([np.zeros(M // 2), np.full(M // 2, 3.0)])
+    else:  # nearly all within 0.02 of one segment's centre
+        t = np.concatenate([[0.0], rng.uniform(0.8, 2.9, few), [3.0],
+                            (0.0 if weak == "second" else 0.98) + rng.uniform(0.0, 0.02, M)])
+    rng.shuffle(t)
+    t[0], t[-1] = 0.0, 3.0
+    t = t.astype(np.float32)
+    k = [rng.uniform(-n / 2, n / 2 - 0.1, t.size).astype(np.float32) if n > 1 else
+         np.zeros(t.size, np.float32) for n in dims]
+    c = dict(dims=dims, L=L, cg=1, fdp=1e-2, tv_num=0, os_q=2.0, os_fh=1.5, t=t, kx=k[0], ky=k[1],
+             kz=k[2])
+    got = gpu_q(pkg, ctx, opts_of(pkg, c), c)
+    want = np.asarray(T.compute_q(*k, t, dims, L, 2.0)).reshape(L + 1, -1)
+    for l in range(L + 1):
+        if np.any(want[l]):
+            assert rel(got[l], want[l]) < 2 * TOL_OP
+        else:
+            assert not np.any(got[l])
