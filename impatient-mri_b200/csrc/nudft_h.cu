@@ -35,7 +35,9 @@
 //   warp 16         bulk loads of the tiles (geometry, B image, scales), three slots
 //   warp 17         MMA issue
 // Every wait is bounded; after one expiry a thread stops waiting, so a broken
-// pipeline ends the launch after one timeout per thread.
+// pipeline ends the launch after one timeout per thread.  The block then waits
+// once more (bounded) for its copies and MMAs in flight before it frees its
+// tensor memory and ends.
 //
 // What bounds it: 30 issued instructions per 32 pairs and scheduler (3 or 4 DFMA,
 // 2 MUFU, the packs, unpacks and subtraction of the split, the drain's share) at
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(HShape<CG>::THREADS, 1)
     extern __shared__ unsigned char smraw[];
     __shared__ __align__(8) uint64_t full[S::NSLOT], tempty[S::NSLOT];
     __shared__ __align__(8) uint64_t afull[S::GROUPS][S::NB], aempty[S::GROUPS][S::NB];
-    __shared__ __align__(8) uint64_t dfull[2], ddone[2];
+    __shared__ __align__(8) uint64_t dfull[2], ddone[2], last;
     __shared__ uint32_t tmem_sh;
 
     const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(HShape<CG>::THREADS, 1)
             mbar_init(&afull[0][0] + i, S::PROD / S::GROUPS);
             mbar_init(&aempty[0][0] + i, 1);
         }
+        mbar_init(&last, 1);
         fence_mbar_init();
     }
     h_fence_before();
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(HShape<CG>::THREADS, 1)
     h_fence_after();
     const uint32_t tmem = warp_uniform(tmem_sh);
     bool ok = true;
+    int issued = 0;  // tiles whose copies were started (bulk-load thread)
 
     if (warp < S::PROD) {
         // ------------------------------ A producers ------------------------------
@@ -440,6 +444,8 @@ __global__ void __launch_bounds__(HShape<CG>::THREADS, 1)
                 // the slot is free once tile t - NSLOT has been drained (its MMAs are then
                 // done and its geometry and scales read)
                 if (t >= S::NSLOT) h_wait(&tempty[s], (unsigned)(t / S::NSLOT - 1) & 1, ok);
+                if (!ok) break;
+                issued = t + 1;
                 fence_proxy_async_smem();
                 mbar_arrive_expect_tx(&full[s], kGeoBytes + S::BTILE + S::SBYTES);
                 bulk_g2s(s_geo + s * kTile, gsrc + (size_t)t * kTile, kGeoBytes, &full[s]);
@@ -489,7 +495,17 @@ __global__ void __launch_bounds__(HShape<CG>::THREADS, 1)
     }
     if (!ok && err) atomicOr(err, DEV_ERR_TIMEOUT);
     h_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {  // a wait ran out: what is in flight ends before the block
+        bool again = true;
+        if (warp == S::PROD && lane == 0)
+            for (int t = max(issued - S::NSLOT, 0); t < issued; ++t)
+                h_wait(&full[t % S::NSLOT], (unsigned)(t / S::NSLOT) & 1, again);
+        if (warp == S::PROD + 1) {
+            if (elect_one()) h_commit(&last);
+            __syncwarp();
+            h_wait(&last, 0, again);
+        }
+    }
     if (warp == S::PROD + 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(S::TMEM)

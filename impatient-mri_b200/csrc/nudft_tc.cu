@@ -64,7 +64,8 @@ __device__ __forceinline__ uint32_t tf32_rna(float v) {
 // the producers, about four times slower per chunk than the MMAs, leave the
 // MMA warp that much slack).
 // After one expiry (ok == false) the thread stops waiting, so a broken
-// pipeline ends the launch after one timeout per thread.
+// pipeline ends the launch after one timeout per thread; the block then waits
+// once more (bounded) for its copies and MMAs in flight.
 template <unsigned SLEEP = 0>
 __device__ __forceinline__ void tc_wait(uint64_t *bar, unsigned parity, bool &ok) {
     if (!ok) return;
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(TcShape<CG, PT, H>::THREADS, 1)
                unsigned *err, const NuSlice *__restrict__ sl, int n_groups) {
     using S = TcShape<CG, PT, H>;
     extern __shared__ unsigned char smraw[];
-    __shared__ __align__(8) uint64_t full[2], tempty[2];
+    __shared__ __align__(8) uint64_t full[2], tempty[2], last;
     __shared__ __align__(8) uint64_t afull[S::NB], aempty[S::NB], dfull[2], ddone[2];
     __shared__ uint32_t tmem_sh;
 
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(TcShape<CG, PT, H>::THREADS, 1)
             mbar_init(&afull[i], S::PROD);
             mbar_init(&aempty[i], 1);
         }
+        mbar_init(&last, 1);
         fence_mbar_init();
     }
     tc_fence_before_sync();
@@ -250,6 +252,7 @@ __global__ void __launch_bounds__(TcShape<CG, PT, H>::THREADS, 1)
     tc_fence_after_sync();
     const uint32_t tmem = tmem_sh;
     bool ok = true;
+    int issued = 0;  // tiles whose copies were started (bulk-load thread)
 
     if (warp < S::PROD) {
         // ------------------------------ A producers ------------------------------
@@ -434,6 +437,8 @@ __global__ void __launch_bounds__(TcShape<CG, PT, H>::THREADS, 1)
             for (int t = 0; t < ntiles; ++t) {
                 const int s = t & 1;
                 if (t >= 2) tc_wait<32>(&tempty[s], (unsigned)((t - 2) >> 1) & 1, ok);
+                if (!ok) break;
+                issued = t + 1;
                 fence_proxy_async_smem();
                 mbar_arrive_expect_tx(&full[s], kGeoBytes + kDatBytes);
                 bulk_g2s(s_geo + s * kTile, gsrc + (size_t)t * kTile, kGeoBytes, &full[s]);
@@ -491,7 +496,17 @@ __global__ void __launch_bounds__(TcShape<CG, PT, H>::THREADS, 1)
     }
     if (!ok && err) atomicOr(err, DEV_ERR_TIMEOUT);
     tc_fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {  // a wait ran out: what is in flight ends before the block
+        bool again = true;
+        if (warp == S::PROD && lane == 0)
+            for (int t = max(issued - 2, 0); t < issued; ++t)
+                tc_wait<32>(&full[t & 1], (unsigned)(t >> 1) & 1, again);
+        if (warp == S::PROD + 1) {
+            if (lane == 0) tc_commit(&last);
+            __syncwarp();
+            tc_wait<32>(&last, 0, again);
+        }
+    }
     if (warp == S::PROD + 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(S::TMEM)
