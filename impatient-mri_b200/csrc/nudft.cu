@@ -554,8 +554,11 @@ NuLaunch nu_default_launch(const NuPlan &p, bool adj) {
     while (blocks * split < target && split < 64 && nu_split_ok(n_theirs, split * 2) &&
            n_theirs / (split * 2) >= 4 * kTile)
         split *= 2;
-    // a problem that leaves SMs without a block splits down to single tiles
-    while (blocks * split < 148L * 4 && split < 64 && nu_split_ok(n_theirs, split * 2)) split *= 2;
+    // While that leaves half of the SMs without a block, down to single tiles (F of 16x16
+    // to 48x48: 71 to 75 us without, 58 to 64 with).  Further gains nothing (64x64, 16 to 64
+    // parts: 71 us; 4 coils 76 against 86) and costs partial sums: up to 1 MB of work memory
+    // comes out of the allocator's blocks, more is a mapping of 0.35 ms in the first call.
+    while (blocks * split * 2 <= 148L && split < 64 && nu_split_ok(n_theirs, split * 2)) split *= 2;
     l.split = split;
     return l;
 }

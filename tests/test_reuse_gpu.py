@@ -88,3 +88,19 @@ def test_launch_counts(pkg, synth):
                 counts[C].append(ctx.launch_count())
     assert counts[8][:2] == [3, 3] and counts[12][:2] == [4, 4]
     assert counts[12][2] - counts[8][2] == 1 + 2 * 5
+
+
+def test_small_operator_call_maps_no_memory(pkg, synth):
+    """The work memory of F and F^H at 64x64, one coil, fits the allocator's 2 MB blocks: a first
+    call on a new context pays for no mapping of its own."""
+    import torch
+    from gpu_util import gpu_ft, gpu_ift
+    c = case_nd(synth, 64, 64, 1, 1, 4096, seed=3)
+    x, d = np.ones(4096), np.ones((1, 4096))
+    for f in (lambda ctx: gpu_ft(pkg, ctx, c, x), lambda ctx: gpu_ift(pkg, ctx, c, d)):
+        with pkg.Context(0) as first:
+            f(first)  # kernels loaded, the arrays' memory cached
+        with pkg.Context(0) as ctx:
+            before = torch.cuda.mem_get_info()[0]
+            f(ctx)
+            assert before - torch.cuda.mem_get_info()[0] <= 2 << 20
