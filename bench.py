@@ -703,6 +703,15 @@ def toep_model_bytes(N, G, C, L1):
     return C * L1 * (8 * G + 32 * G) + C * L1 * 16 * N + 8 * C * N + 48 * N
 
 
+def toep_engine_bytes(N, G, C, L1):
+    """The same for the pruned engine, which holds no padded grid: per (coil, segment)
+    every kernel reads and writes its half spectra once (2-D: rows, columns, rows; 3-D
+    (G = 8N): rows, middle, columns, middle, rows) and the row kernels read S_c twice;
+    Qf_l once per segment, the CG vectors (48N)."""
+    spectra = 192 * N if G == 8 * N else 64 * N
+    return C * L1 * (spectra + 16 * N) + L1 * 8 * G + 48 * N
+
+
 def toep_fp64_check(pkg, ctx, case, B, opts_fields, dev):
     """FP64 oracle on the Toeplitz configuration's timed inputs (checker leg,
     outside every timed region): one A^H A + lambda D^H D application of a
@@ -863,8 +872,8 @@ def run_toeplitz(args, ws, rank, local):
     applies = o["tv_num"] * (o["cg_num"] + 1)
     cg_ms = float(np.mean(parts[:, 2]))
     per_apply_s = cg_ms / 1e3 / applies
-    model = toep_model_bytes(N, G, C, L1)
-    achieved = model / per_apply_s / 1e9
+    bytes_apply, model = toep_engine_bytes(N, G, C, L1), toep_model_bytes(N, G, C, L1)
+    achieved = bytes_apply / per_apply_s / 1e9
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (
         ROOT / "MEASURED_PEAKS.json").exists() else {}
     hbm = float(peaks.get("hbm_gbs", 6650.0))
@@ -891,9 +900,11 @@ def run_toeplitz(args, ws, rank, local):
                                        "of the five engine kernels of one application (ncu)",
                      "kernel": "A^H A application inside the CG (pruned FFT engine: k_row_fwd, k_mid_fwd, "
                                "k_col with x Qf_l, k_mid_inv, k_row_inv with the coil sum; CG update), "
-                               "per application; bytes = the zero-padded FFT model",
+                               "per application; bytes = the engine's half spectra, each kernel's "
+                               "once; bound by issue and latency more than by HBM",
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback",
-                     "algorithmic_bytes_per_apply": model, "apply_ms": per_apply_s * 1e3,
+                     "algorithmic_bytes_per_apply": bytes_apply,
+                     "zero_padded_model_bytes": model, "apply_ms": per_apply_s * 1e3,
                      "applies_per_recon": applies},
         "clocks": clk.summary(),
     }
@@ -1222,11 +1233,11 @@ def run_headline(args, ws, rank, local):
     torch.cuda.synchronize()
     upd_s = e0.elapsed_time(e1) / 1e3 / kcg
     N, G, C = prob.N, 4 * prob.N, prob.C
-    model = toep_model_bytes(N, G, C, 1)
+    bytes_apply, model = toep_engine_bytes(N, G, C, 1), toep_model_bytes(N, G, C, 1)
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (
         ROOT / "MEASURED_PEAKS.json").exists() else {}
     hbm = float(peaks.get("hbm_gbs", 6650.0))
-    achieved = model / upd_s / 1e9
+    achieved = bytes_apply / upd_s / 1e9
     net_ms = []
     for _ in range(5):
         e0.record()
@@ -1285,10 +1296,12 @@ def run_headline(args, ws, rank, local):
                                        "three engine kernels of one application (ncu)",
                      "kernel": "one CG update (A^H A application: k_row_fwd, k_col with x Qf, "
                                "k_row_inv with the coil sum; FD term; vector updates); bytes "
-                               "= the zero-padded FFT model of one A^H A application",
+                               "= the engine's half spectra, each kernel's once; bound by issue "
+                               "and latency more than by HBM",
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else
                                     "fallback 6650 GB/s",
-                     "algorithmic_bytes_per_apply": model, "update_ms": upd_s * 1e3},
+                     "algorithmic_bytes_per_apply": bytes_apply,
+                     "zero_padded_model_bytes": model, "update_ms": upd_s * 1e3},
         "error_vs_fp64": {"warm_start_nrmse_mean": f("ew"),
                           "warm_start_nrmse_max": float(max(r["ew"] for r in rows)),
                           "zero_start_nrmse_max": float(max(r["ez"] for r in rows)),
