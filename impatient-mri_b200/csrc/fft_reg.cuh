@@ -66,9 +66,9 @@ __device__ __forceinline__ float2 mulw(float2 v) {
 
 // a' = a + w b, b' = a - w b with w = exp(-2 pi i K / DEN), DEN = 2 HALF.  For a
 // general w the larger of its parts is taken out, w = c (1 + i t) or s (t + i)
-// with |t| <= 1: two FMAs form (1 + i t) b and four the outputs, instead of eight
-// multiplications and additions (a tenth of a transform's instructions), with
-// one rounding less.
+// with |t| <= 1 (the scaled butterfly of Linzer and Feig, 1993): two FMAs form
+// (1 + i t) b and four the outputs, instead of eight multiplications and additions
+// (a tenth of a transform's instructions), with one rounding less.
 template <int K, int DEN>
 __device__ __forceinline__ void butterfly(float2 &a, float2 &b) {
     if constexpr (K == 0 || 4 * K == DEN) {

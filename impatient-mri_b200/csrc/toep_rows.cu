@@ -239,8 +239,13 @@ struct ColShape {
 // a segment read the same columns of Qf_l close in time (3-D, where Qf_l exceeds
 // the L2; in 2-D the neighbouring columns first are faster, 6.51 against 6.62 ms
 // for 20 updates at 512x512 x 32 coils).
+// Threads per SM that the registers are budgeted for: 16-point transforms fit 80 registers
+// and 24 warps (256x256x32 x 4 coils: 28.1 ms per reconstruction, 28.2 with 16 warps),
+// longer ones take up to 128 and 16 warps (512x512: 6.5 ms for 20 updates, 8.9 with 24);
+// shorter ones need no budget and blocks that do not divide it keep what is left.
 template <int R1, int R2>
-__global__ void __launch_bounds__(ColShape<R1, R2>::T, cmax(1, (R1 == 16 ? 768 : 512) / ColShape<R1, R2>::T))
+__global__ void __launch_bounds__(ColShape<R1, R2>::T,
+                                  cmax(1, (R1 == 16 ? 768 : 512) / ColShape<R1, R2>::T))
     k_col(float2 *__restrict__ b1, const float2 *__restrict__ qf2, int ns, int ncol, int C,
           int job0, int jobs_x, const float2 *__restrict__ tw, const int *__restrict__ done) {
     using S = ColShape<R1, R2>;
