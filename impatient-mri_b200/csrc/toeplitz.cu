@@ -1499,6 +1499,7 @@ imp_status imp_toeplitz_cg(imp_context *ctx, const imp_toeplitz_options *opt, fl
                            int ny, int nz, double tol, int max_iter, int *iterations) {
     if (!x_r || !x_i || !fhd_r || !fhd_i) return fail(IMP_ERR_INVALID_ARG, "null array argument");
     if (max_iter < 0 || !(tol >= 0.0)) return fail(IMP_ERR_INVALID_ARG, "max_iter >= 0, tol >= 0");
+    if (!opt) return fail(IMP_ERR_INVALID_ARG, "null options");
     imp_toeplitz_options o = *opt;
     o.enable_tv = 0;  // one CG run, no reweighting passes
     return in_less_memory(ctx, [&]() -> imp_status {

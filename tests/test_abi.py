@@ -61,3 +61,21 @@ def test_no_cpu_fallback_symbols(pkg):
     L = pkg.lib()
     for n in ("orc_ft", "orc_bf_cg", "ref_bf_cg", "bruteForceCpu"):
         assert not hasattr(L, n)
+
+
+def test_null_options_are_refused(pkg):
+    """Every entry point that takes options returns a status for null ones (imp_toeplitz_cg copied
+    them first)."""
+    import ctypes
+    L = pkg.lib()
+    a = (ctypes.c_float * 16)()
+    p = ctypes.cast(a, ctypes.c_void_p)
+    L.imp_toeplitz_cg.restype = ctypes.c_int
+    assert L.imp_toeplitz_cg(None, None, p, p, p, p, p, p, p, 4, p, p, p, 1, 2, 2, 1,
+                             ctypes.c_double(0.0), 1, None) == 1
+    assert L.imp_toeplitz_recon(None, None, p, p, p, p, p, p, p, 4, p, p, p, 1, 2, 2, 1) == 1
+    assert L.imp_toeplitz_apply(None, None, p, p, p, p, p, p, p, 4, p, p, p, 1, 2, 2, 1) == 1
+    assert L.imp_toeplitz_q(None, None, p, p, p, p, p, p, 4, 2, 2, 1) == 1
+    assert L.imp_toeplitz_fhd(None, None, p, p, p, p, p, p, p, p, p, p, p, 4, 1, 2, 2, 1) == 1
+    assert L.imp_bruteforce_recon(None, None, p, p, p, p, p, p, p, p, p, p, p, p, p, p, 4, 4, 1,
+                                  1) == 1
