@@ -90,11 +90,13 @@ def test_launch_counts(pkg, synth):
     assert counts[12][2] - counts[8][2] == 1 + 2 * 5
 
 
-def test_small_operator_call_maps_no_memory(pkg, synth):
+def test_small_operator_call_maps_no_memory(pkg, synth, monkeypatch):
     """The work memory of F and F^H at 64x64, one coil, fits the allocator's 2 MB blocks: a first
-    call on a new context pays for no mapping of its own."""
+    call on a new context pays for no mapping of its own (default shapes: a shape that an earlier
+    reconstruction of this size was tuned to may have more parts)."""
     import torch
     from gpu_util import gpu_ft, gpu_ift
+    monkeypatch.setenv("IMP_AUTOTUNE", "0")
     c = case_nd(synth, 64, 64, 1, 1, 4096, seed=3)
     x, d = np.ones(4096), np.ones((1, 4096))
     for f in (lambda ctx: gpu_ft(pkg, ctx, c, x), lambda ctx: gpu_ift(pkg, ctx, c, d)):
