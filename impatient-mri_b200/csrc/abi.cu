@@ -132,17 +132,26 @@ imp_status op_work(imp_context *ctx, int M, int N, int C, bool use_z, bool adj, 
     imp::NuPlan &p = w.p;
     const size_t theirs = (size_t)p.G * (adj ? p.Mpad : p.Npad);
     size_t image = imp::nu_wants_image(p.CG) ? imp::nu_image_bytes(p.CG, theirs) : 0;
+    const size_t b_k = align256(sizeof(double4) * (size_t)p.Mpad);
+    const size_t b_v = align256(sizeof(double4) * (size_t)p.Npad);
+    const size_t b_s = adj ? align256(sizeof(float2) * (size_t)p.G * p.Npad * p.CG) : 0;
+    const size_t b_d = align256(sizeof(float2) * theirs * p.CG);
+    auto part_bytes = [&](const imp::NuLaunch &l) {
+        return align256(adj ? imp::nu_adj_partial_bytes(p, l) : imp::nu_fwd_partial_bytes(p, l));
+    };
     for (;;) {
         p.img_bytes = image;
         w.l = imp::nu_default_launch(p, adj);
-        imp::nu_tuned_lookup(p, adj, &w.l);
+        imp::NuLaunch tuned;
+        // A shape tuned for the NUDFT alone can have more parts, whose sum this call pays for:
+        // not where it takes the work memory past the 1 MB that needs no mapping of its own
+        // (F 64x64: 61 us in 64 parts, 55 in the default 16; first call 0.96 against 0.1 ms).
+        const size_t small = (size_t)1 << 20, fixed = b_k + b_v + b_s + b_d + align256(image);
+        if (imp::nu_tuned_lookup(p, adj, &tuned) &&
+            (fixed + part_bytes(tuned) <= small || fixed + part_bytes(w.l) > small))
+            w.l = tuned;
         if (w.l.tc != 2) p.img_bytes = image = 0;
-        const size_t b_k = align256(sizeof(double4) * (size_t)p.Mpad);
-        const size_t b_v = align256(sizeof(double4) * (size_t)p.Npad);
-        const size_t b_s = adj ? align256(sizeof(float2) * (size_t)p.G * p.Npad * p.CG) : 0;
-        const size_t b_d = align256(sizeof(float2) * theirs * p.CG);
-        const size_t b_p = align256(adj ? imp::nu_adj_partial_bytes(p, w.l)
-                                        : imp::nu_fwd_partial_bytes(p, w.l));
+        const size_t b_p = part_bytes(w.l);
         void *base = nullptr;
         const imp_status s = scratch(ctx, b_k + b_v + b_s + b_d + b_p + align256(image), &base);
         if (s == IMP_ERR_NOMEM && image) {  // the kernel that needs no image
