@@ -151,18 +151,33 @@ def test_fhd_needs_no_engine(pkg):
         assert rel(other(ctx), image) < 1e-5
 
 
+def adjoint(pkg, C, M, n=8, seed=0):
+    """call(ctx) -> F^H d, all arrays on the device."""
+    r = np.random.default_rng(seed)
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a, np.float32)).cuda()
+    N = n * n
+    g = (np.arange(n) - n / 2) / n
+    args = [dev(r.standard_normal(C * M)) for _ in range(2)]
+    args += [dev(r.uniform(-n / 2, n / 2, M)) for _ in range(2)] + [torch.zeros(M, device="cuda")]
+    args += [dev(np.repeat(g, n)), dev(np.tile(g, n)), torch.zeros(N, device="cuda"), None,
+             dev(r.uniform(0, 0.01, M))]
+    sens = [dev(r.standard_normal(C * N)) for _ in range(2)]
+    x = [torch.zeros(N, device="cuda") for _ in range(2)]
+
+    def call(ctx):
+        pkg.parallelIftGpu(ctx, *x, *args, M, N, *sens, C, 0)
+        return x[0].cpu().numpy() + 1j * x[1].cpu().numpy()
+    return call
+
+
 def test_kept_memory_is_given_back(pkg, monkeypatch):
     """What earlier calls keep (operator scratch, images, engines) does not refuse a larger one."""
     monkeypatch.setenv("IMP_AUTOTUNE", "0")
-    z = lambda n: torch.zeros(n, device="cuda")
-    M, N, C = 1 << 19, 64, 12
-    args = [z(n) for n in (N, N, C * M, C * M, M, M, M, N, N, N)] + [None, z(M)]
-    sens = [z(C * N), z(C * N)]
-    op = lambda ctx: pkg.parallelIftGpu(ctx, *args, M, N, *sens, C, 0)
-    before = [op, toeplitz(pkg, (512, 512, 1), 4, 20, "apply"), brute_force(pkg, C, 1 << 18, 0),
-              brute_force(pkg, C, 1 << 17, 2)]
+    C = 12
+    before = [adjoint(pkg, C, 1 << 19), toeplitz(pkg, (512, 512, 1), 4, 20, "apply"),
+              brute_force(pkg, C, 1 << 18, 0), brute_force(pkg, C, 1 << 17, 2)]
     for larger in (toeplitz(pkg, (512, 512, 1), 4, 40, "apply"), brute_force(pkg, C, 3 << 17, 0),
-                   brute_force(pkg, C, 3 << 16, 2)):
+                   brute_force(pkg, C, 3 << 16, 2), adjoint(pkg, C, 3 << 18)):
         with pkg.Context(0) as fresh:
             want = larger(fresh)
         with pkg.Context(0) as ctx:
@@ -170,3 +185,17 @@ def test_kept_memory_is_given_back(pkg, monkeypatch):
                 f(ctx)
             with leave(24 << 20):
                 assert rel(larger(ctx), want) < 1e-5
+
+
+def test_operator_without_room_is_refused(pkg):
+    """An operator call that has nothing left to give back ends with the status, and is served
+    once there is room."""
+    call = adjoint(pkg, 12, 1 << 19)
+    with pkg.Context(0) as fresh:
+        want = call(fresh)
+    with pkg.Context(0) as ctx:
+        for room in (4, 20, 40):
+            with leave(room << 20):
+                with pytest.raises(pkg.ImpError, match="NOMEM"):
+                    call(ctx)
+        assert np.array_equal(call(ctx), want)
